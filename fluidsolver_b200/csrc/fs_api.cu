@@ -254,7 +254,7 @@ fs_status free_all(fs_ctx* c) {
                     c->rho_prev, c->vstar, c->anp, c->err, c->gbnd, c->tile_desc, c->tile_ent, c->keys[0], c->keys[1], c->keys64[0], c->keys64[1],
                     c->perm[0], c->perm[1], c->h2d_cell, c->h2d_rank, c->sort_hist, c->hash_table, c->cell_start, c->cell_partials, c->bbox, c->grids, c->nbr, c->nbr_count,
                     c->scene_of[0], c->scene_of[1], c->d_scene_offsets,
-                    c->csr_offsets, c->csr_indices, c->csr_counts, c->staging, c->status, c->small_stamps, c->scalars,
+                    c->csr_offsets, c->csr_members, c->csr_sorted, c->csr_counts, c->staging, c->status, c->small_stamps, c->scalars,
                     c->stats_parts, c->stats_out};
     for (void* q : ptrs)
         if (q) cudaFree(q);
@@ -1703,85 +1703,115 @@ fs_status fs_get_neighbors_csr(fs_ctx* c, int64_t* offsets, int64_t* indices, in
         if (total) *total = 0;
         return FS_OK;
     }
+    // the counts, the longest list after them, and the 64-bit offsets with their scan's tile totals
     if (c->csr_capacity < n + 1) {
         if (c->csr_offsets) cudaFree(c->csr_offsets);
         if (c->csr_counts) cudaFree(c->csr_counts);
         c->csr_offsets = nullptr;
         c->csr_counts = nullptr;
-        FS_TRY(dalloc(&c->csr_offsets, (size_t)n + 1));
-        FS_TRY(dalloc(&c->csr_counts, (size_t)n + 1));
+        c->csr_capacity = 0;
+        FS_TRY(dalloc(&c->csr_offsets, (size_t)(n + 1 + csr_scan_tiles(n + 1))));
+        FS_TRY(dalloc(&c->csr_counts, (size_t)n + 2));
         c->csr_capacity = n + 1;
     }
-    WalkParams w = walk_of(c, false);
+    const WalkParams w = walk_of(c, false);
     const uint32_t mask = contract_owner_mask(c->prm.search);
-    FS_CUDA(cudaMemsetAsync(c->csr_counts, 0, sizeof(uint32_t) * (n + 1), st));
+    const bool rows = !c->reference_order && c->dim == 3;
+    uint32_t* longest = c->csr_counts + n + 1;
+    int64_t* totals = c->csr_offsets + n + 1;
+    FS_CUDA(cudaMemsetAsync(c->csr_counts, 0, sizeof(uint32_t) * (n + 2), st));
+    c->launches += 4;
     if (c->precision == FS_PRECISION_FP64) {
         State<double> s = state_of<double>(c);
-    c->launches++;
-        k_csr_count<double><<<grid_for(ns), kBlock, 0, st>>>(ns, s.pos, s.type, c->cell_start, w, mask,
-                                                             c->csr_counts);
+        k_csr_count<double><<<grid_for(ns), kBlock, 0, st>>>(ns, s.pos, s.type, s.hidx, c->cell_start, w, mask, rows,
+                                                             c->csr_counts, longest);
     } else {
         State<float> s = state_of<float>(c);
-    c->launches++;
-        k_csr_count<float><<<grid_for(ns), kBlock, 0, st>>>(ns, s.pos, s.type, c->cell_start, w, mask,
-                                                            c->csr_counts);
+        k_csr_count<float><<<grid_for(ns), kBlock, 0, st>>>(ns, s.pos, s.type, s.hidx, c->cell_start, w, mask, rows,
+                                                            c->csr_counts, longest);
     }
+    const int64_t tiles = csr_scan_tiles(n + 1);
+    k_csr_scan_tiles<<<(unsigned)tiles, kCsrScanThreads, 0, st>>>(c->csr_counts, n + 1, c->csr_offsets, totals);
+    k_scan_exclusive<int64_t, int64_t><<<1, 1024, 0, st>>>(totals, totals, tiles);
+    k_csr_scan_add<<<grid_for(n + 1, 256), 256, 0, st>>>(c->csr_offsets, n + 1, totals);
     FS_CUDA(cudaGetLastError());
-    c->launches++;
-    k_scan_exclusive<uint32_t, int64_t><<<1, 1024, 0, st>>>(c->csr_counts, c->csr_offsets, n + 1);
-    FS_CUDA(cudaGetLastError());
-    int64_t tot = 0;
-    FS_CUDA(cudaMemcpyAsync(&tot, c->csr_offsets + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    uint32_t most = 0;
+    FS_CUDA(cudaMemcpyAsync(&most, longest, sizeof(most), cudaMemcpyDeviceToHost, st));
+    FS_CUDA(cudaMemcpyAsync(offsets, c->csr_offsets, sizeof(int64_t) * (n + 1), cudaMemcpyDeviceToHost, st));
     FS_CUDA(cudaStreamSynchronize(st));
+    const int64_t tot = offsets[n];
     if (total) *total = tot;
     // per-list capacity of the contract (the reference throws beyond it)
     const int cap = contract_capacity(c->prm.search);
-    std::vector<uint32_t> counts((size_t)n);
-    FS_CUDA(cudaMemcpy(counts.data(), c->csr_counts, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost));
-    std::vector<uint32_t> hidx((size_t)n);
-    FS_CUDA(cudaMemcpy(hidx.data(), c->hidx[c->cur], sizeof(uint32_t) * n, cudaMemcpyDeviceToHost));
-    bool over = false;
-    std::vector<int64_t> cnt_host((size_t)n, 0);
-    for (int64_t k = 0; k < n; k++) {
-        cnt_host[hidx[k]] = counts[k];
-        if (cap > 0 && (int64_t)counts[k] > cap) over = true;
+    const bool over = cap > 0 && (int64_t)most > cap;
+    if (over) g_error = "a neighbor list exceeds the contract's capacity";
+    if (!indices || tot == 0) return over ? FS_ERR_CAPACITY : FS_OK;
+    // The members, then the sorted 64-bit lists a chunk at a time (whole
+    // lists, kCsrChunk entries or one longer list). The workspace stays with
+    // the context up to kCsrKeep members; a larger one lives for this call.
+    constexpr int64_t kCsrChunk = int64_t(1) << 24, kCsrKeep = int64_t(1) << 26;
+    const int64_t chunk = std::min(tot, std::max<int64_t>(kCsrChunk, most));
+    struct Temp {
+        void* p = nullptr;
+        ~Temp() { if (p) cudaFree(p); }
+    } big_members, big_sorted;
+    uint32_t* members = c->csr_members;
+    int64_t* sorted = c->csr_sorted;
+    if (tot > c->csr_members_capacity) {
+        if (c->csr_members) cudaFree(c->csr_members);
+        c->csr_members = members = nullptr;
+        c->csr_members_capacity = 0;
+        FS_TRY(dalloc(&members, (size_t)tot));
+        if (tot <= kCsrKeep) {
+            c->csr_members = members;
+            c->csr_members_capacity = tot;
+        } else {
+            big_members.p = members;
+        }
     }
-    offsets[0] = 0;
-    for (int64_t h = 0; h < n; h++) offsets[h + 1] = offsets[h] + cnt_host[h];
-    if (over) {
-        g_error = "a neighbor list exceeds the contract's capacity";
-        if (!indices) return FS_ERR_CAPACITY;
+    if (chunk > c->csr_sorted_capacity) {
+        if (c->csr_sorted) cudaFree(c->csr_sorted);
+        c->csr_sorted = sorted = nullptr;
+        c->csr_sorted_capacity = 0;
+        FS_TRY(dalloc(&sorted, (size_t)chunk));
+        if (chunk <= kCsrKeep) {
+            c->csr_sorted = sorted;
+            c->csr_sorted_capacity = chunk;
+        } else {
+            big_sorted.p = sorted;
+        }
     }
-    if (!indices) return over ? FS_ERR_CAPACITY : FS_OK;
-    uint32_t* d_idx = nullptr;
-    FS_TRY(dalloc(&d_idx, (size_t)std::max<int64_t>(tot, 1)));
+    c->launches++;
     if (c->precision == FS_PRECISION_FP64) {
         State<double> s = state_of<double>(c);
-    c->launches++;
-        k_csr_fill<double><<<grid_for(ns), kBlock, 0, st>>>(ns, s.pos, s.type, c->cell_start, w, mask,
-                                                            c->csr_offsets, d_idx);
+        k_csr_fill<double><<<grid_for(ns), kBlock, 0, st>>>(ns, s.pos, s.type, s.hidx, c->cell_start, w, mask, rows,
+                                                            c->csr_offsets, members);
     } else {
         State<float> s = state_of<float>(c);
-    c->launches++;
-        k_csr_fill<float><<<grid_for(ns), kBlock, 0, st>>>(ns, s.pos, s.type, c->cell_start, w, mask,
-                                                           c->csr_offsets, d_idx);
+        k_csr_fill<float><<<grid_for(ns), kBlock, 0, st>>>(ns, s.pos, s.type, s.hidx, c->cell_start, w, mask, rows,
+                                                           c->csr_offsets, members);
     }
-    std::vector<uint32_t> idx((size_t)tot);
-    std::vector<int64_t> off_sorted((size_t)n + 1);
-    cudaError_t e1 = cudaGetLastError();
-    cudaError_t e2 = cudaMemcpyAsync(idx.data(), d_idx, sizeof(uint32_t) * tot, cudaMemcpyDeviceToHost, st);
-    cudaError_t e3 = cudaMemcpyAsync(off_sorted.data(), c->csr_offsets, sizeof(int64_t) * (n + 1),
-                                     cudaMemcpyDeviceToHost, st);
-    cudaError_t e4 = cudaStreamSynchronize(st);
-    cudaFree(d_idx);
-    if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess || e4 != cudaSuccess)
-        return fail(FS_ERR_CUDA, "CSR export failed");
-    for (int64_t k = 0; k < n; k++) {
-        const int64_t h = hidx[k];
-        int64_t o = offsets[h];
-        for (int64_t q = off_sorted[k]; q < off_sorted[k + 1]; q++) indices[o++] = hidx[idx[q]];
-        std::sort(indices + offsets[h], indices + offsets[h + 1]);
+    for (int64_t h0 = 0; h0 < n;) {
+        // the last list end within the chunk (offsets ascend), at least one list
+        int64_t h1 = std::upper_bound(offsets + h0 + 1, offsets + n + 1, offsets[h0] + chunk) - offsets - 1;
+        h1 = std::max(h1, h0 + 1);
+        const int64_t entries = offsets[h1] - offsets[h0];
+        if (entries > 0) {
+            c->launches++;
+            k_csr_sort<<<grid_for(h1 - h0, kCsrSortWarps), 32 * kCsrSortWarps, 0, st>>>(h0, h1, c->csr_offsets,
+                                                                                        members, sorted);
+            if (most > (uint32_t)kCsrWarpMax) {
+                c->launches++;
+                k_csr_sort_long<<<(unsigned)std::min<int64_t>(h1 - h0, 148 * 4), kCsrLongThreads, 0, st>>>(
+                    h0, h1, c->csr_offsets, members, sorted);
+            }
+            FS_CUDA(cudaGetLastError());
+            FS_CUDA(cudaMemcpyAsync(indices + offsets[h0], sorted, sizeof(int64_t) * entries, cudaMemcpyDeviceToHost,
+                                    st));
+        }
+        h0 = h1;
     }
+    FS_CUDA(cudaStreamSynchronize(st));
     return over ? FS_ERR_CAPACITY : FS_OK;
 }
 

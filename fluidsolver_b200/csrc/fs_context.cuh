@@ -107,11 +107,15 @@ struct fs_ctx {
     int64_t n_owners = 0;          // owners of the solver lists: [0, n_owners)
     int64_t launches = 0;          // this library's kernel launches
 
-    // CSR export of the last search (sorted space)
+    // workspace of the CSR export (fs_get_neighbors_csr): per-list counts and
+    // offsets, the lists' members, and a chunk of sorted 64-bit lists
     int64_t* csr_offsets = nullptr;
-    uint32_t* csr_indices = nullptr;
-    int64_t csr_capacity = 0;
     uint32_t* csr_counts = nullptr;
+    int64_t csr_capacity = 0;
+    uint32_t* csr_members = nullptr;
+    int64_t csr_members_capacity = 0;
+    int64_t* csr_sorted = nullptr;
+    int64_t csr_sorted_capacity = 0;
 
     // staging for host transfers
     void* staging = nullptr;
