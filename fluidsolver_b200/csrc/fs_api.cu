@@ -2438,22 +2438,29 @@ static fs_status render_scene_of(fs_ctx* c, float surface_fraction, RenderScene&
     if (!(surface_fraction > 0.0f)) return fail(FS_ERR_INVALID, "the surface density fraction must be positive");
     FS_CUDA(cudaSetDevice(c->device));
     FS_TRY(search_for_step(c, c->prm.timestep));
-    int* d_box = nullptr;
-    FS_TRY(dalloc(&d_box, 6));
+    // the box and the map of occupied neighborhoods in the staging buffer,
+    // which nothing else uses until the rays are done
+    constexpr size_t kBoxBytes = 256;
+    FS_TRY(ensure_staging(c, kBoxBytes + (size_t)c->cells));
+    int* d_box = (int*)c->staging;
+    uint8_t* d_map = (uint8_t*)c->staging + kBoxBytes;
     const int init[6] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN};
     int box[6];
     cudaError_t e = cudaMemcpyAsync(d_box, init, sizeof(init), cudaMemcpyHostToDevice, c->stream);
-    c->launches++;
+    rs.w = walk_of(c, false);
+    rs.map = d_map;
+    c->launches += 2;
     if (e == cudaSuccess) {
         if (c->precision == FS_PRECISION_FP64)
             k_particle_box<double><<<grid_for(c->n), kBlock, 0, c->stream>>>(c->n, state_of<double>(c), d_box);
         else
             k_particle_box<float><<<grid_for(c->n), kBlock, 0, c->stream>>>(c->n, state_of<float>(c), d_box);
+        k_neighborhood_map<<<std::min<unsigned>(grid_for(c->cells, 256), 148u * 16u), 256, 0, c->stream>>>(
+            c->cell_start, rs.w, d_map);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(box, d_box, sizeof(box), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    cudaFree(d_box);
     if (e != cudaSuccess) return fail(FS_ERR_CUDA, std::string("particle box: ") + cudaGetErrorString(e));
     auto unord = [](int i) {
         const int b = i >= 0 ? i : i ^ 0x7fffffff;
@@ -2472,7 +2479,6 @@ static fs_status render_scene_of(fs_ctx* c, float surface_fraction, RenderScene&
     rs.kern.alpha = c->kernel_alpha;
     rs.kern.inv_h = 1.0f / c->kernel_h;
     rs.kern.alpha_h = c->kernel_alpha * c->kernel_h;
-    rs.w = walk_of(c, false);
     return FS_OK;
 }
 
@@ -2499,11 +2505,11 @@ fs_status fs_trace_rays(fs_ctx* c, float surface_fraction, int64_t n, const floa
     if (e == cudaSuccess) {
         c->launches++;
         if (c->precision == FS_PRECISION_FP64)
-            k_trace_rays<double><<<grid_for(n), kBlock, 0, st>>>(n, d_in, d_in + 3 * n, state_of<double>(c),
+            k_trace_rays<double><<<grid_for(n, kRayWarps), 32 * kRayWarps, 0, st>>>(n, d_in, d_in + 3 * n, state_of<double>(c),
                                                                  c->cell_start, rs, d_hit, d_out, d_out + 3 * n,
                                                                  d_out + 6 * n);
         else
-            k_trace_rays<float><<<grid_for(n), kBlock, 0, st>>>(n, d_in, d_in + 3 * n, state_of<float>(c),
+            k_trace_rays<float><<<grid_for(n, kRayWarps), 32 * kRayWarps, 0, st>>>(n, d_in, d_in + 3 * n, state_of<float>(c),
                                                                 c->cell_start, rs, d_hit, d_out, d_out + 3 * n,
                                                                 d_out + 6 * n);
         e = cudaGetLastError();
@@ -2612,9 +2618,9 @@ fs_status fs_render(fs_ctx* c, const fs_camera* cam, const fs_render_settings* r
     FS_TRY(dalloc(&d_rad, (size_t)np * 3));
     c->launches++;
     if (c->precision == FS_PRECISION_FP64)
-        k_render<double><<<grid_for(np), kBlock, 0, c->stream>>>(state_of<double>(c), c->cell_start, rs, rc, sh, d_rad);
+        k_render<double><<<grid_for(np, kRayWarps), 32 * kRayWarps, 0, c->stream>>>(state_of<double>(c), c->cell_start, rs, rc, sh, d_rad);
     else
-        k_render<float><<<grid_for(np), kBlock, 0, c->stream>>>(state_of<float>(c), c->cell_start, rs, rc, sh, d_rad);
+        k_render<float><<<grid_for(np, kRayWarps), 32 * kRayWarps, 0, c->stream>>>(state_of<float>(c), c->cell_start, rs, rc, sh, d_rad);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(radiance, d_rad, sizeof(float) * 3 * np, cudaMemcpyDeviceToHost, c->stream);

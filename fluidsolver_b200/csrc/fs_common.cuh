@@ -68,8 +68,8 @@ template <typename R> struct SplineKernel {
     R alpha;  // 5/(14 pi h^2) in 2D, 1/(4 pi h^3) in 3D
 
     // GetKernelValue(position - neighborPosition); d = x_i - x_j
-    __device__ __forceinline__ R W(V3<R> d) const {
-        R q = sqrt_(dot(d, d)) / h;
+    __device__ __forceinline__ R W(V3<R> d) const { return W_of(sqrt_(dot(d, d)) / h); }
+    __device__ __forceinline__ R W_of(R q) const {   // q = |d| / h
         R ret = R(0);
         if (q < R(1)) {
             R a = R(2) - q, b = R(1) - q;
