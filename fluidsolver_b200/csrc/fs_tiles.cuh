@@ -610,22 +610,47 @@ __device__ __forceinline__ void walk_tile_list(const TileLists& T, const TileSla
 }
 
 // Walks owner k's 32-bit list in a fallback tile, the entries of this
-// thread of the owner's TPO (half, half + TPO, ...): f(sorted index, boundary)
-// for each (the fluid entries only with FLUID_ONLY), flush() after every 8
-// visits and at the end, as for_tile_entries does.
-template <bool FLUID_ONLY, int TPO = 2, typename F, typename Flush>
-__device__ __forceinline__ void walk_fallback_list(const Lists& L, int64_t k, int half, F&& f, Flush&& flush) {
+// thread of the owner's TPO (half, half + TPO, ...): use(load(sorted index),
+// boundary) for each (the fluid entries only with FLUID_ONLY), flush() after
+// every 8 visits and at the end, as for_tile_entries does. BATCH entries' loads are in flight together: one at a time, an entry cost two
+// dependent trips to L2, and a fallback tile's acceleration pass took 14,000
+// cycles against 6,600 of a staged tile, which all blocks of a small scene
+// then waited for.
+constexpr int kFallbackBatch = 4;
+template <bool FLUID_ONLY, int TPO = 2, int BATCH = kFallbackBatch, typename Load, typename Use, typename Flush>
+__device__ __forceinline__ void walk_fallback_list(const Lists& L, int64_t k, int half, Load&& load, Use&& use,
+                                                   Flush&& flush) {
     const uint32_t nn = L.size(k);
     uint32_t visited = 0;
-    for (uint32_t q = (uint32_t)half; q < nn; q += TPO) {
-        const uint32_t e = L.at(k, q);
-        const bool bnd = (e & kBoundaryBit) != 0u;
-        if (FLUID_ONLY && bnd) continue;
-        f(e & kIndexMask, bnd);
-        if ((++visited & 7u) == 0u) flush();
+    for (uint32_t q = (uint32_t)half; q < nn; q += TPO * BATCH) {
+        uint32_t e[BATCH];
+#pragma unroll
+        for (int b = 0; b < BATCH; b++) e[b] = L.at(k, min(q + b * TPO, nn - 1));
+        decltype(load(0u)) v[BATCH];
+#pragma unroll
+        for (int b = 0; b < BATCH; b++) v[b] = load(e[b] & kIndexMask);
+#pragma unroll
+        for (int b = 0; b < BATCH; b++) {
+            const bool bnd = (e[b] & kBoundaryBit) != 0u;
+            if (q + b * TPO >= nn || (FLUID_ONLY && bnd)) continue;
+            use(v[b], bnd);
+            if ((++visited & 7u) == 0u) flush();
+        }
     }
     flush();
 }
+// the fields of a neighbor in a fallback tile: position and mass, a float4 field, a float field
+struct Neighbor1 {
+    float4 pos;
+    float f;
+};
+struct Neighbor4 {
+    float4 pos, v;
+};
+struct Neighbor41 {
+    float4 pos, v;
+    float f;
+};
 
 // The pressure passes with TPO threads per owner (1, 2 or 4; fs_autotune
 // chooses): each thread takes a contiguous 8 / TPO of every octet of the
@@ -850,9 +875,9 @@ __global__ void __launch_bounds__(kPassThreads, kL1GlobalEntries ? 4 : 3) k_tile
     if (h.nranges == kTileFallback) {
         // the owner's 32-bit list, split between its two threads
         if (valid)
-            walk_fallback_list<false>(L, k, half, [&](uint32_t j, bool bnd) {
-                pair(s.pos[j], s.vel[j], s.rho_prev[j], bnd);
-            }, flush);
+            walk_fallback_list<false>(L, k, half, [&](uint32_t j) {
+                return Neighbor41{s.pos[j], s.vel[j], s.rho_prev[j]};
+            }, [&](const Neighbor41& n, bool bnd) { pair(n.pos, n.v, n.f, bnd); }, flush);
     } else {
         float4* sp = tile_smem;
         float4* sv = tile_smem + T.cap;
@@ -934,8 +959,8 @@ __global__ void __launch_bounds__(kPassThreads, kL2GlobalEntries ? 4 : 3) k_tile
         // the owner's 32-bit list, split between its two threads; the same sums
         // as a tiled owner's, so that gbnd is there for the pressure passes
         if (valid)
-            walk_fallback_list<false>(L, k, half, [&](uint32_t j, bool bnd) { pair(s.pos[j], s.vstar[j], bnd); },
-                                      flush);
+            walk_fallback_list<false>(L, k, half, [&](uint32_t j) { return Neighbor4{s.pos[j], s.vstar[j]}; },
+                                      [&](const Neighbor4& n, bool bnd) { pair(n.pos, n.v, bnd); }, flush);
     } else {
         float4* sp = tile_smem;
         float4* sa = tile_smem + T.cap;
@@ -1016,7 +1041,8 @@ __global__ void __launch_bounds__(pressure_threads<TPO>(), acc_blocks_per_sm<TPO
     if (h.nranges == kTileFallback) {
         // the owner's 32-bit list, split between its threads
         if (valid)
-            walk_fallback_list<true, TPO>(L, k, half, [&](uint32_t j, bool) { pair(s.pos[j], s.p[j]); }, flush);
+            walk_fallback_list<true, TPO>(L, k, half, [&](uint32_t j) { return Neighbor1{s.pos[j], s.p[j]}; },
+                                          [&](const Neighbor1& n, bool) { pair(n.pos, n.f); }, flush);
     } else {
         float4* sp = tile_smem;
         float* sa = reinterpret_cast<float*>(tile_smem + T.cap);
@@ -1086,7 +1112,8 @@ __global__ void __launch_bounds__(pressure_threads<TPO>(), update_blocks_per_sm<
     if (h.nranges == kTileFallback) {
         // the owner's 32-bit list, split between its threads
         if (valid)
-            walk_fallback_list<true, TPO>(L, k, half, [&](uint32_t j, bool) { pair(s.pos[j], s.acc[j]); }, flush);
+            walk_fallback_list<true, TPO>(L, k, half, [&](uint32_t j) { return Neighbor4{s.pos[j], s.acc[j]}; },
+                                          [&](const Neighbor4& n, bool) { pair(n.pos, n.v); }, flush);
     } else {
         float4* sp = tile_smem;
         float4* sa = tile_smem + T.cap;
@@ -1159,13 +1186,9 @@ __global__ void __launch_bounds__(kPassThreads, 5) k_tile_sesph3d_density(int64_
     };
     if (h.nranges == kTileFallback) {
         // the owner's 32-bit list, split between its two threads
-        const uint32_t nn = valid ? L.size(k) : 0u;
-        for (uint32_t q = half; q < nn; q += 2) {
-            const uint32_t e = L.at(k, q);
-            pair(s.pos[e & kIndexMask], (e & kBoundaryBit) != 0u);
-            if ((q & 15u) >= 14u) flush();
-        }
-        flush();
+        if (valid)
+            walk_fallback_list<false>(L, k, half, [&](uint32_t j) { return s.pos[j]; },
+                                      [&](const float4& pj, bool bnd) { pair(pj, bnd); }, flush);
     } else {
         float4* sp = tile_smem;
         __shared__ TileStage stg;
@@ -1233,14 +1256,10 @@ __global__ void __launch_bounds__(kPassThreads, 4) k_tile_sesph3d_accel(int64_t 
     };
     if (h.nranges == kTileFallback) {
         // the owner's 32-bit list, split between its two threads
-        const uint32_t nn = valid ? L.size(k) : 0u;
-        for (uint32_t q = half; q < nn; q += 2) {
-            const uint32_t e = L.at(k, q);
-            const uint32_t j = e & kIndexMask;
-            pair(s.pos[j], s.vel[j], s.rho[j], (e & kBoundaryBit) != 0u);
-            if ((q & 15u) >= 14u) flush();
-        }
-        flush();
+        if (valid)
+            walk_fallback_list<false, 2, 2>(L, k, half, [&](uint32_t j) {   // (4 would spill)
+                return Neighbor41{s.pos[j], s.vel[j], s.rho[j]};
+            }, [&](const Neighbor41& n, bool bnd) { pair(n.pos, n.v, n.f, bnd); }, flush);
     } else {
         float4* sp = tile_smem;
         float4* sv = tile_smem + T.cap;
