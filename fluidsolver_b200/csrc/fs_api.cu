@@ -160,6 +160,23 @@ Lists lists_of(fs_ctx* c) {
     return L;
 }
 
+// Staged candidates per tile: the caller's (fs_set_tuning, fs_autotune), or
+// kTileCapSmall for scenes where it costs no extra round of resident blocks
+// in the pressure passes (3 instead of 4 per SM; 2 per SM in the loop's form
+// with a block per tile). A dam's tiles have 1,400 candidates on average, and
+// the 5-10 % of them above kTileCap, which fall back to 32-bit lists, are
+// the slowest blocks of every pass. B200, a pressure iteration with 1,536 and
+// with 2,048: 8,000 fluid particles 13.5 and 11.9 us, 100,000 34.7 and 28.9,
+// 165,000 47.1 and 40.6; but 60,800 (475 tiles, two rounds of 444 blocks
+// instead of one of 592) 21.5 and 27.1, 512,000 110.6 and 115.5.
+int tile_cap_of(const fs_ctx* c) {
+    if (c->tuning.cap > 0) return c->tuning.cap;
+    const int64_t tiles = (c->n_owners + kTileOwners - 1) / kTileOwners, sms = c->sms;
+    auto rounds = [&](int64_t per_sm) { return (tiles + per_sm * sms - 1) / (per_sm * sms); };
+    const bool small = tiles <= 2 * sms || (tiles > 4 * sms && rounds(3) <= rounds(4));
+    return small ? kTileCapSmall : kTileCap;
+}
+
 TileLists tile_lists_of(fs_ctx* c) {
     TileLists T;
     T.desc = c->tile_desc;
@@ -167,7 +184,7 @@ TileLists tile_lists_of(fs_ctx* c) {
     T.count = c->nbr_count;
     T.stride = c->tile_stride;
     T.K = c->nbr_capacity;
-    T.cap = c->tuning.cap;
+    T.cap = tile_cap_of(c);
     return T;
 }
 
@@ -731,9 +748,9 @@ template <typename R> fs_status search_impl(fs_ctx* c, bool solver_lists) {
             if (tiled_mode(c) && c->n_owners > 0) {
                 const int64_t tiles = (c->n_owners + kTileOwners - 1) / kTileOwners;
                 c->launches++;
-                k_build_tiles<<<(unsigned)tiles, kTileOwners, tile_build_smem(c->nbr_capacity, c->tuning.cap), st>>>(
+                k_build_tiles<<<(unsigned)tiles, kTileOwners, tile_build_smem(c->nbr_capacity, tile_cap_of(c)), st>>>(
                     c->n_owners, s.pos, s.type, c->cell_start, w, c->tile_desc, c->tile_ent, c->tile_stride, c->nbr,
-                    c->nbr_stride, c->nbr_capacity, c->tuning.cap, c->nbr_count, c->status, c->scalars);
+                    c->nbr_stride, c->nbr_capacity, tile_cap_of(c), c->nbr_count, c->status, c->scalars);
                 built = true;
             }
         }
@@ -951,6 +968,54 @@ void enqueue_tile_pressure_iteration(fs_ctx* c, cudaStream_t bs, unsigned tiles,
 #undef FSB_ACC_LAUNCH
 #undef FSB_UPDATE_LAUNCH
 
+// The form of the pressure loop for a step (k_tile_iisph3d_pressure_loop), with
+// its grid: 0 the graph's WHILE node, 1 a block per tile, 2 several tiles per
+// block. Single scenes with two threads per owner (the only instantiation), up
+// to the size where the launches it saves no longer show: 512,000 particles 110
+// against 115 us an iteration, a million 214 against 213.
+constexpr unsigned kLoopMaxTiles = 4096;
+int pressure_loop_form(const fs_ctx* c, unsigned tiles, unsigned* blocks, size_t* smem) {
+    if (c->scenes > 0 || c->tuning.pressure_tpo != 2 || c->prm.max_iterations <= 0 || tiles > kLoopMaxTiles) return 0;
+    int per_sm = 0;
+    for (int form = 1; form <= 2; form++) {
+        *smem = tile_loop_smem(form == 1, c->nbr_capacity, tile_cap_of(c));
+        if (*smem > kLoopSmemMax) continue;
+        const cudaError_t e =
+            form == 1 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tile_iisph3d_pressure_loop<true>,
+                                                                      kPassThreads, *smem)
+                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tile_iisph3d_pressure_loop<false>,
+                                                                      kPassThreads, *smem);
+        const unsigned resident = e == cudaSuccess ? (unsigned)(per_sm * c->sms) : 0u;
+        *blocks = std::min(tiles, resident);
+        if (*blocks > 0 && (form == 2 || *blocks == tiles)) return form;
+    }
+    return 0;
+}
+
+// The iterations after the first, the test of each and the CFL clamp in one
+// cooperative launch, which guarantees that its blocks are resident together.
+fs_status enqueue_pressure_loop_launch(fs_ctx* c, int form, unsigned blocks, size_t smem, unsigned tiles, int64_t nf,
+                                       const State<float>& s, const TileLists& T, const Lists& L,
+                                       const SolverConsts<float>& k) {
+    const fs_params& p = c->prm;
+    const LoopTest lt{p.min_iterations, p.max_iterations, p.max_density_error, p.particle_size, cfl_default(c),
+                      p.lambda_v, p.lambda_a};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kPassThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    c->launches++;
+    FS_CUDA(cudaLaunchKernelEx(&cfg, form == 1 ? k_tile_iisph3d_pressure_loop<true> : k_tile_iisph3d_pressure_loop<false>,
+                               nf, (int64_t)tiles, s, T, L, k, lt, c->scalars, c->status));
+    return FS_OK;
+}
+
 // the IISPH 3D step on tile lists (fs_tiles.cuh)
 fs_status step_iisph3d_tiled(fs_ctx* c, bool capture) {
     cudaStream_t st = c->stream;
@@ -975,15 +1040,22 @@ fs_status step_iisph3d_tiled(fs_ctx* c, bool capture) {
     FS_CUDA(cudaGetLastError());
     FS_TRY(mark(c, 3, st));
     // the second loop also ran the first pressure iteration (fs_tiles.cuh)
-    FS_TRY(enqueue_pressure_loop(c, capture, false, true, [&](cudaStream_t bs) {
-        c->launches += 2;
-        enqueue_tile_pressure_iteration(c, bs, tiles, nf, s, T, L, k);
-        return true;
-    }, true));
-    FS_TRY(mark(c, 4, st));
-    c->launches++;
-    k_cfl<<<1, 128, 0, st>>>(c->scalars, c->nsc(), c->prm.particle_size, cfl_default(c), c->prm.lambda_v,
-                             c->prm.lambda_a, c->status);
+    unsigned blocks = 0;
+    size_t loop_smem = 0;
+    if (const int form = capture ? pressure_loop_form(c, tiles, &blocks, &loop_smem) : 0) {
+        FS_TRY(enqueue_pressure_loop_launch(c, form, blocks, loop_smem, tiles, nf, s, T, L, k));
+        FS_TRY(mark(c, 4, st));
+    } else {
+        FS_TRY(enqueue_pressure_loop(c, capture, false, true, [&](cudaStream_t bs) {
+            c->launches += 2;
+            enqueue_tile_pressure_iteration(c, bs, tiles, nf, s, T, L, k);
+            return true;
+        }, true));
+        FS_TRY(mark(c, 4, st));
+        c->launches++;
+        k_cfl<<<1, 128, 0, st>>>(c->scalars, c->nsc(), c->prm.particle_size, cfl_default(c), c->prm.lambda_v,
+                                 c->prm.lambda_a, c->status);
+    }
     c->launches++;
     k_iisph3d_integrate<float><<<grid_for(n, c->tuning.block), c->tuning.block, 0, st>>>(n, s, c->scalars, c->status);
     FS_CUDA(cudaGetLastError());
@@ -1519,6 +1591,7 @@ static fs_status create_ctx(const fs_params* p, int32_t scenes, const int64_t* o
     if (!c) return fail(FS_ERR_INVALID, "out of host memory");
     c->prm = *p;
     c->device = p->device;
+    c->sms = prop.multiProcessorCount;
     derive(c);
     c->cap = p->max_particles;
     if (scenes > 0) {
@@ -2215,7 +2288,7 @@ fs_status fs_autotune(fs_ctx* c, fs_tuning* out) {
     *out = fs_tuning{};
     out->first_loop_prefetch = c->tuning.l1_ahead;
     out->pressure_prefetch = c->tuning.pressure_ahead;
-    out->tile_cap = c->tuning.cap;
+    out->tile_cap = tile_cap_of(c);
     out->block_size = c->tuning.block;
     out->pressure_threads_per_owner = c->tuning.pressure_tpo;
     // nothing tunable unless the IISPH passes are tiled
@@ -2292,7 +2365,7 @@ fs_status fs_autotune(fs_ctx* c, fs_tuning* out) {
     // 3. staging cap
     const int caps[4] = {1024, 1536, 2048, 3072};
     double best = 1e30;
-    int best_cap = t->tuning.cap;
+    int best_cap = tile_cap_of(t);
     for (int q = 0; q < 4; q++) {
         FS_TRY(fs_upload(t, &v));
         t->tuning.cap = caps[q];

@@ -229,6 +229,13 @@ struct StepScalars {
     int loop_guard;          // executions of the pressure-loop body this step
     unsigned int gen_v2_bits;   // dynamic time step generator: largest |v|^2, |a|^2 at the step's start
     unsigned int gen_a2_bits;
+    // the one-launch pressure loop (fs_tiles.cuh): the second set of an
+    // iteration's accumulators (iterations alternate between err_sum .. max_v2_bits
+    // and these), and its counters
+    double err_sum_odd;
+    unsigned long long err_count_odd;
+    unsigned int max_err_bits_odd, max_a2_bits_odd, max_v2_bits_odd;
+    unsigned int loop_arrived;   // blocks that have arrived at its grid barriers
 };
 
 }  // namespace fsb

@@ -31,6 +31,7 @@ struct fs_ctx {
     fs_params prm{};
     int dim = 3;
     int device = 0;
+    int sms = 148;            // the device's multiprocessors
     cudaStream_t stream = nullptr;
     int64_t cap = 0;          // particle capacity
     int64_t n = 0;            // particles uploaded

@@ -411,20 +411,14 @@ __device__ __forceinline__ ErrPart iisph3d_first_iteration(int64_t k, const Stat
     return iisph3d_pressure_update_tail<R>(k, s, c, dt, v3<R>(R(0), R(0), R(0)), R(0), vs, aii, R(0));
 }
 
-// block reduction of the ErrParts into StepScalars (FP64 residual sum); every
-// thread of the block calls it. scene: the scene of the thread's particle.
-// A block whose threads all belong to one scene reduces first; a block that
-// spans scenes adds thread by thread.
-__device__ __forceinline__ void reduce_err_parts(ErrPart o, StepScalars* FSB_R sc, int scene = 0) {
-    __shared__ int s_scene;
-    if (threadIdx.x == 0) s_scene = scene;
-    __syncthreads();
-    const int s0 = s_scene;
-    if (!__syncthreads_and(scene == s0)) {
-        add_err_part(o, sc + scene);
-        return;
-    }
-    sc += s0;
+// one set of an iteration's accumulators
+struct ErrSet {
+    double* err_sum;
+    unsigned long long* err_count;
+    unsigned int *max_err_bits, *max_a2_bits, *max_v2_bits;
+};
+// block reduction of the ErrParts of one scene into q; every thread of the block calls it
+__device__ __forceinline__ void reduce_err_parts_to(const ErrPart& o, const ErrSet& q) {
     double e_sum = warp_sum(o.e_sum);
     unsigned int e_cnt = warp_sum(o.e_cnt);
     float e_max = warp_max(o.e_max), a2 = warp_max(o.a2), v2 = warp_max(o.v2);
@@ -451,14 +445,31 @@ __device__ __forceinline__ void reduce_err_parts(ErrPart o, StepScalars* FSB_R s
         v2 = warp_max(v2);
         if (lane == 0) {
             if (e_cnt) {
-                atomicAdd(&sc->err_sum, e_sum);
-                atomicAdd(&sc->err_count, (unsigned long long)e_cnt);
+                atomicAdd(q.err_sum, e_sum);
+                atomicAdd(q.err_count, (unsigned long long)e_cnt);
             }
-            atomic_max_nonneg(&sc->max_err_bits, e_max);
-            atomic_max_nonneg(&sc->max_a2_bits, a2);
-            atomic_max_nonneg(&sc->max_v2_bits, v2);
+            atomic_max_nonneg(q.max_err_bits, e_max);
+            atomic_max_nonneg(q.max_a2_bits, a2);
+            atomic_max_nonneg(q.max_v2_bits, v2);
         }
     }
+}
+
+// block reduction of the ErrParts into StepScalars (FP64 residual sum); every
+// thread of the block calls it. scene: the scene of the thread's particle.
+// A block whose threads all belong to one scene reduces first; a block that
+// spans scenes adds thread by thread.
+__device__ __forceinline__ void reduce_err_parts(ErrPart o, StepScalars* FSB_R sc, int scene = 0) {
+    __shared__ int s_scene;
+    if (threadIdx.x == 0) s_scene = scene;
+    __syncthreads();
+    const int s0 = s_scene;
+    if (!__syncthreads_and(scene == s0)) {
+        add_err_part(o, sc + scene);
+        return;
+    }
+    sc += s0;
+    reduce_err_parts_to(o, ErrSet{&sc->err_sum, &sc->err_count, &sc->max_err_bits, &sc->max_a2_bits, &sc->max_v2_bits});
 }
 
 template <typename R, bool KAHAN>

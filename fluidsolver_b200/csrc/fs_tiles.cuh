@@ -36,7 +36,8 @@ constexpr int kTileOwners = 128;
 constexpr int kPassThreads = 2 * kTileOwners;  // two threads per owner in the passes
 constexpr int kTileGroups = 4;
 constexpr int kTileRanges = 2 * 9 * kTileGroups;
-constexpr int kTileCap = 1536;                 // staged candidates per tile (default; fs_autotune may change it)
+constexpr int kTileCap = 1536;                 // staged candidates per tile of large scenes (tile_cap_of; fs_autotune may change it)
+constexpr int kTileCapSmall = 2048;            // and of small ones
 constexpr int kTileCapMax = 3072;              // the largest cap (entries address up to 4,096 staged candidates)
 constexpr uint32_t kTileFallback = 0xffffffffu;
 // entry: byte offset of the candidate's float4 in a staged array (index << 4),
@@ -127,16 +128,16 @@ struct TileStage {
     uint64_t bar;
 };
 
-// One try of the wait for phase 0: the thread sleeps until the phase
+// One try of the wait for the phase of the given parity: the thread sleeps until the phase
 // completes or kTileWaitHintNs pass (the try's time limit), so that waiting
 // warps issue no instructions while the copies land.
 constexpr uint32_t kTileWaitHintNs = 20000;
-__device__ __forceinline__ uint32_t mbar_try_wait0(TileStage& st) {
+__device__ __forceinline__ uint32_t mbar_try_wait(TileStage& st, uint32_t parity) {
     uint32_t ok;
     asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0, %2;\n selp.u32 %0, 1, 0, p;\n}"
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %3, %2;\n selp.u32 %0, 1, 0, p;\n}"
         : "=r"(ok)
-        : "r"(smem_u32(&st.bar)), "r"(kTileWaitHintNs)
+        : "r"(smem_u32(&st.bar)), "r"(kTileWaitHintNs), "r"(parity)
         : "memory");
     return ok;
 }
@@ -155,15 +156,16 @@ static __device__ int g_tile_wait_tries = kTileWaitTries;
 // (kTileDrainTries, independent of the first's limit) lets copies still in
 // flight land, so that none writes into shared memory after the block has
 // left it.
-__device__ __forceinline__ bool stage_tile_wait(TileStage& st, int* __restrict__ status) {
+// parity: the barrier's phase (0 for a block's first staging, then alternating).
+__device__ __forceinline__ bool stage_tile_wait(TileStage& st, int* __restrict__ status, uint32_t parity = 0u) {
     asm volatile("cp.async.wait_all;" ::: "memory");   // the packed layout's 4-byte copies
     uint32_t ok = 0;
     const int tries = g_tile_wait_tries;
-    for (int it = 0; it < tries && !ok; it++) ok = mbar_try_wait0(st);
+    for (int it = 0; it < tries && !ok; it++) ok = mbar_try_wait(st, parity);
     const int late = __syncthreads_or(!ok);
     if (late) {
         if (threadIdx.x == 0) raise_status(status, FS_ERR_TIMEOUT);
-        for (int it = 0; it < kTileDrainTries && !ok; it++) ok = mbar_try_wait0(st);
+        for (int it = 0; it < kTileDrainTries && !ok; it++) ok = mbar_try_wait(st, parity);
         __syncthreads();
         return false;
     }
@@ -612,10 +614,11 @@ __device__ __forceinline__ void walk_tile_list(const TileLists& T, const TileSla
 // Walks owner k's 32-bit list in a fallback tile, the entries of this
 // thread of the owner's TPO (half, half + TPO, ...): use(load(sorted index),
 // boundary) for each (the fluid entries only with FLUID_ONLY), flush() after
-// every 8 visits and at the end, as for_tile_entries does. BATCH entries' loads are in flight together: one at a time, an entry cost two
-// dependent trips to L2, and a fallback tile's acceleration pass took 14,000
-// cycles against 6,600 of a staged tile, which all blocks of a small scene
-// then waited for.
+// every 8 visits and at the end, as for_tile_entries does. BATCH entries'
+// loads are in flight together: one at a time, an entry cost two dependent
+// trips to L2, and a fallback tile's acceleration pass took 14,000 cycles
+// against 6,600 of a staged tile, which all blocks of a small scene then
+// waited for.
 constexpr int kFallbackBatch = 4;
 template <bool FLUID_ONLY, int TPO = 2, int BATCH = kFallbackBatch, typename Load, typename Use, typename Flush>
 __device__ __forceinline__ void walk_fallback_list(const Lists& L, int64_t k, int half, Load&& load, Use&& use,
@@ -693,21 +696,23 @@ __device__ __forceinline__ void prefetch_shares(const TileLists& T, const TileHe
         }
     }
 }
-// Visits this thread's share of owner k's fluid entries: f(byte offset into
-// a staged float4 array) for each, flush() after every 8 visits and at the
-// end. With TPO 2 the visits and flushes are those of for_tile_entries.
-template <int TPO, int AHEAD, typename F, typename Flush>
-__device__ __forceinline__ void walk_fluid_shares(const TileLists& T, int64_t k, uint32_t cnt, int part,
-                                                  OctetShare<TPO> (&ahead)[AHEAD], F&& f, Flush&& flush) {
+// Visits this thread's share of an owner's fluid entries (cnt: the packed list
+// length, K: the lists' capacity): f(byte offset into a staged float4 array)
+// for each, flush() after every 8 visits and at the end. load(o): the share of
+// octet o; ahead holds the first AHEAD. With TPO 2 the visits and flushes are
+// those of for_tile_entries.
+template <int TPO, int AHEAD, typename LoadShare, typename F, typename Flush>
+__device__ __forceinline__ void walk_shares(uint32_t cnt, int K, int part, OctetShare<TPO> (&ahead)[AHEAD],
+                                            LoadShare&& load, F&& f, Flush&& flush) {
     constexpr int W = 4 / TPO;
-    const uint32_t all = min(cnt & 0xffffu, (uint32_t)T.K);
+    const uint32_t all = min(cnt & 0xffffu, (uint32_t)K);
     const uint32_t n = min(cnt >> 16, all);
     const uint32_t full = n / 8, octets = (n + 7) / 8;
     for (uint32_t o = 0; o < full; o++) {
         const OctetShare<TPO> cur = ahead[0];
 #pragma unroll
         for (int d = 0; d + 1 < AHEAD; d++) ahead[d] = ahead[d + 1];
-        if (o + AHEAD < octets) ahead[AHEAD - 1] = load_share<TPO>(T.ent + k, T.stride, o + AHEAD, part);
+        if (o + AHEAD < octets) ahead[AHEAD - 1] = load(o + AHEAD);
 #pragma unroll
         for (int i = 0; i < W; i++) {
             f(cur.w[i] & 0xffffu);
@@ -726,6 +731,13 @@ __device__ __forceinline__ void walk_fluid_shares(const TileLists& T, int64_t k,
     }
     flush();
 }
+// from the global octet planes
+template <int TPO, int AHEAD, typename F, typename Flush>
+__device__ __forceinline__ void walk_fluid_shares(const TileLists& T, int64_t k, uint32_t cnt, int part,
+                                                  OctetShare<TPO> (&ahead)[AHEAD], F&& f, Flush&& flush) {
+    walk_shares<TPO, AHEAD>(cnt, T.K, part, ahead,
+                            [&](uint32_t o) { return load_share<TPO>(T.ent + k, T.stride, o, part); }, f, flush);
+}
 
 // Octets a pass loads ahead of the one it visits. The first loop's and the
 // pressure passes' depths are chosen per context by fs_autotune among
@@ -736,7 +748,7 @@ constexpr int kL2Ahead = 1;
 struct TileTuning {
     int l1_ahead = 1;
     int pressure_ahead = 3;
-    int cap = kTileCap;   // staged candidates per tile
+    int cap = 0;          // staged candidates per tile (0: by the scene's size, tile_cap_of)
     int block = 128;      // threads per block of the step's per-particle kernels (keys, reorder, integration)
     int pressure_tpo = 2; // threads per owner in the pressure passes (1, 2, 4)
 };
@@ -1002,6 +1014,97 @@ template <int TPO> constexpr int pressure_threads() { return kTileOwners * TPO; 
 template <int TPO> constexpr int acc_blocks_per_sm() { return TPO == 1 ? 6 : (TPO == 2 ? 5 : 2); }
 template <int TPO> constexpr int update_blocks_per_sm() { return TPO == 1 ? 4 : (TPO == 2 ? 4 : 2); }
 
+// The neighbor sums of one owner in the pressure passes, over its staged
+// candidates or its 32-bit list in a fallback tile; every thread of the owner
+// calls and gets the total. COHERENT: the neighbors' fields are written by
+// other blocks of the same launch, so a fallback list reads them past L1.
+template <bool COHERENT, typename T> __device__ __forceinline__ T neighbor_load(const T* p) {
+    return COHERENT ? __ldcg(p) : *p;
+}
+struct AccSum {
+    Acc3<float, true> pa;
+    V3<float> part = v3<float>(0.f, 0.f, 0.f);
+    float4 pk;
+    float prk;
+    const FastSpline& S;
+    __device__ __forceinline__ AccSum(const float4& x, float p, const FastSpline& spline) : pk(x), prk(p), S(spline) {}
+    __device__ __forceinline__ void pair(const float4& pj, float prj) {
+        const V3<float> xij = sub3(pk, pj);
+        const float coef = pj.w * (prk + prj) * S.grad(r2_of(xij));
+        part = fma3(-coef, xij, part);
+    }
+    __device__ __forceinline__ void flush() {
+        pa.add(part);
+        part = v3<float>(0.f, 0.f, 0.f);
+    }
+};
+template <int AHEAD, int TPO>
+__device__ __forceinline__ V3<float> acc_sum_tiled(const TileLists& T, int64_t k, uint32_t cnt, int part, bool valid,
+                                                   OctetShare<TPO> (&ahead)[AHEAD], const float4* sp, const float* sa,
+                                                   const float4& pk, float prk, const FastSpline& S) {
+    AccSum q(pk, prk, S);
+    if (valid)
+        walk_fluid_shares<TPO, AHEAD>(T, k, cnt, part, ahead, [&](uint32_t off) {
+            q.pair(at_offset(sp, off), at_offset(sa, off >> 2));
+        }, [&] { q.flush(); });
+    return pair_total<TPO>(q.pa);
+}
+template <int TPO, bool COHERENT = false>
+__device__ __forceinline__ V3<float> acc_sum_fallback(const Lists& L, int64_t k, int part, bool valid,
+                                                      const State<float>& s, const float4& pk, float prk,
+                                                      const FastSpline& S) {
+    AccSum q(pk, prk, S);
+    if (valid)
+        walk_fallback_list<true, TPO>(L, k, part, [&](uint32_t j) {
+            return Neighbor1{s.pos[j], neighbor_load<COHERENT>(s.p + j)};
+        }, [&](const Neighbor1& n, bool) { q.pair(n.pos, n.f); }, [&] { q.flush(); });
+    return pair_total<TPO>(q.pa);
+}
+// boundary: - sum_bnd (lambda m_j p_i / rho0^2) gradW, lambda = 2 gamma (single layer) or 2
+__device__ __forceinline__ float4 pressure_acc_of(const SolverConsts<float>& c, V3<float> a, float prk,
+                                                  const float4& gbk) {
+    const float wb = (c.single_layer ? c.two_gamma : 2.f) * prk;
+    return v4<float>(c.inv_rho0_sq * (a - wb * v3<float>(gbk.x, gbk.y, gbk.z)), 0.f);
+}
+struct UpdateSum {
+    Acc<float, true> ap;
+    float part = 0.f;
+    float4 pk, ak;
+    const FastSpline& S;
+    __device__ __forceinline__ UpdateSum(const float4& x, const float4& a, const FastSpline& spline)
+        : pk(x), ak(a), S(spline) {}
+    __device__ __forceinline__ void pair(const float4& pj, const float4& aj) {
+        const V3<float> xij = sub3(pk, pj);
+        part = __fmaf_rn(pj.w * S.grad(r2_of(xij)), dot3(sub3(ak, aj), xij), part);
+    }
+    __device__ __forceinline__ void flush() {
+        ap.add(part);
+        part = 0.f;
+    }
+};
+template <int AHEAD, int TPO>
+__device__ __forceinline__ float update_sum_tiled(const TileLists& T, int64_t k, uint32_t cnt, int part, bool valid,
+                                                  OctetShare<TPO> (&ahead)[AHEAD], const float4* sp, const float4* sa,
+                                                  const float4& pk, const float4& ak, const FastSpline& S) {
+    UpdateSum q(pk, ak, S);
+    if (valid)
+        walk_fluid_shares<TPO, AHEAD>(T, k, cnt, part, ahead, [&](uint32_t off) {
+            q.pair(at_offset(sp, off), at_offset(sa, off));
+        }, [&] { q.flush(); });
+    return pair_total<TPO>(q.ap);
+}
+template <int TPO, bool COHERENT = false>
+__device__ __forceinline__ float update_sum_fallback(const Lists& L, int64_t k, int part, bool valid,
+                                                     const State<float>& s, const float4& pk, const float4& ak,
+                                                     const FastSpline& S) {
+    UpdateSum q(pk, ak, S);
+    if (valid)
+        walk_fallback_list<true, TPO>(L, k, part, [&](uint32_t j) {
+            return Neighbor4{s.pos[j], neighbor_load<COHERENT>(s.acc + j)};
+        }, [&](const Neighbor4& n, bool) { q.pair(n.pos, n.v); }, [&] { q.flush(); });
+    return pair_total<TPO>(q.ap);
+}
+
 // iteration (a): pressure acceleration
 template <int AHEAD, int TPO>
 __global__ void __launch_bounds__(pressure_threads<TPO>(), acc_blocks_per_sm<TPO>()) k_tile_iisph3d_pressure_acc(
@@ -1025,24 +1128,11 @@ __global__ void __launch_bounds__(pressure_threads<TPO>(), acc_blocks_per_sm<TPO
     const float4 pk = s.pos[kk], gbk = s.gbnd[kk];
     const float prk = s.p[kk];
     const FastSpline S(c.kern);
-    Acc3<float, true> pa;
-    V3<float> part = v3<float>(0.f, 0.f, 0.f);
-    auto pair = [&](const float4& pj, float prj) {
-        const V3<float> xij = sub3(pk, pj);
-        const float coef = pj.w * (prk + prj) * S.grad(r2_of(xij));
-        part = fma3(-coef, xij, part);
-    };
-    auto flush = [&] {
-        pa.add(part);
-        part = v3<float>(0.f, 0.f, 0.f);
-    };
+    V3<float> a;
     // boundary neighbors enter through sum_bnd m_j gradW (second loop), so
     // only the fluid candidates and entries are visited
     if (h.nranges == kTileFallback) {
-        // the owner's 32-bit list, split between its threads
-        if (valid)
-            walk_fallback_list<true, TPO>(L, k, half, [&](uint32_t j) { return Neighbor1{s.pos[j], s.p[j]}; },
-                                          [&](const Neighbor1& n, bool) { pair(n.pos, n.f); }, flush);
+        a = acc_sum_fallback<TPO>(L, k, half, valid, s, pk, prk, S);
     } else {
         float4* sp = tile_smem;
         float* sa = reinterpret_cast<float*>(tile_smem + T.cap);
@@ -1055,16 +1145,10 @@ __global__ void __launch_bounds__(pressure_threads<TPO>(), acc_blocks_per_sm<TPO
         OctetShare<TPO> ahead[AHEAD];
         prefetch_shares<TPO, AHEAD>(T, h, k, half, ahead);
         if (!stage_tile_wait(stg, status)) return;
-        if (valid)
-            walk_fluid_shares<TPO, AHEAD>(T, k, cnt, half, ahead, [&](uint32_t off) {
-                pair(at_offset(sp, off), at_offset(sa, off >> 2));
-            }, flush);
+        a = acc_sum_tiled<AHEAD, TPO>(T, k, cnt, half, valid, ahead, sp, sa, pk, prk, S);
     }
-    const V3<float> a = pair_total<TPO>(pa);
     if (half || !valid) return;
-    // boundary: - sum_bnd (lambda m_j p_i / rho0^2) gradW, lambda = 2 gamma (single layer) or 2
-    const float wb = (c.single_layer ? c.two_gamma : 2.f) * prk;
-    s.acc[k] = v4<float>(c.inv_rho0_sq * (a - wb * v3<float>(gbk.x, gbk.y, gbk.z)), 0.f);
+    s.acc[k] = pressure_acc_of(c, a, prk, gbk);
 }
 
 // iteration (b): A p, relaxed Jacobi update, density error, fused scan.
@@ -1097,23 +1181,11 @@ __global__ void __launch_bounds__(pressure_threads<TPO>(), update_blocks_per_sm<
     grid_dependency_wait();   // the accelerations of this iteration
     const float4 ak = s.acc[kk];
     const FastSpline S(c.kern);
-    Acc<float, true> ap;
-    float part = 0.f;
-    auto pair = [&](const float4& pj, const float4& aj) {
-        const V3<float> xij = sub3(pk, pj);
-        part = __fmaf_rn(pj.w * S.grad(r2_of(xij)), dot3(sub3(ak, aj), xij), part);
-    };
-    auto flush = [&] {
-        ap.add(part);
-        part = 0.f;
-    };
     // boundary neighbors enter through sum_bnd m_j gradW (second loop)
     bool done = true;
+    float ap = 0.f;
     if (h.nranges == kTileFallback) {
-        // the owner's 32-bit list, split between its threads
-        if (valid)
-            walk_fallback_list<true, TPO>(L, k, half, [&](uint32_t j) { return Neighbor4{s.pos[j], s.acc[j]}; },
-                                          [&](const Neighbor4& n, bool) { pair(n.pos, n.v); }, flush);
+        ap = update_sum_fallback<TPO>(L, k, half, valid, s, pk, ak, S);
     } else {
         float4* sp = tile_smem;
         float4* sa = tile_smem + T.cap;
@@ -1125,18 +1197,353 @@ __global__ void __launch_bounds__(pressure_threads<TPO>(), update_blocks_per_sm<
         OctetShare<TPO> ahead[AHEAD];
         prefetch_shares<TPO, AHEAD>(T, h, k, half, ahead);
         done = stage_tile_wait(stg, status);
-        if (done && valid)
-            walk_fluid_shares<TPO, AHEAD>(T, k, cnt, half, ahead, [&](uint32_t off) {
-                pair(at_offset(sp, off), at_offset(sa, off));
-            }, flush);
+        if (done) ap = update_sum_tiled<AHEAD, TPO>(T, k, cnt, half, valid, ahead, sp, sa, pk, ak, S);
     }
     if (done) {
         // boundary: sum_bnd m_j dot(a_i, gradW) = dot(a_i, sum_bnd m_j gradW)
-        const float sum = pair_total<TPO>(ap) + dot3(v3<float>(ak.x, ak.y, ak.z), v3<float>(gbk.x, gbk.y, gbk.z));
+        const float sum = ap + dot3(v3<float>(ak.x, ak.y, ak.z), v3<float>(gbk.x, gbk.y, gbk.z));
         if (!half && valid)
             o = iisph3d_pressure_update_tail<float>(k, s, c, dt, v3<float>(ak.x, ak.y, ak.z), sum, vsk, aii, prk);
     }
     reduce_err_parts(o, sc, scene);
+}
+
+// ---------------------------------------------------------------------------
+// The pressure iterations after the first, the convergence test and the CFL
+// clamp of a single scene in one cooperative launch.
+//
+// As a graph, an iteration is three launches and a turn of the WHILE node.
+// Here one grid of resident blocks runs all iterations. A grid barrier
+// follows each pass; every block then evaluates the test itself from the
+// iteration's accumulators, which alternate between two sets, so the test
+// needs no barrier of its own. The sums are those of the two passes above, in
+// their order. Two forms:
+//   ONE   a block per tile, up to 3 blocks per SM (444 tiles): the tile's
+//         positions and entries stay in shared memory and its owners' constants
+//         in registers through the loop, so that a pass copies pressures or
+//         accelerations and nothing else;
+//   else  a block stages its tiles one after the other in every pass.
+//
+// Measured on a B200, one iteration of a dam's loop, the WHILE node against this:
+// 512 fluid particles 17.0 -> 12.6 us, 8,000 16.4 -> 11.9, 29,791 18.8 -> 13.9,
+// 100,000 34.6 -> 28.9, 250,047 65.5 -> 60.9, 512,000 115 -> 110. A pass of a
+// small scene is a chain of latencies (copying the field 0.7 us, the walk 1.4,
+// the barrier 1.7), and the fallback tiles' are the longest.
+//
+// Accelerations and pressures cross blocks within the launch: the barrier
+// releases and acquires at GPU scope, fence.proxy.async orders them before the
+// bulk copies, and everything else that another block wrote is read past L1.
+// ---------------------------------------------------------------------------
+constexpr int kLoopAhead = 3;
+constexpr int kLoopBlocksPerSm = 4, kLoopOneBlocksPerSm = 3;
+constexpr int kLoopBarrierTries = 1 << 22;   // polls of a grid barrier (each about 0.4 us) before it gives up
+
+struct LoopTest {
+    int min_it, max_it;
+    float max_err;
+    float particle_size, cfl_timestep, lambda_v, lambda_a;
+};
+
+// Waits until `target` blocks have arrived at the launch's barriers in all
+// (every block adds 1 per barrier). False, in every thread, when the wait ran
+// out (FS_ERR_TIMEOUT raised) or another block failed.
+__device__ __forceinline__ bool loop_barrier(unsigned int* arrived, unsigned int target, int* status) {
+    // this thread's stores, before other blocks' bulk copies (the release and
+    // the block barrier before it order them for the other blocks' loads)
+    asm volatile("fence.proxy.async.global;" ::: "memory");
+    __syncthreads();
+    int failed = 0;
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
+        int tries = 0;
+        while (true) {
+            // (polled relaxed: an acquire per poll would empty L1 each time)
+            unsigned int v;
+            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
+            if ((int)(v - target) >= 0) break;
+            if ((++tries & 63) == 0) {
+                if (*(volatile int*)status) {
+                    failed = 1;
+                    break;
+                }
+                if (tries > kLoopBarrierTries) {
+                    raise_status(status, FS_ERR_TIMEOUT);
+                    failed = 1;
+                    break;
+                }
+            }
+        }
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    }
+    failed = __syncthreads_or(failed);
+    asm volatile("fence.proxy.async.global;" ::: "memory");
+    return !failed;
+}
+
+// The bytes that stage_loop_field's bulk copies add for a tile
+__device__ __forceinline__ uint32_t loop_field_bytes(const TileHead& h, int float4_arrays, bool float_array) {
+    return h.staged_fluid * 16u * (uint32_t)float4_arrays + (float_array ? h.slots_fluid * 4u : 0u);   // slots 0: packed
+}
+__device__ __forceinline__ void loop_expect(TileStage& stg, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&stg.bar)), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void loop_bulk(TileStage& stg, const void* dst, const void* src, uint32_t bytes) {
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+        "l"(src), "r"(bytes), "r"(smem_u32(&stg.bar))
+        : "memory");
+}
+// One field of the tile's fluid candidate ranges into shared memory: a float4
+// array, or a float array (through plain loads past L1 in the packed layout)
+__device__ __forceinline__ void stage_loop_field(TileStage& stg, const TileHead& h, const TileRange& rg,
+                                                 const float4* src, float4* dst) {
+    if (threadIdx.x < h.nranges && !(rg.len_base & kRangeBoundary))
+        loop_bulk(stg, dst + (rg.len_base >> 16), src + rg.start, (rg.len_base & kRangeLen) * 16u);
+}
+__device__ __forceinline__ void stage_loop_field(TileStage& stg, const TileDesc* __restrict__ d, const TileHead& h,
+                                                 const TileRange& rg, const float* src, float* dst) {
+    if (h.slots) {
+        if (threadIdx.x < h.nranges && !(rg.len_base & kRangeBoundary)) {
+            const uint32_t a = rg.start, len = rg.len_base & kRangeLen, base = rg.len_base >> 16;
+            loop_bulk(stg, dst + (base - (a & 3u)), src + (a & ~3u), padded_slots(a, len) * 4u);
+        }
+        return;
+    }
+    const int lane = threadIdx.x & 31;
+    for (uint32_t q = threadIdx.x >> 5; q < h.nranges; q += blockDim.x / 32) {
+        const uint32_t a = d->start[q], lb = d->len_base[q];
+        if (lb & kRangeBoundary) continue;
+        const uint32_t len = lb & kRangeLen, base = lb >> 16;
+        for (uint32_t i = lane; i < len; i += 32) dst[base + i] = __ldcg(src + a + i);
+    }
+}
+
+// The test of iteration `it` from its accumulators (check_scene's, with the
+// FP64 average); thread 0 of every block calls it. When the loop ends, block 0
+// stores the results and clamps the time step; else it clears the set of
+// iteration it - 1, which every block has read, for iteration it + 1.
+__device__ __forceinline__ bool loop_test(int it, const LoopTest& lt, StepScalars* __restrict__ sc) {
+    volatile StepScalars* v = sc;
+    const bool even = (it & 1) == 0;
+    const unsigned long long cnt = even ? v->err_count_odd : v->err_count;
+    const double sum = even ? v->err_sum_odd : v->err_sum;
+    const double avg = cnt > 0 ? sum / (double)cnt : 0.0;
+    const bool done = (lt.min_it >= 1 && it >= lt.min_it && avg <= (double)lt.max_err) || it >= lt.max_it;
+    if (blockIdx.x != 0) return done;
+    if (done) {
+        sc->avg_err = (float)avg;
+        sc->avg_err64 = avg;
+        sc->max_err = __uint_as_float(even ? v->max_err_bits_odd : v->max_err_bits);
+        sc->final_max_a2 = __uint_as_float(even ? v->max_a2_bits_odd : v->max_a2_bits);
+        sc->final_max_v2 = __uint_as_float(even ? v->max_v2_bits_odd : v->max_v2_bits);
+        sc->iteration = it;
+        sc->done = 1;
+        cfl_one(sc, lt.particle_size, lt.cfl_timestep, lt.lambda_v, lt.lambda_a);
+    } else if (it >= 2) {
+        if (even) {
+            v->err_sum = 0.0;
+            v->err_count = 0ull;
+            v->max_err_bits = v->max_a2_bits = v->max_v2_bits = 0u;
+        } else {
+            v->err_sum_odd = 0.0;
+            v->err_count_odd = 0ull;
+            v->max_err_bits_odd = v->max_a2_bits_odd = v->max_v2_bits_odd = 0u;
+        }
+    }
+    return done;
+}
+// the accumulators of iteration it + 1
+__device__ __forceinline__ ErrSet loop_err_set(int it, StepScalars* sc) {
+    return (it & 1) == 0 ? ErrSet{&sc->err_sum, &sc->err_count, &sc->max_err_bits, &sc->max_a2_bits, &sc->max_v2_bits}
+                         : ErrSet{&sc->err_sum_odd, &sc->err_count_odd, &sc->max_err_bits_odd, &sc->max_a2_bits_odd,
+                                  &sc->max_v2_bits_odd};
+}
+
+// dynamic shared memory of the loop: positions and the pass's field, and for
+// ONE the tile's entries
+constexpr size_t kLoopSmemMax = 225 * 1024;   // a block's dynamic shared memory at most, beside its static part
+inline size_t tile_loop_smem(bool one, int K, int cap) {
+    return tile_pass_smem(32, K, false, cap) + (one ? (size_t)(K / 8) * kTileOwners * 16 : 0);
+}
+
+template <bool ONE>
+__global__ void __launch_bounds__(kPassThreads, ONE ? kLoopOneBlocksPerSm : kLoopBlocksPerSm)
+    k_tile_iisph3d_pressure_loop(int64_t n_fluid, int64_t tiles, State<float> s, TileLists T, Lists L,
+                                 SolverConsts<float> c, LoopTest lt, StepScalars* __restrict__ sc,
+                                 int* __restrict__ status) {
+    extern __shared__ float4 tile_smem[];
+    __shared__ TileStage stg;
+    __shared__ int s_done;
+    float4* sp = tile_smem;
+    float4* sa = tile_smem + T.cap;
+    float* s1 = reinterpret_cast<float*>(sa);
+    const int half = threadIdx.x & 1;
+    const int err = *(volatile int*)status;
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&stg.bar)) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (__syncthreads_or(err)) return;
+    uint32_t parity = 0u;
+    unsigned int barriers = 0;
+    const float dt = sc->dt;
+    const FastSpline S(c.kern);
+    int it = 1;   // iterations done: the second loop ran the first
+    if constexpr (ONE) {
+        const uint4* ent = reinterpret_cast<const uint4*>(tile_smem + 2 * T.cap) + (threadIdx.x >> 1);
+        const TileDesc* d = T.desc + blockIdx.x;
+        const TileHead h = load_head(d);
+        const TileRange rg = load_range(d, threadIdx.x);
+        const int64_t k = blockIdx.x * (int64_t)kTileOwners + (threadIdx.x >> 1);
+        const bool valid = k < n_fluid, tiled = h.nranges != kTileFallback;
+        const int64_t kk = valid ? k : 0;
+        const float4 pk = s.pos[kk], gbk = s.gbnd[kk], vsk = s.vstar[kk];
+        const uint32_t cnt = T.count[kk];
+        auto share = [&](uint32_t o) {
+            const uint2 v = reinterpret_cast<const uint2*>(ent + o * kTileOwners)[half];
+            return OctetShare<2>{{v.x, v.y}};
+        };
+        if (tiled) {   // positions and entries, completed with the first pass's pressures
+            stage_loop_field(stg, h, rg, s.pos, sp);
+            if (threadIdx.x < h.octets)
+                loop_bulk(stg, tile_smem + 2 * T.cap + threadIdx.x * kTileOwners,
+                          T.ent + threadIdx.x * T.stride + blockIdx.x * (int64_t)kTileOwners, kTileOwners * 16u);
+        }
+        uint32_t first = tiled ? loop_field_bytes(h, 1, false) + h.octets * (kTileOwners * 16u) : 0u;
+        for (;; it++) {
+            // accelerations; the pressures are on their way while the test of the last iteration runs
+            if (tiled) {
+                if (threadIdx.x == 0) loop_expect(stg, first + loop_field_bytes(h, 0, true));
+                first = 0u;
+                stage_loop_field(stg, d, h, rg, s.p, s1);
+            }
+            const float prk = __ldcg(s.p + kk);
+            if (threadIdx.x == 0) s_done = loop_test(it, lt, sc);
+            if (tiled) {
+                const bool ok = stage_tile_wait(stg, status, parity);
+                parity ^= 1u;
+                if (!ok) return;
+            } else {
+                __syncthreads();
+            }
+            if (s_done) return;
+            V3<float> a;
+            if (tiled) {
+                AccSum q(pk, prk, S);
+                OctetShare<2> ahead[1] = {share(0)};
+                if (valid)
+                    walk_shares<2, 1>(cnt, T.K, half, ahead, share, [&](uint32_t off) {
+                        q.pair(at_offset(sp, off), at_offset(s1, off >> 2));
+                    }, [&] { q.flush(); });
+                a = pair_total<2>(q.pa);
+            } else {
+                a = acc_sum_fallback<2, true>(L, k, half, valid, s, pk, prk, S);
+            }
+            const float4 ak = pressure_acc_of(c, a, prk, gbk);
+            if (!half && valid) s.acc[k] = ak;
+            if (!loop_barrier(&sc->loop_arrived, ++barriers * gridDim.x, status)) return;
+            // update
+            float sum;
+            if (tiled) {
+                if (threadIdx.x == 0) loop_expect(stg, loop_field_bytes(h, 1, false));
+                stage_loop_field(stg, h, rg, s.acc, sa);
+                const bool ok = stage_tile_wait(stg, status, parity);
+                parity ^= 1u;
+                if (!ok) return;
+                UpdateSum q(pk, ak, S);
+                OctetShare<2> ahead[1] = {share(0)};
+                if (valid)
+                    walk_shares<2, 1>(cnt, T.K, half, ahead, share, [&](uint32_t off) {
+                        q.pair(at_offset(sp, off), at_offset(sa, off));
+                    }, [&] { q.flush(); });
+                sum = pair_total<2>(q.ap);
+            } else {
+                sum = update_sum_fallback<2, true>(L, k, half, valid, s, pk, ak, S);
+            }
+            sum += dot3(v3<float>(ak.x, ak.y, ak.z), v3<float>(gbk.x, gbk.y, gbk.z));
+            ErrPart o;
+            if (!half && valid)
+                o = iisph3d_pressure_update_tail<float>(k, s, c, dt, v3<float>(ak.x, ak.y, ak.z), sum, vsk, gbk.w, prk);
+            reduce_err_parts_to(o, loop_err_set(it, sc));
+            if (!loop_barrier(&sc->loop_arrived, ++barriers * gridDim.x, status)) return;
+        }
+    } else {
+        for (;; it++) {
+            if (threadIdx.x == 0) s_done = loop_test(it, lt, sc);
+            __syncthreads();
+            if (s_done) return;
+            // accelerations
+            for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+                const TileDesc* d = T.desc + tile;
+                const TileHead h = load_head(d);
+                const int64_t k = tile * kTileOwners + (threadIdx.x >> 1);
+                const bool valid = k < n_fluid;
+                const int64_t kk = valid ? k : 0;
+                const float4 pk = s.pos[kk], gbk = s.gbnd[kk];
+                const float prk = __ldcg(s.p + kk);
+                V3<float> a;
+                if (h.nranges == kTileFallback) {
+                    a = acc_sum_fallback<2, true>(L, k, half, valid, s, pk, prk, S);
+                } else {
+                    const TileRange rg = load_range(d, threadIdx.x);
+                    if (threadIdx.x == 0) loop_expect(stg, loop_field_bytes(h, 1, true));
+                    stage_loop_field(stg, h, rg, s.pos, sp);
+                    stage_loop_field(stg, d, h, rg, s.p, s1);
+                    const uint32_t cnt = T.count[kk];
+                    OctetShare<2> ahead[kLoopAhead];
+                    prefetch_shares<2, kLoopAhead>(T, h, k, half, ahead);
+                    const bool ok = stage_tile_wait(stg, status, parity);
+                    parity ^= 1u;
+                    if (!ok) return;
+                    a = acc_sum_tiled<kLoopAhead, 2>(T, k, cnt, half, valid, ahead, sp, s1, pk, prk, S);
+                    __syncthreads();   // the staged fields have been read
+                }
+                if (!half && valid) s.acc[k] = pressure_acc_of(c, a, prk, gbk);
+            }
+            if (!loop_barrier(&sc->loop_arrived, ++barriers * gridDim.x, status)) return;
+            // update
+            ErrPart o;
+            for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+                const TileDesc* d = T.desc + tile;
+                const TileHead h = load_head(d);
+                const int64_t k = tile * kTileOwners + (threadIdx.x >> 1);
+                const bool valid = k < n_fluid;
+                const int64_t kk = valid ? k : 0;
+                const float4 pk = s.pos[kk], gbk = s.gbnd[kk];
+                const float4 ak = __ldcg(s.acc + kk);
+                float sum;
+                if (h.nranges == kTileFallback) {
+                    sum = update_sum_fallback<2, true>(L, k, half, valid, s, pk, ak, S);
+                } else {
+                    const TileRange rg = load_range(d, threadIdx.x);
+                    if (threadIdx.x == 0) loop_expect(stg, loop_field_bytes(h, 2, false));
+                    stage_loop_field(stg, h, rg, s.pos, sp);
+                    stage_loop_field(stg, h, rg, s.acc, sa);
+                    const uint32_t cnt = T.count[kk];
+                    OctetShare<2> ahead[kLoopAhead];
+                    prefetch_shares<2, kLoopAhead>(T, h, k, half, ahead);
+                    const bool ok = stage_tile_wait(stg, status, parity);
+                    parity ^= 1u;
+                    if (!ok) return;
+                    sum = update_sum_tiled<kLoopAhead, 2>(T, k, cnt, half, valid, ahead, sp, sa, pk, ak, S);
+                    __syncthreads();   // the staged fields have been read
+                }
+                sum += dot3(v3<float>(ak.x, ak.y, ak.z), v3<float>(gbk.x, gbk.y, gbk.z));
+                if (!half && valid) {
+                    const ErrPart q = iisph3d_pressure_update_tail<float>(k, s, c, dt, v3<float>(ak.x, ak.y, ak.z), sum,
+                                                                          s.vstar[kk], gbk.w, __ldcg(s.p + kk));
+                    o.e_sum += q.e_sum;
+                    o.e_cnt += q.e_cnt;
+                    o.e_max = fmaxf(o.e_max, q.e_max);
+                    o.a2 = fmaxf(o.a2, q.a2);
+                    o.v2 = fmaxf(o.v2, q.v2);
+                }
+            }
+            reduce_err_parts_to(o, loop_err_set(it, sc));
+            if (!loop_barrier(&sc->loop_arrived, ++barriers * gridDim.x, status)) return;
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1376,6 +1783,12 @@ template <int AHEAD> inline cudaError_t set_tuned_pass_smem(int K) {
 inline cudaError_t set_tile_pass_smem(int K) {
     cudaError_t e = cudaFuncSetAttribute(k_tile_iisph3d_l2, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)tile_pass_smem(32, K, !kL2GlobalEntries, kTileCapMax));
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_tile_iisph3d_pressure_loop<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)tile_loop_smem(false, K, kTileCapMax));
+    if (e == cudaSuccess)   // (the launch asks for no more than a block may have, pressure_loop_form)
+        e = cudaFuncSetAttribute(k_tile_iisph3d_pressure_loop<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)std::min<size_t>(tile_loop_smem(true, K, kTileCapMax), kLoopSmemMax));
     if (e == cudaSuccess) e = set_tuned_pass_smem<1>(K);
     if (e == cudaSuccess) e = set_tuned_pass_smem<2>(K);
     if (e == cudaSuccess) e = set_tuned_pass_smem<3>(K);
