@@ -17,6 +17,7 @@
 #include "fs_search.cuh"
 #include "fs_solvers.cuh"
 #include "fs_entities.cuh"
+#include "fs_gather.cuh"
 #include "fs_io.hpp"
 #include "fs_render.cuh"
 #include "fs_small.cuh"
@@ -1063,6 +1064,18 @@ fs_status step_iisph3d_tiled(fs_ctx* c, bool capture) {
     return FS_OK;
 }
 
+// Whether the gather phases take kGroup threads per owner (fs_gather.cuh):
+// below the size where one thread per owner fills the device. B200, one
+// against eight threads: 2D SESPH forces 18.4 -> 8.2 us at 2,500 fluid
+// particles, 20.5 -> 18.4 at 40,000, 22.6 -> 24.5 at 67,600 (3D, 50,000: 74 ->
+// 41); a 2D IISPH iteration 39 -> 22 at 2,500, 44 -> 48 at 25,600; a 3D one 60
+// -> 25 at 8,000, 66 -> 48 at 32,800, 77 -> 104 at 100,000, in FP64 83 -> 51 at
+// 20,700 and 93 -> 92 at 50,700.
+bool grouped(const fs_ctx* c) {
+    const int64_t most = c->prm.solver == FS_SOLVER_IISPH_2D ? 24576 : (c->prm.solver == FS_SOLVER_IISPH_3D ? 45056 : 65536);
+    return c->n_fluid <= most;
+}
+
 template <typename R, bool KAHAN> fs_status step_iisph3d(fs_ctx* c, bool capture) {
     if constexpr (std::is_same<R, float>::value && KAHAN) {
         if (tiled_mode(c) && c->n_owners > 0) return step_iisph3d_tiled(c, capture);
@@ -1076,8 +1089,17 @@ template <typename R, bool KAHAN> fs_status step_iisph3d(fs_ctx* c, bool capture
     // density double buffer: the current density becomes rho_prev
     std::swap(c->rho[c->cur], c->rho_prev);
     State<R> s = state_of<R>(c);
+    const bool group = grouped(c);
+    const unsigned gn = group_grid(n), go = group_grid(no);
     FS_TRY(mark(c, 1, st));
-    if (split) {
+    if (group && split) {
+        c->launches += 2;
+        k_group_iisph_density<R, KAHAN, true><<<gn, kGroupThreads, 0, st>>>(n, s, L, k, c->status);
+        k_group_iisph_l1<R, KAHAN, true, false><<<gn, kGroupThreads, 0, st>>>(n, s, L, k, c->scalars, c->status);
+    } else if (group) {
+        c->launches++;
+        k_group_iisph_l1<R, KAHAN, false, false><<<gn, kGroupThreads, 0, st>>>(n, s, L, k, c->scalars, c->status);
+    } else if (split) {
     c->launches++;
         k_iisph3d_density<R, KAHAN><<<grid_for(n), kBlock, 0, st>>>(n, s, L, k, c->status);
     c->launches++;
@@ -1088,7 +1110,11 @@ template <typename R, bool KAHAN> fs_status step_iisph3d(fs_ctx* c, bool capture
     }
     FS_CUDA(cudaGetLastError());
     FS_TRY(mark(c, 2, st));
-    if (fp32) {
+    if (group) {
+        c->launches++;
+        if (fp32) k_group_iisph3d_l2<R, KAHAN, true><<<go, kGroupThreads, 0, st>>>(no, s, L, k, c->scalars, c->status);
+        else k_group_iisph3d_l2<R, KAHAN, false><<<go, kGroupThreads, 0, st>>>(no, s, L, k, c->scalars, c->status);
+    } else if (fp32) {
     c->launches++;
         k_iisph3d_l2<R, KAHAN, true><<<grid_for(no), kBlock, 0, st>>>(no, s, L, k, c->scalars, c->status);
     } else {
@@ -1099,8 +1125,13 @@ template <typename R, bool KAHAN> fs_status step_iisph3d(fs_ctx* c, bool capture
     FS_TRY(mark(c, 3, st));
     FS_TRY(enqueue_pressure_loop(c, capture, false, !fp32, [&](cudaStream_t bs) {
         c->launches += 2;
-        k_iisph3d_pressure_acc<R, KAHAN><<<grid_for(no), kBlock, 0, bs>>>(no, s, L, k, c->scalars, c->status);
-        k_iisph3d_pressure_update<R, KAHAN><<<grid_for(no), kBlock, 0, bs>>>(no, s, L, k, c->scalars, c->status);
+        if (group) {
+            k_group_iisph3d_pressure_acc<R, KAHAN><<<go, kGroupThreads, 0, bs>>>(no, s, L, k, c->scalars, c->status);
+            k_group_iisph3d_pressure_update<R, KAHAN><<<go, kGroupThreads, 0, bs>>>(no, s, L, k, c->scalars, c->status);
+        } else {
+            k_iisph3d_pressure_acc<R, KAHAN><<<grid_for(no), kBlock, 0, bs>>>(no, s, L, k, c->scalars, c->status);
+            k_iisph3d_pressure_update<R, KAHAN><<<grid_for(no), kBlock, 0, bs>>>(no, s, L, k, c->scalars, c->status);
+        }
         return false;
     }));
     FS_TRY(mark(c, 4, st));
@@ -1161,10 +1192,14 @@ template <typename R, bool KAHAN> fs_status step_sesph(fs_ctx* c) {
     State<R> s = state_of<R>(c);
     FS_TRY(mark(c, 1, st));
     c->launches++;
-    k_sesph_density<R, KAHAN><<<grid_for(no), kBlock, 0, st>>>(no, s, L, k, c->status);
+    const bool group = grouped(c);
+    const unsigned go = group_grid(no);
+    if (group) k_group_sesph_density<R, KAHAN><<<go, kGroupThreads, 0, st>>>(no, s, L, k, c->status);
+    else k_sesph_density<R, KAHAN><<<grid_for(no), kBlock, 0, st>>>(no, s, L, k, c->status);
     FS_TRY(mark(c, 2, st));
     c->launches++;
-    k_sesph_accel<R, KAHAN><<<grid_for(no), kBlock, 0, st>>>(no, s, L, k, c->status);
+    if (group) k_group_sesph_accel<R, KAHAN><<<go, kGroupThreads, 0, st>>>(no, s, L, k, c->status);
+    else k_sesph_accel<R, KAHAN><<<grid_for(no), kBlock, 0, st>>>(no, s, L, k, c->status);
     FS_TRY(mark(c, 3, st));
     if (c->dim == 3) {
     c->launches++;
@@ -1191,8 +1226,17 @@ template <typename R, bool KAHAN> fs_status step_iisph2d(fs_ctx* c, bool capture
     const bool split = c->reference_order;
     std::swap(c->rho[c->cur], c->rho_prev);
     State<R> s = state_of<R>(c);
+    const bool group = grouped(c);
+    const unsigned gn = group_grid(n), go = group_grid(no);
     FS_TRY(mark(c, 1, st));
-    if (split) {
+    if (group && split) {
+        c->launches += 2;
+        k_group_iisph_density<R, KAHAN, false><<<gn, kGroupThreads, 0, st>>>(n, s, L, k, c->status);
+        k_group_iisph_l1<R, KAHAN, true, true><<<gn, kGroupThreads, 0, st>>>(n, s, L, k, c->scalars, c->status);
+    } else if (group) {
+        c->launches++;
+        k_group_iisph_l1<R, KAHAN, false, true><<<gn, kGroupThreads, 0, st>>>(n, s, L, k, c->scalars, c->status);
+    } else if (split) {
     c->launches++;
         k_iisph2d_density<R, KAHAN><<<grid_for(n), kBlock, 0, st>>>(n, s, L, k, c->status);
     c->launches++;
@@ -1203,14 +1247,20 @@ template <typename R, bool KAHAN> fs_status step_iisph2d(fs_ctx* c, bool capture
     }
     FS_TRY(mark(c, 2, st));
     c->launches++;
-    k_iisph2d_l2<R, KAHAN><<<grid_for(no), kBlock, 0, st>>>(no, s, L, k, c->scalars, c->status);
+    if (group) k_group_iisph2d_l2<R, KAHAN><<<go, kGroupThreads, 0, st>>>(no, s, L, k, c->scalars, c->status);
+    else k_iisph2d_l2<R, KAHAN><<<grid_for(no), kBlock, 0, st>>>(no, s, L, k, c->scalars, c->status);
     FS_CUDA(cudaGetLastError());
     FS_TRY(mark(c, 3, st));
     FS_TRY(enqueue_pressure_loop(c, capture, true, c->precision != FS_PRECISION_FP32,
                                  [&](cudaStream_t bs) {
         c->launches += 2;
-        k_iisph2d_pressure_acc<R, KAHAN><<<grid_for(no), kBlock, 0, bs>>>(no, s, L, k, c->scalars, c->status);
-        k_iisph2d_pressure_update<R, KAHAN><<<grid_for(no), kBlock, 0, bs>>>(no, s, L, k, c->scalars, c->status);
+        if (group) {
+            k_group_iisph2d_pressure_acc<R, KAHAN><<<go, kGroupThreads, 0, bs>>>(no, s, L, k, c->scalars, c->status);
+            k_group_iisph2d_pressure_update<R, KAHAN><<<go, kGroupThreads, 0, bs>>>(no, s, L, k, c->scalars, c->status);
+        } else {
+            k_iisph2d_pressure_acc<R, KAHAN><<<grid_for(no), kBlock, 0, bs>>>(no, s, L, k, c->scalars, c->status);
+            k_iisph2d_pressure_update<R, KAHAN><<<grid_for(no), kBlock, 0, bs>>>(no, s, L, k, c->scalars, c->status);
+        }
         return false;
     }));
     FS_TRY(mark(c, 4, st));

@@ -1,0 +1,531 @@
+// The gather phases of fs_solvers.cuh with kGroup threads per owner.
+//
+// With one thread per owner a phase is a serial chain: 20 to 33 neighbors, each
+// with gathers, a square root and divisions, on as few threads as there are
+// particles. 2,500 owners are 20 blocks of four warps, and a 2D SESPH force
+// pass took 20 us of which almost all was that chain's latency; at 100,000
+// owners the device was still a quarter busy. Here the threads of a group take
+// the list's entries kGroup at a time, a window of kWindow entries in flight
+// together, and write every entry's terms to shared memory; then one thread per
+// sum adds its terms in list order. So each sum is the one the single thread
+// forms, bit for bit, plain or compensated, and only its terms are computed
+// side by side. The formulas and their order are those of the functions in
+// fs_solvers.cuh (the reference lines stand there).
+//
+// With many owners the lanes that idle while one of them adds cost more than the
+// latency: fs_api.cu (grouped) has the sizes and both sides' times.
+#pragma once
+
+#include "fs_common.cuh"
+#include "fs_solvers.cuh"
+
+namespace fsb {
+
+constexpr int kGroup = 8;            // threads per owner
+constexpr int kWindow = 32;          // entries whose terms are in shared memory at a time
+constexpr int kGroupThreads = 128;   // 16 owners per block
+constexpr int kGroupsPerBlock = kGroupThreads / kGroup;
+
+inline unsigned group_grid(int64_t owners) {
+    const int64_t g = (owners + kGroupsPerBlock - 1) / kGroupsPerBlock;
+    return (unsigned)(g > 1 ? g : 1);
+}
+
+// one group's terms, a row per sum (rows start in different banks)
+template <typename R, int NC> struct alignas(16) GroupRows {
+    R v[NC][kWindow + 4];
+};
+
+template <int G = kGroup> __device__ __forceinline__ int group_lane() { return (int)(threadIdx.x & (G - 1)); }
+__device__ __forceinline__ int64_t group_owner() {
+    return blockIdx.x * (int64_t)kGroupsPerBlock + threadIdx.x / kGroup;
+}
+
+// Adds the terms of the first n entries of owner k's list to the sums: lane c
+// of the group holds sum c in acc. load(j): the fields of neighbor j;
+// term(entry, fields, t): the entry's NC terms, and which of them count: bit 0
+// for t[0 .. H), bit 1 for t[H .. NC). INTERLEAVED: two terms per entry of one
+// sum, t[0] then t[1], held by lane 0. Every thread of the warp calls it.
+template <int NC, int H, bool INTERLEAVED = false, typename R, bool KAHAN, typename Load, typename Term>
+__device__ __forceinline__ void group_sum(const Lists& L, int64_t k, uint32_t n, GroupRows<R, NC>& rows,
+                                          Acc<R, KAHAN>& acc, Load&& load, Term&& term) {
+    constexpr int kRounds = kWindow / kGroup;
+    const int g = group_lane();
+    const unsigned all = 0xffffffffu, shift = threadIdx.x & 31u & ~(unsigned)(kGroup - 1);
+    const uint32_t most = __reduce_max_sync(all, n);
+    for (uint32_t base = 0; base < most; base += kWindow) {
+        uint32_t e[kRounds];
+        decltype(load(0u)) d[kRounds];
+#pragma unroll
+        for (int r = 0; r < kRounds; r++) {
+            const uint32_t q = base + r * kGroup + g;
+            e[r] = q < n ? FSB_LDG(&L.nbr[(int64_t)q * L.stride + k]) : 0u;
+        }
+#pragma unroll
+        for (int r = 0; r < kRounds; r++) d[r] = load(e[r] & kIndexMask);
+        uint32_t lo = 0, hi = 0;
+#pragma unroll
+        for (int r = 0; r < kRounds; r++) {
+            R t[NC];
+            const unsigned ok = term(e[r], d[r], t);
+            const bool in = base + r * kGroup + g < n;
+#pragma unroll
+            for (int c = 0; c < NC; c++) rows.v[c][r * kGroup + g] = t[c];
+            constexpr unsigned kMask = (1u << kGroup) - 1u;
+            lo |= ((__ballot_sync(all, in && (ok & 1u)) >> shift) & kMask) << (r * kGroup);
+            if (H < NC) hi |= ((__ballot_sync(all, in && (ok & 2u)) >> shift) & kMask) << (r * kGroup);
+        }
+        __syncwarp();
+        if (g < (INTERLEAVED ? 1 : NC)) {
+            const R* row = rows.v[g];
+            const uint32_t mask = INTERLEAVED ? lo | hi : (H < NC && g >= H ? hi : lo);
+            const int m = 32 - __clz((int)mask);
+#pragma unroll 4
+            for (int i = 0; i < m; i++) {
+                if (INTERLEAVED) {
+                    if ((lo >> i) & 1u) acc.add(row[i]);
+                    if ((hi >> i) & 1u) acc.add(rows.v[NC - 1][i]);
+                } else {
+                    if ((mask >> i) & 1u) acc.add(row[i]);
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
+// sum c of the group, in every thread
+template <typename R, bool KAHAN> __device__ __forceinline__ R group_total(const Acc<R, KAHAN>& acc, int c) {
+    return __shfl_sync(0xffffffffu, acc.get(), c, kGroup);
+}
+template <typename R, bool KAHAN> __device__ __forceinline__ V3<R> group_total3(const Acc<R, KAHAN>& acc, int c) {
+    return v3<R>(group_total(acc, c), group_total(acc, c + 1), group_total(acc, c + 2));
+}
+
+// neighbor fields
+template <typename R> struct GPos {
+    V4<R> x;
+};
+template <typename R> struct GPosVec {
+    V4<R> x, v;
+};
+template <typename R> struct GPosScalar {
+    V4<R> x;
+    R a;
+};
+template <typename R> struct GVisc {
+    V4<R> x, v;
+    R rho;
+};
+template <typename R> struct GForce {
+    V4<R> x, v;
+    R rho, p;
+};
+
+// the viscosity term of neighbor (xj, vj, rj) without the factor 2 nu
+// (viscosity() in fs_solvers.cuh); false where the density is 0
+template <typename R, bool KAHAN>
+__device__ __forceinline__ bool viscosity_term(const SolverConsts<R>& c, V3<R> xij, V3<R> g, V3<R> vij, R m, R rj,
+                                               R* t) {
+    if (rj == R(0)) {
+        t[0] = t[1] = t[2] = R(0);
+        return false;
+    }
+    const R f = KAHAN ? fdiv<true>(m * dotf<true>(vij, xij), rj * (dotf<true>(xij, xij) + c.visc_eps))
+                      : (m / rj) * (dot(vij, xij) / (dot(xij, xij) + c.visc_eps));
+    const V3<R> v = f * g;
+    t[0] = v.x;
+    t[1] = v.y;
+    t[2] = v.z;
+    return true;
+}
+template <typename R> __device__ __forceinline__ void put3(R* t, V3<R> v) {
+    t[0] = v.x;
+    t[1] = v.y;
+    t[2] = v.z;
+}
+
+// ---------------------------------------------------------------------------
+// density sums: SESPH (with the pressure), IISPH 3D and 2D (split first loop)
+// ---------------------------------------------------------------------------
+// GAMMA: boundary neighbors weighted by gamma_1 in the single-layer model (3D)
+template <typename R, bool KAHAN, bool GAMMA>
+__device__ __forceinline__ R group_density(int64_t k, uint32_t n, V3<R> xk, const State<R>& s, const Lists& L,
+                                           const SolverConsts<R>& c, GroupRows<R, 1>& rows) {
+    Acc<R, KAHAN> acc;
+    group_sum<1, 1>(L, k, n, rows, acc, [&](uint32_t j) { return GPos<R>{s.pos[j]}; },
+                    [&](uint32_t e, const GPos<R>& d, R* t) {
+                        R m = d.x.w;
+                        if (GAMMA && c.single_layer && (e & kBoundaryBit)) m = m * c.gamma1;
+                        t[0] = m * c.kern.template w<KAHAN>(xk - xyz<R>(d.x));
+                        return 1u;
+                    });
+    return group_total(acc, 0);
+}
+
+template <typename R, bool KAHAN>
+__global__ void __launch_bounds__(kGroupThreads) k_group_sesph_density(int64_t n, State<R> s, Lists L,
+                                                                       SolverConsts<R> c, const int* FSB_R status) {
+    __shared__ GroupRows<R, 1> rows[kGroupsPerBlock];
+    if (*status) return;
+    const int64_t k = group_owner();
+    const bool fluid = k < n && s.type[k] == FS_TYPE_NORMAL;
+    const int64_t kk = fluid ? k : 0;
+    const R r = group_density<R, KAHAN, true>(kk, fluid ? L.size(kk) : 0u, xyz<R>(s.pos[kk]), s, L, c,
+                                              rows[threadIdx.x / kGroup]);
+    if (!fluid || group_lane() != 0) return;
+    s.rho[k] = r;
+    const R pr = c.stiffness * (r / c.rest_density - R(1));
+    s.p[k] = (pr < R(0)) ? R(0) : pr;
+}
+
+// the split first loop's density: 3D (IISPHFluidSolver3D) or 2D
+template <typename R, bool KAHAN, bool GAMMA>
+__global__ void __launch_bounds__(kGroupThreads) k_group_iisph_density(int64_t n, State<R> s, Lists L,
+                                                                       SolverConsts<R> c, const int* FSB_R status) {
+    __shared__ GroupRows<R, 1> rows[kGroupsPerBlock];
+    if (*status) return;
+    const int64_t k = group_owner();
+    const bool in = k < n, fluid = in && s.type[k] == FS_TYPE_NORMAL;
+    const int64_t kk = in ? k : 0;
+    const R r = group_density<R, KAHAN, GAMMA>(kk, fluid ? L.size(kk) : 0u, xyz<R>(s.pos[kk]), s, L, c,
+                                               rows[threadIdx.x / kGroup]);
+    if (in && group_lane() == 0) s.rho[k] = fluid ? r : s.rho_prev[k];
+}
+
+// ---------------------------------------------------------------------------
+// SESPH accelerations (sesph_accel_one)
+// ---------------------------------------------------------------------------
+template <typename R, bool KAHAN>
+__global__ void __launch_bounds__(kGroupThreads) k_group_sesph_accel(int64_t n, State<R> s, Lists L, SolverConsts<R> c,
+                                                                     const int* FSB_R status) {
+    __shared__ GroupRows<R, 6> rows[kGroupsPerBlock];
+    if (*status) return;
+    const int64_t k = group_owner();
+    const bool fluid = k < n && s.type[k] == FS_TYPE_NORMAL;
+    const int64_t kk = fluid ? k : 0;
+    const V4<R> pk = s.pos[kk];
+    const V3<R> xk = xyz<R>(pk), vk = xyz<R>(s.vel[kk]);
+    const R rk = s.rho[kk];
+    const R pdd = rk == R(0) ? R(0) : s.p[kk] / (rk * rk);
+    Acc<R, KAHAN> acc;   // viscosity 0-2, pressure 3-5
+    group_sum<6, 3>(L, kk, fluid ? L.size(kk) : 0u, rows[threadIdx.x / kGroup], acc,
+                    [&](uint32_t j) { return GForce<R>{s.pos[j], s.vel[j], s.rho[j], s.p[j]}; },
+                    [&](uint32_t e, const GForce<R>& d, R* t) {
+                        const V3<R> xij = xk - xyz<R>(d.x);
+                        const V3<R> g = c.kern.template grad<KAHAN>(xij);
+                        const bool visc = viscosity_term<R, KAHAN>(c, xij, g, vk - xyz<R>(d.v), d.x.w, d.rho, t);
+                        V3<R> p;
+                        if (e & kBoundaryBit) {
+                            const R f = -pk.w * (pdd + pdd);
+                            p = c.single_layer ? (f * g) * c.gamma2 : f * g;
+                        } else {
+                            const R pddj = d.rho == R(0) ? R(0) : fdiv<KAHAN>(d.p, d.rho * d.rho);
+                            p = (-d.x.w * (pdd + pddj)) * g;
+                        }
+                        put3(t + 3, p);
+                        return visc ? 3u : 2u;
+                    });
+    const V3<R> visc = group_total3(acc, 0), pa = group_total3(acc, 3);
+    if (!fluid || group_lane() != 0) return;
+    V3<R> npa = v3<R>(R(0), R(0), R(0)) + v3<R>(R(0), -c.gravity, R(0));
+    npa = npa + c.two_nu * visc;
+    s.acc[k] = v4<R>(pa + npa, R(0));
+}
+
+// ---------------------------------------------------------------------------
+// IISPH first loop (iisph3d_l1_one, iisph2d_l1_at)
+// ---------------------------------------------------------------------------
+// TWO_D: IISPHFluidSolver's loop (no pressure reset, no a_np; a particle's own
+// density is the new one). SPLIT: the density has run before, and viscosity
+// reads a fluid neighbor with a smaller host index at its new density.
+template <typename R, bool KAHAN, bool SPLIT, bool TWO_D>
+__global__ void __launch_bounds__(kGroupThreads) k_group_iisph_l1(int64_t n, State<R> s, Lists L, SolverConsts<R> c,
+                                                                  const StepScalars* FSB_R sc,
+                                                                  const int* FSB_R status) {
+    __shared__ GroupRows<R, 3> rows3[kGroupsPerBlock];
+    __shared__ GroupRows<R, 1> rows1[SPLIT ? 1 : kGroupsPerBlock];
+    if (*status) return;
+    const int64_t k = group_owner();
+    const bool in = k < n;
+    const uint8_t ty = in ? s.type[k] : (uint8_t)FS_TYPE_INACTIVE;
+    const bool fluid = ty == FS_TYPE_NORMAL;
+    const int64_t kk = in ? k : 0;
+    const V4<R> pk = s.pos[kk], vk = s.vel[kk];
+    const uint32_t nn = fluid ? L.size(kk) : 0u;
+    R rk = s.rho_prev[kk];
+    if constexpr (!SPLIT) {
+        const R r = group_density<R, KAHAN, !TWO_D>(kk, nn, xyz<R>(pk), s, L, c, rows1[threadIdx.x / kGroup]);
+        if (fluid) rk = r;
+    } else {
+        rk = s.rho[kk];
+    }
+    const uint32_t hk = SPLIT ? s.hidx[kk] : 0u;
+    Acc<R, KAHAN> acc;
+    group_sum<3, 3>(L, kk, nn, rows3[threadIdx.x / kGroup], acc,
+                    [&](uint32_t j) {
+                        R rj = s.rho_prev[j];
+                        // (a boundary particle's density is the same in both)
+                        if (SPLIT && s.hidx[j] < hk) rj = s.rho[j];
+                        return GVisc<R>{s.pos[j], s.vel[j], rj};
+                    },
+                    [&](uint32_t e, const GVisc<R>& d, R* t) {
+                        const V3<R> xij = xyz<R>(pk) - xyz<R>(d.x);
+                        R rj = d.rho;
+                        if (TWO_D && (e & kIndexMask) == (uint32_t)k) rj = rk;
+                        return viscosity_term<R, KAHAN>(c, xij, c.kern.template grad<KAHAN>(xij),
+                                                        xyz<R>(vk) - xyz<R>(d.v), d.x.w, rj, t) ? 1u : 0u;
+                    });
+    const V3<R> visc = group_total3(acc, 0);
+    if (!in || group_lane() != 0) return;
+    if (ty == FS_TYPE_INACTIVE) {
+        if (!SPLIT) s.rho[k] = s.rho_prev[k];   // carry the density through the double buffer
+        return;
+    }
+    if (!TWO_D) s.p[k] = R(0);
+    V3<R> npa = xyz<R>(s.ext[k]);
+    if (ty != FS_TYPE_BOUNDARY) {
+        npa = npa + v3<R>(R(0), -c.gravity, R(0));
+        npa = npa + c.two_nu * visc;
+    }
+    s.vstar[k] = v4<R>(xyz<R>(vk) + (R)sc->dt * npa, R(0));
+    if (!TWO_D) s.anp[k] = v4<R>(npa, R(0));
+    s.ext[k] = v4<R>(v3<R>(R(0), R(0), R(0)), R(0));
+    if (!SPLIT) s.rho[k] = rk;   // boundary: the previous density
+}
+
+// ---------------------------------------------------------------------------
+// IISPH 3D second loop and pressure iteration (iisph3d_l2_one, ...)
+// ---------------------------------------------------------------------------
+template <typename R, bool KAHAN, bool TWO_PASS>
+__global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_l2(int64_t n, State<R> s, Lists L, SolverConsts<R> c,
+                                                                    const StepScalars* FSB_R sc,
+                                                                    const int* FSB_R status) {
+    constexpr int NC = TWO_PASS ? 4 : 8;
+    __shared__ GroupRows<R, NC> rows[kGroupsPerBlock];
+    if (*status) return;
+    const int64_t k = group_owner();
+    const bool fluid = k < n && s.type[k] == FS_TYPE_NORMAL;
+    const int64_t kk = fluid ? k : 0;
+    const uint32_t nn = fluid ? L.size(kk) : 0u;
+    const V4<R> pk = s.pos[kk], vsk4 = s.vstar[kk];
+    const V3<R> xk = xyz<R>(pk), vsk = xyz<R>(vsk4);
+    // contrib 0, inner 1-3; in the single pass sum m gradW 4-6 and sum_fluid m |gradW|^2 7
+    Acc<R, KAHAN> acc;
+    group_sum<NC, TWO_PASS ? NC : 7>(L, kk, nn, rows[threadIdx.x / kGroup], acc,
+                                     [&](uint32_t j) { return GPosVec<R>{s.pos[j], s.vstar[j]}; },
+                                     [&](uint32_t e, const GPosVec<R>& d, R* t) {
+        const V3<R> g = c.kern.template grad<KAHAN>(xk - xyz<R>(d.x));
+        const bool bnd = (e & kBoundaryBit) != 0u;
+        V3<R> in;
+        if (!bnd) {
+            t[0] = d.x.w * dotf<KAHAN>(vsk - xyz<R>(d.v), g);
+            in = (KAHAN ? d.x.w * c.inv_rho0_sq : d.x.w / c.rho0_sq) * g;
+        } else {
+            t[0] = d.x.w * dotf<KAHAN>(vsk, g);
+            const R w = c.single_layer ? c.two_gamma * d.x.w : R(2) * d.x.w;
+            in = (KAHAN ? w * c.inv_rho0_sq : w / c.rho0_sq) * g;
+        }
+        put3(t + 1, -in);
+        if constexpr (!TWO_PASS) {
+            put3(t + 4, d.x.w * g);
+            t[7] = d.x.w * dotf<KAHAN>(g, g);
+        }
+        return bnd ? 1u : 3u;
+    });
+    const R contrib = group_total(acc, 0);
+    const V3<R> in = group_total3(acc, 1);
+    const R dt = (R)sc->dt;
+    R diag;
+    if constexpr (TWO_PASS) {
+        __shared__ GroupRows<R, 2> rows2[kGroupsPerBlock];
+        Acc<R, KAHAN> d;
+        const R mi = pk.w / c.rho0_sq;
+        group_sum<2, 1, true>(L, kk, nn, rows2[threadIdx.x / kGroup], d, [&](uint32_t j) { return GPos<R>{s.pos[j]}; },
+                              [&](uint32_t e, const GPos<R>& q, R* t) {
+            const V3<R> g = c.kern.template grad<KAHAN>(xk - xyz<R>(q.x));
+            t[0] = q.x.w * dot(in, g);
+            t[1] = q.x.w * dot(mi * (-g), g);
+            return (e & kBoundaryBit) ? 1u : 3u;
+        });
+        diag = group_total(d, 0) * (dt * dt);
+    } else {
+        const V3<R> mg = group_total3(acc, 4);
+        const R mg2 = group_total(acc, 7);
+        diag = (dot(in, mg) - (pk.w / c.rho0_sq) * mg2) * (dt * dt);
+    }
+    if (!fluid || group_lane() != 0) return;
+    const R source = (c.rest_density - s.rho[k]) - dt * contrib;
+    s.vstar[k] = v4<R>(vsk, source);
+    s.anp[k].w = diag;
+}
+
+template <typename R, bool KAHAN>
+__global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_pressure_acc(int64_t n, State<R> s, Lists L,
+                                                                              SolverConsts<R> c,
+                                                                              const StepScalars* FSB_R sc,
+                                                                              const int* FSB_R status) {
+    __shared__ GroupRows<R, 3> rows[kGroupsPerBlock];
+    if (*status || sc->done) return;
+    const int64_t k = group_owner();
+    const bool fluid = k < n && s.type[k] == FS_TYPE_NORMAL;
+    const int64_t kk = fluid ? k : 0;
+    const V3<R> xk = xyz<R>(s.pos[kk]);
+    const R pk = s.p[kk];
+    const R qk = pk / c.rho0_sq;
+    Acc<R, KAHAN> acc;
+    group_sum<3, 3>(L, kk, fluid ? L.size(kk) : 0u, rows[threadIdx.x / kGroup], acc,
+                    [&](uint32_t j) { return GPosScalar<R>{s.pos[j], s.p[j]}; },
+                    [&](uint32_t e, const GPosScalar<R>& d, R* t) {
+        const V3<R> g = c.kern.template grad<KAHAN>(xk - xyz<R>(d.x));
+        const bool bnd = (e & kBoundaryBit) != 0u;
+        V3<R> v;
+        if (KAHAN) {
+            const R f = !bnd ? d.x.w * (pk + d.a) : (c.single_layer ? c.two_gamma : R(2)) * d.x.w * pk;
+            v = (f * c.inv_rho0_sq) * g;
+        } else if (!bnd) {
+            v = (d.x.w * (qk + d.a / c.rho0_sq)) * g;
+        } else if (c.single_layer) {
+            v = ((((c.gamma * d.x.w) * R(2)) * pk) / c.rho0_sq) * g;
+        } else {
+            v = (((d.x.w * R(2)) * pk) / c.rho0_sq) * g;
+        }
+        put3(t, -v);
+        return 1u;
+    });
+    const V3<R> a = group_total3(acc, 0);
+    if (fluid && group_lane() == 0) s.acc[k] = v4<R>(a, R(0));
+}
+
+template <typename R, bool KAHAN>
+__global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_pressure_update(int64_t n, State<R> s, Lists L,
+                                                                                 SolverConsts<R> c,
+                                                                                 StepScalars* FSB_R sc,
+                                                                                 const int* FSB_R status) {
+    __shared__ GroupRows<R, 1> rows[kGroupsPerBlock];
+    if (*status || sc->done) return;
+    const int64_t k = group_owner();
+    const bool fluid = k < n && s.type[k] == FS_TYPE_NORMAL;
+    const int64_t kk = fluid ? k : 0;
+    const V3<R> xk = xyz<R>(s.pos[kk]), ak = xyz<R>(s.acc[kk]);
+    Acc<R, KAHAN> acc;
+    group_sum<1, 1>(L, kk, fluid ? L.size(kk) : 0u, rows[threadIdx.x / kGroup], acc,
+                    [&](uint32_t j) { return GPosVec<R>{s.pos[j], s.acc[j]}; },
+                    [&](uint32_t e, const GPosVec<R>& d, R* t) {
+        const V3<R> g = c.kern.template grad<KAHAN>(xk - xyz<R>(d.x));
+        t[0] = d.x.w * ((e & kBoundaryBit) ? dotf<KAHAN>(ak, g) : dotf<KAHAN>(ak - xyz<R>(d.v), g));
+        return 1u;
+    });
+    const R ap = group_total(acc, 0);
+    ErrPart o;
+    if (fluid && group_lane() == 0)
+        o = iisph3d_pressure_update_tail<R>(k, s, c, (R)sc->dt, ak, ap, s.vstar[k], s.anp[k].w, s.p[k]);
+    reduce_err_parts(o, sc);
+}
+
+// ---------------------------------------------------------------------------
+// IISPH 2D second loop and pressure iteration (iisph2d_l2_at, ...)
+// ---------------------------------------------------------------------------
+template <typename R, bool KAHAN>
+__global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_l2(int64_t n, State<R> s, Lists L, SolverConsts<R> c,
+                                                                    const StepScalars* FSB_R sc,
+                                                                    const int* FSB_R status) {
+    __shared__ GroupRows<R, 4> rows[kGroupsPerBlock];
+    __shared__ GroupRows<R, 1> rows1[kGroupsPerBlock];
+    if (*status) return;
+    const int64_t k = group_owner();
+    const bool fluid = k < n && s.type[k] == FS_TYPE_NORMAL;
+    const int64_t kk = fluid ? k : 0;
+    const uint32_t nn = fluid ? L.size(kk) : 0u;
+    const V4<R> pk = s.pos[kk];
+    const V3<R> xk = xyz<R>(pk), vsk = xyz<R>(s.vstar[kk]);
+    Acc<R, KAHAN> acc;   // sum 0, internal 1-3
+    group_sum<4, 4>(L, kk, nn, rows[threadIdx.x / kGroup], acc,
+                    [&](uint32_t j) { return GPosVec<R>{s.pos[j], s.vstar[j]}; },
+                    [&](uint32_t e, const GPosVec<R>& d, R* t) {
+        const V3<R> g = c.kern.template grad<KAHAN>(xk - xyz<R>(d.x));
+        t[0] = d.x.w * dot(vsk - xyz<R>(d.v), g);
+        if (!(e & kBoundaryBit)) put3(t + 1, ((d.x.w / c.rest_density) / c.rest_density) * g);
+        else put3(t + 1, (((c.two_gamma * d.x.w) / c.rest_density) / c.rest_density) * g);
+        return 1u;
+    });
+    const R sum = group_total(acc, 0);
+    const V3<R> neg_in = -group_total3(acc, 1);
+    const R mi = (pk.w / c.rest_density) / c.rest_density;
+    auto pos = [&](uint32_t j) { return GPos<R>{s.pos[j]}; };
+    GroupRows<R, 1>& row = rows1[threadIdx.x / kGroup];
+    Acc<R, KAHAN> d;   // over every neighbor, then over the fluid ones
+    group_sum<1, 1>(L, kk, nn, row, d, pos, [&](uint32_t, const GPos<R>& q, R* t) {
+        t[0] = q.x.w * dot(neg_in, c.kern.template grad<KAHAN>(xk - xyz<R>(q.x)));
+        return 1u;
+    });
+    group_sum<1, 1>(L, kk, nn, row, d, pos, [&](uint32_t e, const GPos<R>& q, R* t) {
+        const V3<R> g = c.kern.template grad<KAHAN>(xk - xyz<R>(q.x));
+        t[0] = q.x.w * dot(mi * (-g), g);
+        return (e & kBoundaryBit) ? 0u : 1u;
+    });
+    const R dd = group_total(d, 0);
+    if (!fluid || group_lane() != 0) return;
+    const R dt = (R)sc->dt;
+    const R source = (c.rest_density - s.rho[k]) - dt * sum;
+    s.vstar[k] = v4<R>(vsk, source);
+    s.anp[k] = v4<R>(v3<R>(R(0), R(0), R(0)), (dt * dt) * dd);
+    s.p[k] = R(0);
+}
+
+template <typename R, bool KAHAN>
+__global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_pressure_acc(int64_t n, State<R> s, Lists L,
+                                                                              SolverConsts<R> c,
+                                                                              const StepScalars* FSB_R sc,
+                                                                              const int* FSB_R status) {
+    __shared__ GroupRows<R, 3> rows[kGroupsPerBlock];
+    if (*status || sc->done) return;
+    const int64_t k = group_owner();
+    const bool fluid = k < n && s.type[k] == FS_TYPE_NORMAL;
+    const int64_t kk = fluid ? k : 0;
+    const V3<R> xk = xyz<R>(s.pos[kk]);
+    const R pr = (s.p[kk] / c.rest_density) / c.rest_density;
+    Acc<R, KAHAN> acc;
+    group_sum<3, 3>(L, kk, fluid ? L.size(kk) : 0u, rows[threadIdx.x / kGroup], acc,
+                    [&](uint32_t j) { return GPosScalar<R>{s.pos[j], s.p[j]}; },
+                    [&](uint32_t e, const GPosScalar<R>& d, R* t) {
+        const V3<R> g = c.kern.template grad<KAHAN>(xk - xyz<R>(d.x));
+        if (!(e & kBoundaryBit)) put3(t, (d.x.w * (pr + (d.a / c.rest_density) / c.rest_density)) * g);
+        else put3(t, (((c.gamma * d.x.w) * R(2)) * pr) * g);
+        return 1u;
+    });
+    const V3<R> a = group_total3(acc, 0);
+    if (fluid && group_lane() == 0) s.acc[k] = v4<R>(-a, R(0));
+}
+
+template <typename R, bool KAHAN>
+__global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_pressure_update(int64_t n, State<R> s, Lists L,
+                                                                                 SolverConsts<R> c,
+                                                                                 StepScalars* FSB_R sc,
+                                                                                 const int* FSB_R status) {
+    __shared__ GroupRows<R, 1> rows[kGroupsPerBlock];
+    if (*status || sc->done) return;
+    const int64_t k = group_owner();
+    const bool fluid = k < n && s.type[k] == FS_TYPE_NORMAL;
+    const int64_t kk = fluid ? k : 0;
+    const V3<R> xk = xyz<R>(s.pos[kk]), ak = xyz<R>(s.acc[kk]);
+    Acc<R, KAHAN> acc;
+    group_sum<1, 1>(L, kk, fluid ? L.size(kk) : 0u, rows[threadIdx.x / kGroup], acc,
+                    [&](uint32_t j) { return GPosVec<R>{s.pos[j], s.acc[j]}; },
+                    [&](uint32_t e, const GPosVec<R>& d, R* t) {
+        const V3<R> g = c.kern.template grad<KAHAN>(xk - xyz<R>(d.x));
+        t[0] = d.x.w * ((e & kBoundaryBit) ? dot(ak, g) : dot(ak - xyz<R>(d.v), g));
+        return 1u;
+    });
+    const R sum = group_total(acc, 0);
+    double e_sum = 0.0;
+    unsigned int e_cnt = 0;
+    if (fluid && group_lane() == 0) iisph2d_pressure_update_tail<R>(k, s, c, (R)sc->dt, sum, e_sum, e_cnt);
+    e_sum = warp_sum(e_sum);
+    e_cnt = warp_sum(e_cnt);
+    if ((threadIdx.x & 31) == 0 && e_cnt) {
+        atomicAdd(&sc->err_sum, e_sum);
+        atomicAdd(&sc->err_count, (unsigned long long)e_cnt);
+    }
+}
+
+}  // namespace fsb

@@ -1000,6 +1000,26 @@ __global__ void k_iisph2d_pressure_acc(int64_t n, State<R> s, Lists L, SolverCon
     iisph2d_pressure_acc_at<R, KAHAN>(k, s, L, c);
 }
 
+// the 2D update of fluid particle k given its neighbor sum; adds its error to e_sum / e_cnt
+template <typename R>
+__device__ __forceinline__ void iisph2d_pressure_update_tail(int64_t k, const State<R>& s, const SolverConsts<R>& c,
+                                                             R dt, R sum, double& e_sum, unsigned int& e_cnt) {
+    const R Ap = (dt * dt) * sum;
+    const R aii = s.anp[k].w;
+    const R src = s.vstar[k].w;
+    R p = s.p[k];
+    const bool has_diag = abs_(aii) > R(kFltEps);
+    if (has_diag) p = fmax_(R(0), p + c.omega * ((src - Ap) / aii));
+    else p = R(0);
+    s.p[k] = p;
+    R perr = abs_(src - Ap);
+    if (has_diag) {
+        if (abs_(p) <= R(kFltEps)) perr = R(0);
+        e_sum += (double)perr;
+        e_cnt += 1;
+    }
+}
+
 // 2D iteration (b) (:447-511): Ap = dt^2 sum, update, density error
 // particle k's update; adds its error to e_sum / e_cnt
 template <typename R, bool KAHAN>
@@ -1019,20 +1039,7 @@ __device__ __forceinline__ void iisph2d_pressure_update_at(int64_t k, const Stat
             if (!(e & kBoundaryBit)) sum.add(pj.w * dot(ak - xyz<R>(s.acc[j]), g));
             else sum.add(pj.w * dot(ak, g));
         }
-        const R Ap = (dt * dt) * sum.get();
-        const R aii = s.anp[k].w;
-        const R src = s.vstar[k].w;
-        R p = s.p[k];
-        const bool has_diag = abs_(aii) > R(kFltEps);
-        if (has_diag) p = fmax_(R(0), p + c.omega * ((src - Ap) / aii));
-        else p = R(0);
-        s.p[k] = p;
-        R perr = abs_(src - Ap);
-        if (has_diag) {
-            if (abs_(p) <= R(kFltEps)) perr = R(0);
-            e_sum += (double)perr;
-            e_cnt += 1;
-        }
+        iisph2d_pressure_update_tail<R>(k, s, c, dt, sum.get(), e_sum, e_cnt);
     }
 }
 template <typename R, bool KAHAN>
