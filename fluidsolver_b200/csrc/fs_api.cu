@@ -270,7 +270,7 @@ fs_status free_all(fs_ctx* c) {
     void* ptrs[] = {c->pos[0], c->pos[1], c->vel[0], c->vel[1], c->acc[0], c->acc[1], c->ext[0], c->ext[1],
                     c->rho[0], c->rho[1], c->p[0], c->p[1], c->type[0], c->type[1], c->hidx[0], c->hidx[1],
                     c->rho_prev, c->vstar, c->anp, c->err, c->gbnd, c->tile_desc, c->tile_ent, c->keys[0], c->keys[1], c->keys64[0], c->keys64[1],
-                    c->perm[0], c->perm[1], c->h2d_cell, c->h2d_rank, c->sort_hist, c->hash_table, c->cell_start, c->cell_partials, c->bbox, c->grids, c->nbr, c->nbr_count,
+                    c->perm[0], c->perm[1], c->h2d_cell, c->h2d_rank, c->sort_hist, c->hash_table, c->cell_start, c->cell_partials, c->look_tiles, c->search_box, c->search_state, c->bbox, c->grids, c->nbr, c->nbr_count,
                     c->scene_of[0], c->scene_of[1], c->d_scene_offsets,
                     c->csr_offsets, c->csr_members, c->csr_sorted, c->csr_counts, c->staging, c->status, c->small_stamps, c->scalars,
                     c->stats_parts, c->stats_out};
@@ -352,12 +352,19 @@ void choose_dims(int dim, int64_t max_cells, const int* lo_in, const int* hi_in,
 fs_status choose_grids(fs_ctx* c, const int* lo, const int* hi) {
     const int S = c->nsc();
     c->grids_host.assign(S, SceneGrid{});
+    c->box_cells = 0;
     int64_t base = 0;
     for (int sidx = 0; sidx < S; sidx++) {
         const int64_t np = c->scenes > 0 ? c->scene_offsets[sidx + 1] - c->scene_offsets[sidx] : c->cap;
         const int64_t max_cells = std::max<int64_t>(int64_t(1) << 22, 8 * std::max<int64_t>(np, 1));
         int d[3];
         choose_dims(c->dim, max_cells, lo + 3 * sidx, hi + 3 * sidx, d);
+        int64_t in_box = 1;   // cells of the box that the grid holds
+        for (int a = 0; a < c->dim; a++) {
+            const int64_t e = (int64_t)hi[3 * sidx + a] - lo[3 * sidx + a] + 1;
+            in_box *= std::max<int64_t>(1, std::min<int64_t>(e, d[a]));
+        }
+        c->box_cells += in_box;
         SceneGrid& g = c->grids_host[sidx];
         g.d0 = d[0];
         g.d1 = d[1];
@@ -382,9 +389,12 @@ fs_status ensure_cells(fs_ctx* c) {
         clear_graphs(c);
         if (c->cell_start) cudaFree(c->cell_start);
         if (c->cell_partials) cudaFree(c->cell_partials);
+        if (c->look_tiles) cudaFree(c->look_tiles);
         c->cell_start = c->cell_partials = nullptr;
-        FS_TRY(dalloc(&c->cell_start, (size_t)3 * need));
+        c->look_tiles = nullptr;
+        FS_TRY(dalloc(&c->cell_start, (size_t)3 * need + 4));   // the counting path's extra entry, whole uint4
         FS_TRY(dalloc(&c->cell_partials, (size_t)scan_tiles(3 * need)));
+        FS_TRY(dalloc(&c->look_tiles, (size_t)look_tiles(3 * need + 1)));
         c->cell_alloc = need;
     }
     return FS_OK;
@@ -675,17 +685,12 @@ template <typename R> fs_status compact_search_impl(fs_ctx* c, State<R> s, bool 
     return FS_OK;
 }
 
-template <typename R> fs_status search_impl(fs_ctx* c, bool solver_lists) {
+// The particles' new order, their fields moved into it, and the cell table, by
+// the radix sort.
+template <typename R> fs_status order_by_radix_sort(fs_ctx* c, State<R> s) {
     const int64_t n = c->n;
     cudaStream_t st = c->stream;
     const bool single = c->reference_order;
-    if (n == 0) {
-        c->have_lists = solver_lists;
-        c->have_cells = true;
-        return FS_OK;
-    }
-    State<R> s = state_of<R>(c);
-    if (c->hash_table) return compact_search_impl<R>(c, s, solver_lists);
     // bbox of the structure's cells -> grid origin
     FS_TRY(reset_bbox(c));
     c->launches++;
@@ -740,6 +745,66 @@ template <typename R> fs_status search_impl(fs_ctx* c, bool solver_lists) {
                                                              c->cell_start, s.hidx, c->h2d_rank);
         FS_CUDA(cudaGetLastError());
     }
+    return FS_OK;
+}
+
+// Whether the search orders its particles by counting (fs_search.cuh): not
+// with many excluded inactive particles, which share one entry, nor where the
+// uploaded particles' box has few cells for them (a particle's place is counted
+// over its entry; 128 a cell is 16 times a dam's).
+bool counting_order(const fs_ctx* c) {
+    return c->n - c->n_struct <= 1024 && c->n_struct <= 128 * c->box_cells;
+}
+
+// The same order and table as order_by_radix_sort, by counting.
+template <typename R> fs_status order_by_counting(fs_ctx* c, State<R> s) {
+    const int64_t n = c->n;
+    cudaStream_t st = c->stream;
+    const bool single = c->reference_order;
+    const int64_t table = (int64_t)c->regions * (c->cells + 1);
+    const uint32_t excluded = (uint32_t)table;
+    const int64_t entries = table + 1, tiles = look_tiles(entries);
+    const int pb = c->tuning.block;   // the per-particle kernels' block size (fs_autotune)
+    const unsigned gb = c->scenes > 0 ? grid_for(n, 256) : std::min<unsigned>(grid_for(std::max(n, entries / 16), 256), 148u * 8u);
+    uint32_t* entry = c->keys[0];
+    uint32_t* slot = c->keys[1];
+    uint32_t* list = c->perm[0];
+    uint32_t* order = single ? c->perm[1] : nullptr;
+    const int nx = c->cur ^ 1;
+    c->launches += 5;
+    k_search_box<R><<<gb, 256, 0, st>>>(n, s.pos, s.type, s.scene, c->nsc(), c->include_inactive, c->search_radius,
+                                        c->truncate_cells, c->search_box, c->grids, c->search_state,
+                                        (uint4*)c->cell_start, (entries + 3) / 4, c->look_tiles, tiles);
+    k_search_keys<R><<<grid_for(n, pb), pb, 0, st>>>(n, s.pos, s.type, s.hidx, c->include_inactive, single,
+                                                     c->search_radius, c->truncate_cells, c->grids, s.scene, c->cells,
+                                                     excluded, entry, slot, order, c->h2d_cell, c->h2d_rank,
+                                                     c->cell_start, c->status);
+    k_search_scan<<<(unsigned)tiles, kLookThreads, 0, st>>>(c->cell_start, entries, c->look_tiles, c->search_state,
+                                                            c->status);
+    k_search_scatter<<<grid_for(n, pb), pb, 0, st>>>(n, entry, slot, c->cell_start, list, c->status);
+    k_search_reorder<R><<<grid_for(n, pb), pb, 0, st>>>(
+        n, c->n_struct, excluded, list, entry, order, c->cell_start, (const V4<R>*)c->pos[c->cur], (V4<R>*)c->pos[nx],
+        (const V4<R>*)c->vel[c->cur], (V4<R>*)c->vel[nx], (const V4<R>*)c->acc[c->cur], (V4<R>*)c->acc[nx],
+        (const V4<R>*)c->ext[c->cur], (V4<R>*)c->ext[nx], (const R*)c->rho[c->cur], (R*)c->rho[nx],
+        (const R*)c->p[c->cur], (R*)c->p[nx], c->type[c->cur], c->type[nx], c->hidx[c->cur], c->hidx[nx],
+        c->scene_of[c->cur], c->scene_of[nx], c->h2d_rank, c->status);
+    FS_CUDA(cudaGetLastError());
+    c->cur = nx;
+    return FS_OK;
+}
+
+template <typename R> fs_status search_impl(fs_ctx* c, bool solver_lists) {
+    const int64_t n = c->n;
+    cudaStream_t st = c->stream;
+    if (n == 0) {
+        c->have_lists = solver_lists;
+        c->have_cells = true;
+        return FS_OK;
+    }
+    State<R> s = state_of<R>(c);
+    if (c->hash_table) return compact_search_impl<R>(c, s, solver_lists);
+    FS_TRY(counting_order(c) ? order_by_counting<R>(c, s) : order_by_radix_sort<R>(c, s));
+    s = state_of<R>(c);
     if (solver_lists) {
         WalkParams w = walk_of(c, true);
         const uint32_t owners = 1u << FS_TYPE_NORMAL;
@@ -1694,6 +1759,8 @@ static fs_status create_ctx(const fs_params* p, int32_t scenes, const int64_t* o
     FS_ALLOC(*(char**)&c->gbnd, cap * v4);
     const int S = c->nsc();
     FS_ALLOC(c->bbox, 6 * S);
+    FS_ALLOC(c->search_box, 6 * S);
+    FS_ALLOC(c->search_state, 1);
     FS_ALLOC(c->grids, S);
     FS_ALLOC(c->status, 1);
     FS_ALLOC(c->small_stamps, 8);
@@ -1721,6 +1788,9 @@ static fs_status create_ctx(const fs_params* p, int32_t scenes, const int64_t* o
     for (auto& e : c->ev)
         if (cudaEventCreate(&e) != cudaSuccess) return bail(fail(FS_ERR_CUDA, "cudaEventCreate failed"));
     if (cudaMemsetAsync(c->status, 0, sizeof(int), c->stream) != cudaSuccess ||
+        cudaMemsetAsync(c->search_state, 0, sizeof(SearchState), c->stream) != cudaSuccess ||
+        cudaMemsetAsync(c->search_box, 0x7f, 3 * S * sizeof(int), c->stream) != cudaSuccess ||
+        cudaMemsetAsync(c->search_box + 3 * S, 0x80, 3 * S * sizeof(int), c->stream) != cudaSuccess ||
         cudaStreamSynchronize(c->stream) != cudaSuccess)
         return bail(fail(FS_ERR_CUDA, "initialisation failed"));
 #undef FS_ALLOC

@@ -90,6 +90,10 @@ struct fs_ctx {
     uint32_t hash_mask = 0;           // slots - 1 (a power of two, >= 2 x capacity)
     uint32_t* cell_start = nullptr;   // [regions][cells + 1] first sorted index of cell >= c
     uint32_t* cell_partials = nullptr;  // tile totals of the cell table's scan
+    unsigned long long* look_tiles = nullptr;   // tile states of k_search_scan
+    int* search_box = nullptr;                  // k_search_box's per-scene boxes (as bbox) and its state
+    fsb::SearchState* search_state = nullptr;
+    int64_t box_cells = 0;            // cells of the uploaded particles' boxes, all scenes
     int64_t cells = 0;                // dims[0] * dims[1] * dims[2]
     int key_bits = 30;                // bits of the linear cell index in the sort keys
     int64_t cell_alloc = 0;           // entries allocated per table

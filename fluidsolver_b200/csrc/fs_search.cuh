@@ -58,10 +58,11 @@ template <typename R> __device__ __forceinline__ int cell_coord(R x, float r, bo
 // scene ids (null: one scene). A block whose particles all belong to one
 // scene reduces first and issues one atomic per bound; a mixed block (a scene
 // boundary inside it) issues one per particle.
+// Every thread of the block calls it.
 template <typename R>
-__global__ void k_bbox(int64_t n, const V4<R>* FSB_R pos, const uint8_t* FSB_R type,
-                       const uint16_t* FSB_R scene, int scenes, bool include_inactive, float r, bool trunc,
-                       int* FSB_R bbox) {
+__device__ __forceinline__ void bbox_block(int64_t n, const V4<R>* FSB_R pos, const uint8_t* FSB_R type,
+                                           const uint16_t* FSB_R scene, int scenes, bool include_inactive, float r,
+                                           bool trunc, int* FSB_R bbox) {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     int mn[3] = {INT_MAX, INT_MAX, INT_MAX}, mx[3] = {INT_MIN, INT_MIN, INT_MIN};
     const int sk = (k < n && scene) ? scene[k] : 0;
@@ -125,6 +126,12 @@ __global__ void k_bbox(int64_t n, const V4<R>* FSB_R pos, const uint8_t* FSB_R t
         }
     }
 }
+template <typename R>
+__global__ void k_bbox(int64_t n, const V4<R>* FSB_R pos, const uint8_t* FSB_R type,
+                       const uint16_t* FSB_R scene, int scenes, bool include_inactive, float r, bool trunc,
+                       int* FSB_R bbox) {
+    bbox_block<R>(n, pos, type, scene, scenes, include_inactive, r, trunc, bbox);
+}
 
 // Grid origin of every scene for this step: the bbox minimum, shifted so that
 // the box is centred in the scene's dims when it is smaller.
@@ -170,6 +177,47 @@ __device__ __forceinline__ uint32_t region_of(uint8_t t, bool single_region) {
 // a particle that stays in its cell keeps its rank from the last search, and
 // one that arrives goes after every stayer, arrivals by ascending index (the
 // reference appends them to the cell's std::list in its i-ascending loop).
+// key_of: the region, linear cell and order within the cell of particle k;
+// false for an excluded inactive particle. with_order: the order is wanted
+// (keys64).
+template <typename R>
+__device__ __forceinline__ bool key_of(int64_t k, const V4<R>* FSB_R pos, const uint8_t* FSB_R type,
+                                       const uint32_t* FSB_R hidx, bool include_inactive, bool single_region,
+                                       float r, bool trunc, const SceneGrid* FSB_R grids, const uint16_t* FSB_R scene,
+                                       bool with_order, int2* FSB_R h2d_cell, const uint32_t* FSB_R h2d_rank,
+                                       int* FSB_R status, uint32_t& region, uint32_t& lin, uint32_t& order) {
+    const uint8_t t = type[k];
+    order = with_order ? hidx[k] : 0u;
+    if (!include_inactive && t == FS_TYPE_INACTIVE) return false;
+    V4<R> p = pos[k];
+    if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z))) {
+        // a position that is NaN or infinite ends the step with FS_ERR_NAN
+        // (and stays out of the cell structure, which the rest of the
+        // step then no longer builds on)
+        raise_status(status, FS_ERR_NAN);
+        p.x = p.y = p.z = R(0);
+    }
+    const SceneGrid g = grids[scene ? scene[k] : 0];
+    bool cl = false;
+    const int cx = cell_coord<R>(p.x, r, trunc), cy = cell_coord<R>(p.y, r, trunc);
+    int lx = local_cell(cx, g.o0, g.d0, cl);
+    int ly = local_cell(cy, g.o1, g.d1, cl);
+    int lz = local_cell(cell_coord<R>(p.z, r, trunc), g.o2, g.d2, cl);
+    lin = (uint32_t)(g.base + ((int64_t)lz * g.d1 + ly) * g.d0 + lx);
+    region = region_of(t, single_region);
+    if (h2d_cell) {
+        const uint32_t h = order;
+        const int2 was = h2d_cell[h];
+        const uint32_t rank = h2d_rank[h];
+        if (rank != 0xffffffffu && was.x == cx && was.y == cy) {
+            order = rank;
+        } else {
+            order = 0x80000000u | h;
+            h2d_cell[h] = make_int2(cx, cy);
+        }
+    }
+    return true;
+}
 template <typename R>
 __device__ __forceinline__ void keys_at(int64_t k, const V4<R>* FSB_R pos, const uint8_t* FSB_R type,
                                         const uint32_t* FSB_R hidx, bool include_inactive, bool single_region,
@@ -178,40 +226,10 @@ __device__ __forceinline__ void keys_at(int64_t k, const V4<R>* FSB_R pos, const
                                         unsigned long long* FSB_R keys64, uint32_t* FSB_R perm,
                                         int2* FSB_R h2d_cell, const uint32_t* FSB_R h2d_rank,
                                         int* FSB_R status) {
-    uint8_t t = type[k];
-    uint32_t key;
-    uint32_t order = keys64 ? hidx[k] : 0u;
-    if (!include_inactive && t == FS_TYPE_INACTIVE) {
-        key = inactive_key(key_bits);
-    } else {
-        V4<R> p = pos[k];
-        if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z))) {
-            // a position that is NaN or infinite ends the step with FS_ERR_NAN
-            // (and stays out of the cell structure, which the rest of the
-            // step then no longer builds on)
-            raise_status(status, FS_ERR_NAN);
-            p.x = p.y = p.z = R(0);
-        }
-        const SceneGrid g = grids[scene ? scene[k] : 0];
-        bool cl = false;
-        const int cx = cell_coord<R>(p.x, r, trunc), cy = cell_coord<R>(p.y, r, trunc);
-        int lx = local_cell(cx, g.o0, g.d0, cl);
-        int ly = local_cell(cy, g.o1, g.d1, cl);
-        int lz = local_cell(cell_coord<R>(p.z, r, trunc), g.o2, g.d2, cl);
-        const uint32_t lin = (uint32_t)(g.base + ((int64_t)lz * g.d1 + ly) * g.d0 + lx);
-        key = (region_of(t, single_region) << key_bits) | lin;
-        if (h2d_cell) {
-            const uint32_t h = order;
-            const int2 was = h2d_cell[h];
-            const uint32_t rank = h2d_rank[h];
-            if (rank != 0xffffffffu && was.x == cx && was.y == cy) {
-                order = rank;
-            } else {
-                order = 0x80000000u | h;
-                h2d_cell[h] = make_int2(cx, cy);
-            }
-        }
-    }
+    uint32_t region, lin, order, key = inactive_key(key_bits);
+    if (key_of<R>(k, pos, type, hidx, include_inactive, single_region, r, trunc, grids, scene, keys64 != nullptr,
+                  h2d_cell, h2d_rank, status, region, lin, order))
+        key = (region << key_bits) | lin;
     if (keys64) keys64[k] = ((unsigned long long)key << 32) | order;
     else keys[k] = key;
     perm[k] = (uint32_t)k;
@@ -283,6 +301,229 @@ __global__ void k_reorder(int64_t n, const uint32_t* FSB_R perm, const V4<R>* FS
     if (k >= n) return;
     reorder_at<R>(k, perm, pos0, pos1, vel0, vel1, acc0, acc1, ext0, ext1, rho0, rho1, p0, p1, t0, t1, h0, h1, sc0,
                   sc1);
+}
+
+// ---------------------------------------------------------------------------
+// The search's order by counting instead of the radix sort: five launches that
+// give the same stable order and the same cell table.
+//   k_search_box      the cells' bounding box; its last block sets the grid
+//                     origins. Clears the table and the scan's state on the way.
+//   k_search_keys     every particle's table entry, counted there (one atomic
+//                     per run of equal entries in a warp), and its place among
+//                     the entry's particles in the order of the atomics
+//   k_search_scan     the counts' exclusive scan, which is the cell-start table
+//   k_search_scatter  the particles' indices by entry, in the atomics' order
+//   k_search_reorder  a particle's place within its entry is the number of the
+//                     entry's particles before it (by index, or by the order
+//                     within the cell), counted over them; its fields go there
+// Counting within an entry is quadratic in the entry's size, 8 particles in
+// 3D, and cheap against the list builder, which tests 27 such entries for
+// every particle; scenes with hundreds of particles per cell, and with many
+// excluded inactive particles (one entry), keep the radix sort (fs_api.cu).
+//
+// Against the radix path (bounding box, origin, keys, 3 launches per 8-bit
+// digit, reorder, run counts, scan; 8 to 18 launches), a whole search on a B200:
+// SEARCH_FIGURES
+// ---------------------------------------------------------------------------
+struct SearchState {
+    uint32_t box_ticket;     // blocks of k_search_box that are done (its last block clears it)
+    uint32_t scan_ticket;    // tiles of the scan handed out (cleared by k_search_box)
+};
+
+template <typename R>
+__global__ void k_search_box(int64_t n, const V4<R>* FSB_R pos, const uint8_t* FSB_R type, const uint16_t* FSB_R scene,
+                             int scenes, bool include_inactive, float r, bool trunc, int* FSB_R box,
+                             SceneGrid* FSB_R grids, SearchState* FSB_R st, uint4* FSB_R table, int64_t table16,
+                             unsigned long long* FSB_R tiles, int64_t ntiles) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, total = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = t; i < table16; i += total) table[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (int64_t i = t; i < ntiles; i += total) tiles[i] = 0ull;
+    if (t == 0) st->scan_ticket = 0u;
+    bbox_block<R>(n, pos, type, scene, scenes, include_inactive, r, trunc, box);
+    __threadfence();
+    __syncthreads();
+    __shared__ bool s_last;
+    if (threadIdx.x == 0) s_last = atomicAdd(&st->box_ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (int s = threadIdx.x; s < scenes; s += blockDim.x) {
+        int b[6];
+        for (int a = 0; a < 3; a++) {
+            b[a] = __ldcg(box + 3 * s + a);
+            b[3 + a] = __ldcg(box + 3 * scenes + 3 * s + a);
+            box[3 * s + a] = 0x7f7f7f7f;   // for the next search
+            box[3 * scenes + 3 * s + a] = (int)0x80808080;
+        }
+        grid_origin_at(0, b, grids + s, 1);
+    }
+    if (threadIdx.x == 0) st->box_ticket = 0u;
+}
+
+// entry[k]: particle k's entry in the concatenated per-region tables (excluded
+// inactive particles: `excluded`, one past them); slot[k]: its place among the
+// entry's particles as counted; order[k] (reference order): its order in the cell
+template <typename R>
+__global__ void k_search_keys(int64_t n, const V4<R>* FSB_R pos, const uint8_t* FSB_R type, const uint32_t* FSB_R hidx,
+                              bool include_inactive, bool single_region, float r, bool trunc,
+                              const SceneGrid* FSB_R grids, const uint16_t* FSB_R scene, int64_t cells,
+                              uint32_t excluded, uint32_t* FSB_R entry, uint32_t* FSB_R slot, uint32_t* FSB_R order,
+                              int2* FSB_R h2d_cell, const uint32_t* FSB_R h2d_rank, uint32_t* FSB_R counts,
+                              int* FSB_R status) {
+    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    uint32_t e = 0xffffffffu;   // no particle
+    if (k < n) {
+        uint32_t region = 0, lin = 0, o = 0;
+        e = key_of<R>(k, pos, type, hidx, include_inactive, single_region, r, trunc, grids, scene, order != nullptr,
+                      h2d_cell, h2d_rank, status, region, lin, o)
+                ? (uint32_t)(region * (cells + 1) + lin)
+                : excluded;
+        entry[k] = e;
+        if (order) order[k] = o;
+    }
+    const unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned peers = __match_any_sync(all, e);
+    const int lead = __ffs(peers) - 1;
+    uint32_t base = 0;
+    if (lane == lead && e != 0xffffffffu) base = atomicAdd(counts + e, (uint32_t)__popc(peers));
+    base = __shfl_sync(all, base, lead);
+    if (k < n) slot[k] = base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+}
+
+// Exclusive scan of m counts in place, one launch: tiles in the order of a
+// ticket, each adding the totals of the tiles before it (decoupled look-back;
+// a tile's predecessors have started before it). tiles[t]: 0, or (1: the tile's
+// total, 2: the total up to its end) << 32 | value.
+constexpr int kLookThreads = 256;
+constexpr int kLookTile = kLookThreads * 16;
+constexpr int kLookTries = 1 << 22;   // polls of a predecessor before the scan gives up (FS_ERR_TIMEOUT)
+inline int64_t look_tiles(int64_t m) { return (m + kLookTile - 1) / kLookTile; }
+static __global__ void __launch_bounds__(kLookThreads) k_search_scan(uint32_t* FSB_R a, int64_t m,
+                                                                     unsigned long long* FSB_R tiles,
+                                                                     SearchState* FSB_R st, int* FSB_R status) {
+    __shared__ uint32_t s_warp[kLookThreads / 32], s_tile, s_before;
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const unsigned all = 0xffffffffu;
+    if (t == 0) s_tile = atomicAdd(&st->scan_ticket, 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    // a warp's 512 consecutive entries, 128 at a time (the table is padded to whole uint4)
+    const int64_t base = (int64_t)tile * kLookTile + w * 512 + lane * 4;
+    uint4 v[4];
+    uint32_t excl[4], run = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        v[j] = base + j * 128 < m ? *reinterpret_cast<const uint4*>(a + base + j * 128) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const uint32_t sum = v[j].x + v[j].y + v[j].z + v[j].w;
+        uint32_t incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(all, incl, o);
+            if (lane >= o) incl += y;
+        }
+        excl[j] = run + incl - sum;
+        run += __shfl_sync(all, incl, 31);
+    }
+    if (lane == 0) s_warp[w] = run;
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+#pragma unroll
+    for (int q = 0; q < kLookThreads / 32; q++) {
+        if (q < w) before += s_warp[q];
+        total += s_warp[q];
+    }
+    if (w == 0) {
+        volatile unsigned long long* look = tiles;
+        uint32_t prefix = 0;
+        if (tile > 0) {
+            if (lane == 0) look[tile] = (1ull << 32) | total;
+            for (int64_t last = (int64_t)tile - 1; last >= 0; last -= 32) {
+                const int64_t i = last - lane;
+                unsigned long long x = 2ull << 32;   // before the first tile: a total of 0
+                if (i >= 0) {
+                    int tries = 0;
+                    while (((x = look[i]) >> 32) == 0ull && ++tries < kLookTries) {}
+                    if ((x >> 32) == 0ull) {
+                        raise_status(status, FS_ERR_TIMEOUT);
+                        x = 2ull << 32;
+                    }
+                }
+                const unsigned done = __ballot_sync(all, (x >> 32) == 2ull);
+                const int end = done ? __ffs(done) - 1 : 31;   // up to the nearest total so far
+                prefix += __reduce_add_sync(all, lane <= end ? (uint32_t)x : 0u);
+                if (done) break;
+            }
+        }
+        if (lane == 0) {
+            look[tile] = (2ull << 32) | (prefix + total);
+            s_before = prefix;
+        }
+    }
+    __syncthreads();
+    before += s_before;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        if (base + j * 128 >= m) continue;
+        const uint32_t x = before + excl[j];
+        *reinterpret_cast<uint4*>(a + base + j * 128) =
+            make_uint4(x, x + v[j].x, x + v[j].x + v[j].y, x + v[j].x + v[j].y + v[j].z);
+    }
+}
+
+// (after a scan that gave up nothing may be placed: the table is incomplete)
+static __global__ void k_search_scatter(int64_t n, const uint32_t* FSB_R entry, const uint32_t* FSB_R slot,
+                                        const uint32_t* FSB_R cell_start, uint32_t* FSB_R list,
+                                        const int* FSB_R status) {
+    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (k >= n || *status == FS_ERR_TIMEOUT) return;
+    list[cell_start[entry[k]] + slot[k]] = (uint32_t)k;
+}
+
+// Particle list[i]'s place, and its fields moved there (k_reorder's); with the
+// 2D hashed grid's history also its rank in the cell (k_h2d_rank's)
+template <typename R>
+__global__ void k_search_reorder(int64_t n, int64_t n_struct, uint32_t excluded, const uint32_t* FSB_R list,
+                                 const uint32_t* FSB_R entry, const uint32_t* FSB_R order,
+                                 const uint32_t* FSB_R cell_start, const V4<R>* FSB_R pos0, V4<R>* FSB_R pos1,
+                                 const V4<R>* FSB_R vel0, V4<R>* FSB_R vel1, const V4<R>* FSB_R acc0,
+                                 V4<R>* FSB_R acc1, const V4<R>* FSB_R ext0, V4<R>* FSB_R ext1, const R* FSB_R rho0,
+                                 R* FSB_R rho1, const R* FSB_R p0, R* FSB_R p1, const uint8_t* FSB_R t0,
+                                 uint8_t* FSB_R t1, const uint32_t* FSB_R h0, uint32_t* FSB_R h1,
+                                 const uint16_t* FSB_R sc0, uint16_t* FSB_R sc1, uint32_t* FSB_R h2d_rank,
+                                 const int* FSB_R status) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n || *status == FS_ERR_TIMEOUT) return;
+    const uint32_t k = list[i], e = entry[k];
+    const uint32_t b = cell_start[e], end = e == excluded ? (uint32_t)n : cell_start[e + 1];
+    // the particle's fields, on their way while its place is counted
+    const V4<R> x = pos0[k], v = vel0[k], a = acc0[k], f = ext0[k];
+    const R rho = rho0[k], p = p0[k];
+    const uint8_t ty = t0[k];
+    const uint32_t h = h0[k];
+    uint32_t rank = 0;
+    if (order) {
+        const uint32_t mine = order[k];
+        for (uint32_t j = b; j < end; j++) {
+            const uint32_t q = list[j], o = order[q];
+            rank += (o < mine || (o == mine && q < k)) ? 1u : 0u;
+        }
+    } else {
+        for (uint32_t j = b; j < end; j++) rank += list[j] < k ? 1u : 0u;
+    }
+    const uint32_t d = b + rank;
+    pos1[d] = x;
+    vel1[d] = v;
+    acc1[d] = a;
+    ext1[d] = f;
+    rho1[d] = rho;
+    p1[d] = p;
+    t1[d] = ty;
+    h1[d] = h;
+    if (sc0) sc1[d] = sc0[k];
+    if (h2d_rank && d < (uint32_t)n_struct) h2d_rank[h] = rank;
 }
 
 // ---------------------------------------------------------------------------
