@@ -685,6 +685,15 @@ template <typename R> fs_status compact_search_impl(fs_ctx* c, State<R> s, bool 
     return FS_OK;
 }
 
+// Whether the solver lists are built with kGroup threads per owner
+// (fs_gather.cuh): below the size where one thread per owner fills the device.
+// B200, a whole search with one thread and with eight: 2D, 2,500 fluid particles
+// 45 and 27 us, 40,000 53 and 41, 160,000 86 and 88; 3D, 8,000 86 and 39, 100,000
+// 123 and 121, 250,047 232 and 266; FP64 20,700 90 and 51, 250,047 217 and 309.
+bool grouped_lists(const fs_ctx* c) {
+    return c->n_fluid <= (c->dim == 2 ? 131072 : (c->precision == FS_PRECISION_FP64 ? 65536 : 98304));
+}
+
 // The particles' new order, their fields moved into it, and the cell table, by
 // the radix sort.
 template <typename R> fs_status order_by_radix_sort(fs_ctx* c, State<R> s) {
@@ -820,15 +829,23 @@ template <typename R> fs_status search_impl(fs_ctx* c, bool solver_lists) {
                 built = true;
             }
         }
-        if (!built) {
+        const bool group = !built && grouped_lists(c);
+        if (group) {
+            c->launches++;
+            auto* kernel = c->dim == 2 ? (c->sort_lists_by_host ? k_group_lists<R, 3, true> : k_group_lists<R, 3, false>)
+                                       : (c->sort_lists_by_host ? k_group_lists<R, 7, true> : k_group_lists<R, 7, false>);
+            kernel<<<group_grid(c->n_owners), kGroupThreads, 0, st>>>(
+                c->n_owners, s.pos, s.type, s.hidx, c->cell_start, w, owners, rows, c->nbr, c->nbr_stride,
+                c->nbr_capacity, c->nbr_count, c->status, c->scalars);
+        } else if (!built) {
             c->launches++;
             k_build_lists<R><<<grid_for(c->n_owners), kBlock, 0, st>>>(
                 c->n_owners, s.pos, s.type, c->cell_start, w, owners, rows, c->nbr, c->nbr_stride,
                 c->nbr_capacity, c->nbr_count, c->status, c->scalars);
         }
         FS_CUDA(cudaGetLastError());
-        if (c->sort_lists_by_host) {
-    c->launches++;
+        if (c->sort_lists_by_host && !group) {
+            c->launches++;
             k_sort_lists_by_host<<<grid_for(c->n_owners), kBlock, 0, st>>>(c->n_owners, c->nbr, c->nbr_stride,
                                                                            c->nbr_capacity, c->nbr_count, s.hidx);
             FS_CUDA(cudaGetLastError());

@@ -528,4 +528,170 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_pressure_update
     }
 }
 
+// ---------------------------------------------------------------------------
+// solver lists with kGroup threads per owner
+// ---------------------------------------------------------------------------
+// The lists of k_build_lists (and, SORT, k_sort_lists_by_host), entry for entry.
+// The group's threads look up the ranges of sorted particles that the walk
+// visits (a cell and region each, or rows of three cells away from the grid's
+// border), all together; list their particles in the walk's order; and test
+// them kGroup at a time, the hits taking their places by ballot. SORT: a hit's
+// place is the number of hits with a smaller host index. Owners whose
+// neighborhood leaves the grid take the serial walk, which checks every
+// candidate's own cell. ROUNDS: ranges per thread, 18 in 2D and at most 54 in
+// 3D over kGroup.
+//
+// One thread per owner walks 9 or 27 cells in a row: 28 us for the 3,688
+// particles of a 2D dam. fs_api.cu (grouped_lists) has the sizes at which each
+// is faster, and the times.
+constexpr int kListWindow = 128;   // candidates listed at a time; hits sorted in shared memory
+struct ListGroup {
+    uint32_t cand[kListWindow];
+};
+struct ListSort {
+    uint32_t hit[kListWindow], host[kListWindow];
+};
+template <typename R, int ROUNDS, bool SORT>
+__global__ void __launch_bounds__(kGroupThreads) k_group_lists(int64_t n_owners, const V4<R>* FSB_R pos,
+                                                               const uint8_t* FSB_R type, const uint32_t* FSB_R hidx,
+                                                               const uint32_t* FSB_R cell_start, WalkParams w,
+                                                               uint32_t owner_mask, bool rows, uint32_t* FSB_R nbr,
+                                                               int64_t stride, int K, uint32_t* FSB_R count,
+                                                               int* FSB_R status, StepScalars* FSB_R sc) {
+    __shared__ ListGroup lists[kGroupsPerBlock];
+    __shared__ ListSort sorts[SORT ? kGroupsPerBlock : 1];
+    {   // an overflow elsewhere does not stop the counting: the largest list decides how far the lists grow
+        const int err = *status;
+        if (err && err != FS_ERR_CAPACITY) return;
+    }
+    const unsigned all = 0xffffffffu, shift = threadIdx.x & 31u & ~(unsigned)(kGroup - 1);
+    constexpr unsigned kMask = (1u << kGroup) - 1u;
+    const int g = group_lane();
+    ListGroup& sh = lists[threadIdx.x / kGroup];
+    const int64_t k = group_owner();
+    const bool in = k < n_owners;
+    const int64_t kk = in ? k : 0;
+    const bool owner = in && ((owner_mask >> type[kk]) & 1u);
+    const V3<R> xi = xyz<R>(pos[kk]);
+    const SceneGrid gr = w.grid_of(kk);
+    const int c0 = cell_coord<R>(xi.x, w.r, w.trunc), c1 = cell_coord<R>(xi.y, w.r, w.trunc),
+              c2 = cell_coord<R>(xi.z, w.r, w.trunc);
+    const int l0 = c0 - gr.o0, l1 = c1 - gr.o1, l2 = c2 - gr.o2;
+    // walk_rows' condition, and whether every neighbor cell lies in the grid
+    const bool row = rows && !(l0 < 2 || l1 < 2 || l2 < 2 || l0 > gr.d0 - 3 || l1 > gr.d1 - 3 || l2 > gr.d2 - 3);
+    const bool inside = l0 >= 1 && l1 >= 1 && l0 < gr.d0 - 1 && l1 < gr.d1 - 1 &&
+                        (w.dim == 2 ? l2 >= 0 && l2 < gr.d2 : l2 >= 1 && l2 < gr.d2 - 1);
+    const int nranges = !owner || !inside ? 0 : row ? 18 : (w.dim == 2 ? 9 : 27) * w.regions;
+    uint32_t rb[ROUNDS], rn[ROUNDS];
+#pragma unroll
+    for (int r = 0; r < ROUNDS; r++) {
+        const int q = r * kGroup + g;
+        rb[r] = rn[r] = 0u;
+        if (q >= nranges) continue;
+        int region, x, y, z, len = 1;
+        if (row) {
+            region = q / 9;
+            x = l0 - 1;
+            y = l1 + q % 9 % 3 - 1;
+            z = l2 + q % 9 / 3 - 1;
+            len = 3;
+        } else {   // cells dx, dy, dz ascending, the regions of a cell together
+            const int c = w.regions == 2 ? q >> 1 : q;
+            region = w.regions == 2 ? q & 1 : 0;
+            x = l0 + (w.dim == 2 ? c / 3 : c / 9) - 1;
+            y = l1 + (w.dim == 2 ? c % 3 : c / 3 % 3) - 1;
+            z = l2 + (w.dim == 2 ? 0 : c % 3 - 1);
+        }
+        const uint32_t* cs = cell_start + region * (w.cells + 1) + gr.base + ((int64_t)z * gr.d1 + y) * gr.d0 + x;
+        rb[r] = cs[0] | (region == 1 ? kBoundaryBit : 0u);
+        rn[r] = cs[len] - cs[0];
+    }
+    // places of the ranges in the list of candidates
+    uint32_t off[ROUNDS], total = 0;
+#pragma unroll
+    for (int r = 0; r < ROUNDS; r++) {
+        uint32_t incl = rn[r];
+#pragma unroll
+        for (int o = 1; o < kGroup; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(all, incl, o, kGroup);
+            if (g >= o) incl += y;
+        }
+        off[r] = total + incl - rn[r];
+        total += __shfl_sync(all, incl, kGroup - 1, kGroup);
+    }
+    const uint32_t most = __reduce_max_sync(all, total);
+    const float x0 = (float)xi.x, x1 = (float)xi.y, x2 = (float)xi.z;
+    uint32_t c = 0;
+    for (uint32_t base = 0; base < most; base += kListWindow) {
+#pragma unroll
+        for (int r = 0; r < ROUNDS; r++) {
+            const uint32_t to = min(off[r] + rn[r], base + kListWindow);
+            for (uint32_t i = max(off[r], base); i < to; i++) sh.cand[i - base] = rb[r] + (i - off[r]);
+        }
+        __syncwarp();
+        const uint32_t m = total > base ? min(total - base, (uint32_t)kListWindow) : 0u;
+        const uint32_t mm = __reduce_max_sync(all, m);
+        constexpr int U = 4;   // candidates in flight per thread
+        for (uint32_t i = 0; i < mm; i += kGroup * U) {
+            uint32_t j[U];
+            V4<R> pj[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const uint32_t q = i + u * kGroup + g;
+                j[u] = q < m ? sh.cand[q] : 0u;
+                pj[u] = pos[j[u] & kIndexMask];
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                bool hit = i + u * kGroup + g < m;
+                if (row) {
+                    const float d0 = x0 - (float)pj[u].x, d1 = x1 - (float)pj[u].y, d2 = x2 - (float)pj[u].z;
+                    hit = hit && (d0 * d0 + d1 * d1) + d2 * d2 <= w.r2;
+                } else {
+                    hit = hit && within<R>(xi - xyz<R>(pj[u]), w);
+                }
+                uint32_t e = j[u];
+                if (hit && w.regions == 1) {   // one region for all types
+                    const uint8_t tj = type[e];
+                    hit = tj != FS_TYPE_INACTIVE;
+                    if (tj == FS_TYPE_BOUNDARY) e |= kBoundaryBit;
+                }
+                const unsigned bal = (__ballot_sync(all, hit) >> shift) & kMask;
+                const uint32_t at = c + __popc(bal & ((1u << g) - 1u));
+                if (hit) {
+                    if (SORT && at < (uint32_t)kListWindow) {
+                        sorts[threadIdx.x / kGroup].hit[at] = e;
+                        sorts[threadIdx.x / kGroup].host[at] = hidx[e & kIndexMask];
+                    } else if ((int)at < K) {
+                        nbr[(int64_t)at * stride + k] = e;
+                    }
+                }
+                c += __popc(bal);
+            }
+        }
+        __syncwarp();
+    }
+    if (SORT && c > 0) {
+        ListSort& so = sorts[threadIdx.x / kGroup];
+        const int h = (int)min(c, (uint32_t)kListWindow);
+        for (int a = g; a < h; a += kGroup) {
+            const uint32_t mine = so.host[a];
+            int place = a;
+            if (c <= (uint32_t)kListWindow) {
+                place = 0;
+                for (int b = 0; b < h; b++) place += so.host[b] < mine ? 1 : 0;
+            }
+            if (place < K) nbr[(int64_t)place * stride + k] = so.hit[a];
+        }
+    }
+    __syncwarp();
+    if (g == 0 && in) {
+        if (owner && !inside) c = build_list_one<R>(k, pos, type, cell_start, w, rows, nbr, stride, K);
+        count[k] = c;
+        if (SORT && (c > (uint32_t)kListWindow || (owner && !inside)))
+            sort_list_by_host_at(k, nbr, stride, K, count, hidx);
+        note_list_length(c, K, status, sc);
+    }
+}
+
 }  // namespace fsb

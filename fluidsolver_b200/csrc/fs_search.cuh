@@ -322,8 +322,9 @@ __global__ void k_reorder(int64_t n, const uint32_t* FSB_R perm, const V4<R>* FS
 // excluded inactive particles (one entry), keep the radix sort (fs_api.cu).
 //
 // Against the radix path (bounding box, origin, keys, 3 launches per 8-bit
-// digit, reorder, run counts, scan; 8 to 18 launches), a whole search on a B200:
-// SEARCH_FIGURES
+// digit, reorder, run counts, scan; 8 to 18 launches), a whole search with its
+// lists on a B200: the 2D dam of 3,688 particles 67 -> 45 us, 40,000 in 2D 90 ->
+// 53, the 8,000-particle dam 131 -> 64, 100,000 117 -> 79, a million 484 -> 414.
 // ---------------------------------------------------------------------------
 struct SearchState {
     uint32_t box_ticket;     // blocks of k_search_box that are done (its last block clears it)
