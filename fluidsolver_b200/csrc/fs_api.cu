@@ -17,6 +17,7 @@
 #include "fs_search.cuh"
 #include "fs_solvers.cuh"
 #include "fs_entities.cuh"
+#include "fs_cached.cuh"
 #include "fs_gather.cuh"
 #include "fs_io.hpp"
 #include "fs_render.cuh"
@@ -269,7 +270,7 @@ void clear_graphs(fs_ctx* c) {
 fs_status free_all(fs_ctx* c) {
     void* ptrs[] = {c->pos[0], c->pos[1], c->vel[0], c->vel[1], c->acc[0], c->acc[1], c->ext[0], c->ext[1],
                     c->rho[0], c->rho[1], c->p[0], c->p[1], c->type[0], c->type[1], c->hidx[0], c->hidx[1],
-                    c->rho_prev, c->vstar, c->anp, c->err, c->gbnd, c->tile_desc, c->tile_ent, c->keys[0], c->keys[1], c->keys64[0], c->keys64[1],
+                    c->rho_prev, c->vstar, c->anp, c->err, c->gbnd, c->gradients, c->tile_desc, c->tile_ent, c->keys[0], c->keys[1], c->keys64[0], c->keys64[1],
                     c->perm[0], c->perm[1], c->h2d_cell, c->h2d_rank, c->sort_hist, c->hash_table, c->cell_start, c->cell_partials, c->look_tiles, c->search_box, c->search_state, c->bbox, c->grids, c->nbr, c->nbr_count,
                     c->scene_of[0], c->scene_of[1], c->d_scene_offsets,
                     c->csr_offsets, c->csr_members, c->csr_sorted, c->csr_counts, c->staging, c->status, c->small_stamps, c->scalars,
@@ -296,6 +297,7 @@ fs_status ensure_staging(fs_ctx* c, size_t bytes) {
     return FS_OK;
 }
 
+constexpr size_t kGradientBytes = size_t(6) << 30;        // stored gradients at most
 fs_status ensure_lists(fs_ctx* c, int K) {
     const int64_t stride = ((c->cap + 31) / 32) * 32;
     const bool tiled = tiled_mode(c);
@@ -307,6 +309,8 @@ fs_status ensure_lists(fs_ctx* c, int K) {
     if (c->nbr) cudaFree(c->nbr);
     if (c->tile_ent) cudaFree(c->tile_ent);
     if (c->tile_desc) cudaFree(c->tile_desc);
+    if (c->gradients) cudaFree(c->gradients);
+    c->gradients = nullptr;
     c->nbr = nullptr;
     c->tile_ent = nullptr;
     c->tile_desc = nullptr;
@@ -319,6 +323,15 @@ fs_status ensure_lists(fs_ctx* c, int K) {
         FS_CUDA(cudaFuncSetAttribute(k_build_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)tile_build_smem(K, kTileCapMax)));
         FS_CUDA(set_tile_pass_smem(K));
+    }
+    // stored gradients of the IISPH gather phases (fs_cached.cuh): up to
+    // kGradientBytes, and as a convenience only (without them the phases
+    // evaluate the kernel)
+    const size_t grad = (size_t)K * stride * 4 * c->real_size;
+    const bool iisph = c->prm.solver == FS_SOLVER_IISPH_3D || c->prm.solver == FS_SOLVER_IISPH_2D;
+    if (!tiled && iisph && grad <= kGradientBytes && cudaMalloc(&c->gradients, grad) != cudaSuccess) {
+        (void)cudaGetLastError();
+        c->gradients = nullptr;
     }
     c->nbr_capacity = K;
     c->nbr_stride = stride;
@@ -1150,12 +1163,23 @@ fs_status step_iisph3d_tiled(fs_ctx* c, bool capture) {
 // below the size where one thread per owner fills the device. B200, one
 // against eight threads: 2D SESPH forces 18.4 -> 8.2 us at 2,500 fluid
 // particles, 20.5 -> 18.4 at 40,000, 22.6 -> 24.5 at 67,600 (3D, 50,000: 74 ->
-// 41); a 2D IISPH iteration 39 -> 22 at 2,500, 44 -> 48 at 25,600; a 3D one 60
-// -> 25 at 8,000, 66 -> 48 at 32,800, 77 -> 104 at 100,000, in FP64 83 -> 51 at
-// 20,700 and 93 -> 92 at 50,700.
+// 41); the 2D IISPH loops 35 -> 16 at 2,500, 37 -> 31 at 25,600, 37 -> 39 at
+// 40,000; the 3D first loop 66 -> 21 at 8,000, 76 -> 51 at 50,700 (FP64 78 -> 86).
 bool grouped(const fs_ctx* c) {
-    const int64_t most = c->prm.solver == FS_SOLVER_IISPH_2D ? 24576 : (c->prm.solver == FS_SOLVER_IISPH_3D ? 45056 : 65536);
-    return c->n_fluid <= most;
+    switch (c->prm.solver) {
+        case FS_SOLVER_IISPH_2D: return c->n_fluid <= 32768;
+        case FS_SOLVER_IISPH_3D: return c->n_fluid <= (c->precision == FS_PRECISION_FP64 ? 45056 : 65536);
+        default: return c->n_fluid <= 65536;
+    }
+}
+// The same for the IISPH second loop and pressure iterations, whose terms are
+// cheaper on stored gradients: a 3D iteration 32.2 -> 19.2 us at 8,000, 32.3 ->
+// 27.1 at 15,000, 33.3 -> 36.6 at 24,400 (FP64 37.4 -> 21.7, 37.4 -> 30.7, 42.1 ->
+// 69.0 at 50,700); without them 60 -> 25 at 8,000, 66 -> 48 at 32,800, 77 -> 104 at
+// 100,000. In 2D (one thread per owner evaluates) 40 -> 18 at 2,500, 42 -> 39 at
+// 25,600, 43 -> 49 at 40,000.
+bool grouped_pressure(const fs_ctx* c) {
+    return c->n_fluid <= (c->prm.solver == FS_SOLVER_IISPH_2D ? 32768 : (c->gradients ? 20480 : 45056));
 }
 
 template <typename R, bool KAHAN> fs_status step_iisph3d(fs_ctx* c, bool capture) {
@@ -1171,16 +1195,25 @@ template <typename R, bool KAHAN> fs_status step_iisph3d(fs_ctx* c, bool capture
     // density double buffer: the current density becomes rho_prev
     std::swap(c->rho[c->cur], c->rho_prev);
     State<R> s = state_of<R>(c);
-    const bool group = grouped(c);
+    const bool group = grouped(c), group_p = grouped_pressure(c), cached = c->gradients != nullptr;
+    const Gradients<R> G{(V4<R>*)c->gradients};
     const unsigned gn = group_grid(n), go = group_grid(no);
     FS_TRY(mark(c, 1, st));
     if (group && split) {
         c->launches += 2;
         k_group_iisph_density<R, KAHAN, true><<<gn, kGroupThreads, 0, st>>>(n, s, L, k, c->status);
-        k_group_iisph_l1<R, KAHAN, true, false><<<gn, kGroupThreads, 0, st>>>(n, s, L, k, c->scalars, c->status);
+        k_group_iisph_l1<R, KAHAN, true, false><<<gn, kGroupThreads, 0, st>>>(n, s, L, k, G, c->scalars, c->status);
     } else if (group) {
         c->launches++;
-        k_group_iisph_l1<R, KAHAN, false, false><<<gn, kGroupThreads, 0, st>>>(n, s, L, k, c->scalars, c->status);
+        k_group_iisph_l1<R, KAHAN, false, false><<<gn, kGroupThreads, 0, st>>>(n, s, L, k, G, c->scalars, c->status);
+    } else if (cached) {
+        c->launches += split ? 2 : 1;
+        if (split) {
+            k_iisph3d_density<R, KAHAN><<<grid_for(n), kBlock, 0, st>>>(n, s, L, k, c->status);
+            k_cached_iisph3d_l1<R, KAHAN, true><<<grid_for(n), kBlock, 0, st>>>(n, s, L, k, G, c->scalars, c->status);
+        } else {
+            k_cached_iisph3d_l1<R, KAHAN, false><<<grid_for(n), kBlock, 0, st>>>(n, s, L, k, G, c->scalars, c->status);
+        }
     } else if (split) {
     c->launches++;
         k_iisph3d_density<R, KAHAN><<<grid_for(n), kBlock, 0, st>>>(n, s, L, k, c->status);
@@ -1192,10 +1225,15 @@ template <typename R, bool KAHAN> fs_status step_iisph3d(fs_ctx* c, bool capture
     }
     FS_CUDA(cudaGetLastError());
     FS_TRY(mark(c, 2, st));
-    if (group) {
+    if (group_p) {
         c->launches++;
-        if (fp32) k_group_iisph3d_l2<R, KAHAN, true><<<go, kGroupThreads, 0, st>>>(no, s, L, k, c->scalars, c->status);
-        else k_group_iisph3d_l2<R, KAHAN, false><<<go, kGroupThreads, 0, st>>>(no, s, L, k, c->scalars, c->status);
+        auto* l2 = fp32 ? (G.g ? k_group_iisph3d_l2<R, KAHAN, true, true> : k_group_iisph3d_l2<R, KAHAN, true, false>)
+                        : (G.g ? k_group_iisph3d_l2<R, KAHAN, false, true> : k_group_iisph3d_l2<R, KAHAN, false, false>);
+        l2<<<go, kGroupThreads, 0, st>>>(no, s, L, k, G, c->scalars, c->status);
+    } else if (cached) {
+        c->launches++;
+        if (fp32) k_cached_iisph3d_l2<R, KAHAN, true><<<grid_for(no), kBlock, 0, st>>>(no, s, L, k, G, c->scalars, c->status);
+        else k_cached_iisph3d_l2<R, KAHAN, false><<<grid_for(no), kBlock, 0, st>>>(no, s, L, k, G, c->scalars, c->status);
     } else if (fp32) {
     c->launches++;
         k_iisph3d_l2<R, KAHAN, true><<<grid_for(no), kBlock, 0, st>>>(no, s, L, k, c->scalars, c->status);
@@ -1207,9 +1245,16 @@ template <typename R, bool KAHAN> fs_status step_iisph3d(fs_ctx* c, bool capture
     FS_TRY(mark(c, 3, st));
     FS_TRY(enqueue_pressure_loop(c, capture, false, !fp32, [&](cudaStream_t bs) {
         c->launches += 2;
-        if (group) {
-            k_group_iisph3d_pressure_acc<R, KAHAN><<<go, kGroupThreads, 0, bs>>>(no, s, L, k, c->scalars, c->status);
-            k_group_iisph3d_pressure_update<R, KAHAN><<<go, kGroupThreads, 0, bs>>>(no, s, L, k, c->scalars, c->status);
+        if (group_p) {
+            auto* acc = G.g ? k_group_iisph3d_pressure_acc<R, KAHAN, true> : k_group_iisph3d_pressure_acc<R, KAHAN, false>;
+            auto* upd = G.g ? k_group_iisph3d_pressure_update<R, KAHAN, true>
+                            : k_group_iisph3d_pressure_update<R, KAHAN, false>;
+            acc<<<go, kGroupThreads, 0, bs>>>(no, s, L, k, G, c->scalars, c->status);
+            upd<<<go, kGroupThreads, 0, bs>>>(no, s, L, k, G, c->scalars, c->status);
+        } else if (cached) {
+            k_cached_iisph3d_pressure_acc<R, KAHAN><<<grid_for(no), kBlock, 0, bs>>>(no, s, L, k, G, c->scalars, c->status);
+            k_cached_iisph3d_pressure_update<R, KAHAN><<<grid_for(no), kBlock, 0, bs>>>(no, s, L, k, G, c->scalars,
+                                                                                        c->status);
         } else {
             k_iisph3d_pressure_acc<R, KAHAN><<<grid_for(no), kBlock, 0, bs>>>(no, s, L, k, c->scalars, c->status);
             k_iisph3d_pressure_update<R, KAHAN><<<grid_for(no), kBlock, 0, bs>>>(no, s, L, k, c->scalars, c->status);
@@ -1309,15 +1354,16 @@ template <typename R, bool KAHAN> fs_status step_iisph2d(fs_ctx* c, bool capture
     std::swap(c->rho[c->cur], c->rho_prev);
     State<R> s = state_of<R>(c);
     const bool group = grouped(c);
+    const Gradients<R> G{(V4<R>*)c->gradients};
     const unsigned gn = group_grid(n), go = group_grid(no);
     FS_TRY(mark(c, 1, st));
     if (group && split) {
         c->launches += 2;
         k_group_iisph_density<R, KAHAN, false><<<gn, kGroupThreads, 0, st>>>(n, s, L, k, c->status);
-        k_group_iisph_l1<R, KAHAN, true, true><<<gn, kGroupThreads, 0, st>>>(n, s, L, k, c->scalars, c->status);
+        k_group_iisph_l1<R, KAHAN, true, true><<<gn, kGroupThreads, 0, st>>>(n, s, L, k, G, c->scalars, c->status);
     } else if (group) {
         c->launches++;
-        k_group_iisph_l1<R, KAHAN, false, true><<<gn, kGroupThreads, 0, st>>>(n, s, L, k, c->scalars, c->status);
+        k_group_iisph_l1<R, KAHAN, false, true><<<gn, kGroupThreads, 0, st>>>(n, s, L, k, G, c->scalars, c->status);
     } else if (split) {
     c->launches++;
         k_iisph2d_density<R, KAHAN><<<grid_for(n), kBlock, 0, st>>>(n, s, L, k, c->status);
@@ -1329,7 +1375,10 @@ template <typename R, bool KAHAN> fs_status step_iisph2d(fs_ctx* c, bool capture
     }
     FS_TRY(mark(c, 2, st));
     c->launches++;
-    if (group) k_group_iisph2d_l2<R, KAHAN><<<go, kGroupThreads, 0, st>>>(no, s, L, k, c->scalars, c->status);
+    if (group) {
+        auto* l2 = G.g ? k_group_iisph2d_l2<R, KAHAN, true> : k_group_iisph2d_l2<R, KAHAN, false>;
+        l2<<<go, kGroupThreads, 0, st>>>(no, s, L, k, G, c->scalars, c->status);
+    }
     else k_iisph2d_l2<R, KAHAN><<<grid_for(no), kBlock, 0, st>>>(no, s, L, k, c->scalars, c->status);
     FS_CUDA(cudaGetLastError());
     FS_TRY(mark(c, 3, st));
@@ -1337,8 +1386,11 @@ template <typename R, bool KAHAN> fs_status step_iisph2d(fs_ctx* c, bool capture
                                  [&](cudaStream_t bs) {
         c->launches += 2;
         if (group) {
-            k_group_iisph2d_pressure_acc<R, KAHAN><<<go, kGroupThreads, 0, bs>>>(no, s, L, k, c->scalars, c->status);
-            k_group_iisph2d_pressure_update<R, KAHAN><<<go, kGroupThreads, 0, bs>>>(no, s, L, k, c->scalars, c->status);
+            auto* acc = G.g ? k_group_iisph2d_pressure_acc<R, KAHAN, true> : k_group_iisph2d_pressure_acc<R, KAHAN, false>;
+            auto* upd = G.g ? k_group_iisph2d_pressure_update<R, KAHAN, true>
+                            : k_group_iisph2d_pressure_update<R, KAHAN, false>;
+            acc<<<go, kGroupThreads, 0, bs>>>(no, s, L, k, G, c->scalars, c->status);
+            upd<<<go, kGroupThreads, 0, bs>>>(no, s, L, k, G, c->scalars, c->status);
         } else {
             k_iisph2d_pressure_acc<R, KAHAN><<<grid_for(no), kBlock, 0, bs>>>(no, s, L, k, c->scalars, c->status);
             k_iisph2d_pressure_update<R, KAHAN><<<grid_for(no), kBlock, 0, bs>>>(no, s, L, k, c->scalars, c->status);

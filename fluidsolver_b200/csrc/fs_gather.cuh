@@ -16,6 +16,7 @@
 // latency: fs_api.cu (grouped) has the sizes and both sides' times.
 #pragma once
 
+#include "fs_cached.cuh"
 #include "fs_common.cuh"
 #include "fs_solvers.cuh"
 
@@ -42,8 +43,8 @@ __device__ __forceinline__ int64_t group_owner() {
 }
 
 // Adds the terms of the first n entries of owner k's list to the sums: lane c
-// of the group holds sum c in acc. load(j): the fields of neighbor j;
-// term(entry, fields, t): the entry's NC terms, and which of them count: bit 0
+// of the group holds sum c in acc. load(j, at): the fields of neighbor j, the
+// entry lying at `at` in the lists (-1: none, j is then 0); term(entry, fields, t): the entry's NC terms, and which of them count: bit 0
 // for t[0 .. H), bit 1 for t[H .. NC). INTERLEAVED: two terms per entry of one
 // sum, t[0] then t[1], held by lane 0. Every thread of the warp calls it.
 template <int NC, int H, bool INTERLEAVED = false, typename R, bool KAHAN, typename Load, typename Term>
@@ -55,14 +56,16 @@ __device__ __forceinline__ void group_sum(const Lists& L, int64_t k, uint32_t n,
     const uint32_t most = __reduce_max_sync(all, n);
     for (uint32_t base = 0; base < most; base += kWindow) {
         uint32_t e[kRounds];
-        decltype(load(0u)) d[kRounds];
+        decltype(load(0u, (int64_t)0)) d[kRounds];
+        int64_t at[kRounds];
 #pragma unroll
         for (int r = 0; r < kRounds; r++) {
             const uint32_t q = base + r * kGroup + g;
-            e[r] = q < n ? FSB_LDG(&L.nbr[(int64_t)q * L.stride + k]) : 0u;
+            at[r] = q < n ? (int64_t)q * L.stride + k : -1;
+            e[r] = q < n ? FSB_LDG(&L.nbr[at[r]]) : 0u;
         }
 #pragma unroll
-        for (int r = 0; r < kRounds; r++) d[r] = load(e[r] & kIndexMask);
+        for (int r = 0; r < kRounds; r++) d[r] = load(e[r] & kIndexMask, at[r]);
         uint32_t lo = 0, hi = 0;
 #pragma unroll
         for (int r = 0; r < kRounds; r++) {
@@ -115,11 +118,23 @@ template <typename R> struct GPosScalar {
 template <typename R> struct GVisc {
     V4<R> x, v;
     R rho;
+    int64_t at;
 };
 template <typename R> struct GForce {
     V4<R> x, v;
     R rho, p;
 };
+
+// CACHED: the stored gradient and mass of the entry (fs_cached.cuh) instead of
+// the neighbor's position and mass; then gradW of either
+template <bool CACHED, typename R>
+__device__ __forceinline__ V4<R> position_or_gradient(const State<R>& s, const Gradients<R>& G, uint32_t j, int64_t at) {
+    return CACHED ? G.g[at < 0 ? 0 : at] : s.pos[j];
+}
+template <bool CACHED, bool KAHAN, typename R>
+__device__ __forceinline__ V3<R> gradient_of(const SolverConsts<R>& c, V3<R> xk, const V4<R>& x) {
+    return CACHED ? xyz<R>(x) : c.kern.template grad<KAHAN>(xk - xyz<R>(x));
+}
 
 // the viscosity term of neighbor (xj, vj, rj) without the factor 2 nu
 // (viscosity() in fs_solvers.cuh); false where the density is 0
@@ -152,7 +167,7 @@ template <typename R, bool KAHAN, bool GAMMA>
 __device__ __forceinline__ R group_density(int64_t k, uint32_t n, V3<R> xk, const State<R>& s, const Lists& L,
                                            const SolverConsts<R>& c, GroupRows<R, 1>& rows) {
     Acc<R, KAHAN> acc;
-    group_sum<1, 1>(L, k, n, rows, acc, [&](uint32_t j) { return GPos<R>{s.pos[j]}; },
+    group_sum<1, 1>(L, k, n, rows, acc, [&](uint32_t j, int64_t) { return GPos<R>{s.pos[j]}; },
                     [&](uint32_t e, const GPos<R>& d, R* t) {
                         R m = d.x.w;
                         if (GAMMA && c.single_layer && (e & kBoundaryBit)) m = m * c.gamma1;
@@ -209,7 +224,7 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_sesph_accel(int64_t n, 
     const R pdd = rk == R(0) ? R(0) : s.p[kk] / (rk * rk);
     Acc<R, KAHAN> acc;   // viscosity 0-2, pressure 3-5
     group_sum<6, 3>(L, kk, fluid ? L.size(kk) : 0u, rows[threadIdx.x / kGroup], acc,
-                    [&](uint32_t j) { return GForce<R>{s.pos[j], s.vel[j], s.rho[j], s.p[j]}; },
+                    [&](uint32_t j, int64_t) { return GForce<R>{s.pos[j], s.vel[j], s.rho[j], s.p[j]}; },
                     [&](uint32_t e, const GForce<R>& d, R* t) {
                         const V3<R> xij = xk - xyz<R>(d.x);
                         const V3<R> g = c.kern.template grad<KAHAN>(xij);
@@ -235,12 +250,13 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_sesph_accel(int64_t n, 
 // ---------------------------------------------------------------------------
 // IISPH first loop (iisph3d_l1_one, iisph2d_l1_at)
 // ---------------------------------------------------------------------------
+// Stores the gradients where the context keeps them (G.g not null).
 // TWO_D: IISPHFluidSolver's loop (no pressure reset, no a_np; a particle's own
 // density is the new one). SPLIT: the density has run before, and viscosity
 // reads a fluid neighbor with a smaller host index at its new density.
 template <typename R, bool KAHAN, bool SPLIT, bool TWO_D>
 __global__ void __launch_bounds__(kGroupThreads) k_group_iisph_l1(int64_t n, State<R> s, Lists L, SolverConsts<R> c,
-                                                                  const StepScalars* FSB_R sc,
+                                                                  Gradients<R> G, const StepScalars* FSB_R sc,
                                                                   const int* FSB_R status) {
     __shared__ GroupRows<R, 3> rows3[kGroupsPerBlock];
     __shared__ GroupRows<R, 1> rows1[SPLIT ? 1 : kGroupsPerBlock];
@@ -262,18 +278,19 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph_l1(int64_t n, Sta
     const uint32_t hk = SPLIT ? s.hidx[kk] : 0u;
     Acc<R, KAHAN> acc;
     group_sum<3, 3>(L, kk, nn, rows3[threadIdx.x / kGroup], acc,
-                    [&](uint32_t j) {
+                    [&](uint32_t j, int64_t at) {
                         R rj = s.rho_prev[j];
                         // (a boundary particle's density is the same in both)
                         if (SPLIT && s.hidx[j] < hk) rj = s.rho[j];
-                        return GVisc<R>{s.pos[j], s.vel[j], rj};
+                        return GVisc<R>{s.pos[j], s.vel[j], rj, at};
                     },
                     [&](uint32_t e, const GVisc<R>& d, R* t) {
                         const V3<R> xij = xyz<R>(pk) - xyz<R>(d.x);
                         R rj = d.rho;
                         if (TWO_D && (e & kIndexMask) == (uint32_t)k) rj = rk;
-                        return viscosity_term<R, KAHAN>(c, xij, c.kern.template grad<KAHAN>(xij),
-                                                        xyz<R>(vk) - xyz<R>(d.v), d.x.w, rj, t) ? 1u : 0u;
+                        const V3<R> g = c.kern.template grad<KAHAN>(xij);
+                        if (G.g && d.at >= 0) G.g[d.at] = v4<R>(g, d.x.w);   // for the passes that follow
+                        return viscosity_term<R, KAHAN>(c, xij, g, xyz<R>(vk) - xyz<R>(d.v), d.x.w, rj, t) ? 1u : 0u;
                     });
     const V3<R> visc = group_total3(acc, 0);
     if (!in || group_lane() != 0) return;
@@ -296,8 +313,8 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph_l1(int64_t n, Sta
 // ---------------------------------------------------------------------------
 // IISPH 3D second loop and pressure iteration (iisph3d_l2_one, ...)
 // ---------------------------------------------------------------------------
-template <typename R, bool KAHAN, bool TWO_PASS>
-__global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_l2(int64_t n, State<R> s, Lists L, SolverConsts<R> c,
+template <typename R, bool KAHAN, bool TWO_PASS, bool CACHED>
+__global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_l2(int64_t n, State<R> s, Lists L, SolverConsts<R> c, Gradients<R> G,
                                                                     const StepScalars* FSB_R sc,
                                                                     const int* FSB_R status) {
     constexpr int NC = TWO_PASS ? 4 : 8;
@@ -312,9 +329,11 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_l2(int64_t n, S
     // contrib 0, inner 1-3; in the single pass sum m gradW 4-6 and sum_fluid m |gradW|^2 7
     Acc<R, KAHAN> acc;
     group_sum<NC, TWO_PASS ? NC : 7>(L, kk, nn, rows[threadIdx.x / kGroup], acc,
-                                     [&](uint32_t j) { return GPosVec<R>{s.pos[j], s.vstar[j]}; },
+                                     [&](uint32_t j, int64_t at) {
+                                         return GPosVec<R>{position_or_gradient<CACHED>(s, G, j, at), s.vstar[j]};
+                                     },
                                      [&](uint32_t e, const GPosVec<R>& d, R* t) {
-        const V3<R> g = c.kern.template grad<KAHAN>(xk - xyz<R>(d.x));
+        const V3<R> g = gradient_of<CACHED, KAHAN>(c, xk, d.x);
         const bool bnd = (e & kBoundaryBit) != 0u;
         V3<R> in;
         if (!bnd) {
@@ -340,9 +359,9 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_l2(int64_t n, S
         __shared__ GroupRows<R, 2> rows2[kGroupsPerBlock];
         Acc<R, KAHAN> d;
         const R mi = pk.w / c.rho0_sq;
-        group_sum<2, 1, true>(L, kk, nn, rows2[threadIdx.x / kGroup], d, [&](uint32_t j) { return GPos<R>{s.pos[j]}; },
+        group_sum<2, 1, true>(L, kk, nn, rows2[threadIdx.x / kGroup], d, [&](uint32_t j, int64_t at) { return GPos<R>{position_or_gradient<CACHED>(s, G, j, at)}; },
                               [&](uint32_t e, const GPos<R>& q, R* t) {
-            const V3<R> g = c.kern.template grad<KAHAN>(xk - xyz<R>(q.x));
+            const V3<R> g = gradient_of<CACHED, KAHAN>(c, xk, q.x);
             t[0] = q.x.w * dot(in, g);
             t[1] = q.x.w * dot(mi * (-g), g);
             return (e & kBoundaryBit) ? 1u : 3u;
@@ -359,9 +378,9 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_l2(int64_t n, S
     s.anp[k].w = diag;
 }
 
-template <typename R, bool KAHAN>
+template <typename R, bool KAHAN, bool CACHED>
 __global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_pressure_acc(int64_t n, State<R> s, Lists L,
-                                                                              SolverConsts<R> c,
+                                                                              SolverConsts<R> c, Gradients<R> G,
                                                                               const StepScalars* FSB_R sc,
                                                                               const int* FSB_R status) {
     __shared__ GroupRows<R, 3> rows[kGroupsPerBlock];
@@ -374,9 +393,9 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_pressure_acc(in
     const R qk = pk / c.rho0_sq;
     Acc<R, KAHAN> acc;
     group_sum<3, 3>(L, kk, fluid ? L.size(kk) : 0u, rows[threadIdx.x / kGroup], acc,
-                    [&](uint32_t j) { return GPosScalar<R>{s.pos[j], s.p[j]}; },
+                    [&](uint32_t j, int64_t at) { return GPosScalar<R>{position_or_gradient<CACHED>(s, G, j, at), s.p[j]}; },
                     [&](uint32_t e, const GPosScalar<R>& d, R* t) {
-        const V3<R> g = c.kern.template grad<KAHAN>(xk - xyz<R>(d.x));
+        const V3<R> g = gradient_of<CACHED, KAHAN>(c, xk, d.x);
         const bool bnd = (e & kBoundaryBit) != 0u;
         V3<R> v;
         if (KAHAN) {
@@ -396,9 +415,9 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_pressure_acc(in
     if (fluid && group_lane() == 0) s.acc[k] = v4<R>(a, R(0));
 }
 
-template <typename R, bool KAHAN>
+template <typename R, bool KAHAN, bool CACHED>
 __global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_pressure_update(int64_t n, State<R> s, Lists L,
-                                                                                 SolverConsts<R> c,
+                                                                                 SolverConsts<R> c, Gradients<R> G,
                                                                                  StepScalars* FSB_R sc,
                                                                                  const int* FSB_R status) {
     __shared__ GroupRows<R, 1> rows[kGroupsPerBlock];
@@ -409,9 +428,9 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_pressure_update
     const V3<R> xk = xyz<R>(s.pos[kk]), ak = xyz<R>(s.acc[kk]);
     Acc<R, KAHAN> acc;
     group_sum<1, 1>(L, kk, fluid ? L.size(kk) : 0u, rows[threadIdx.x / kGroup], acc,
-                    [&](uint32_t j) { return GPosVec<R>{s.pos[j], s.acc[j]}; },
+                    [&](uint32_t j, int64_t at) { return GPosVec<R>{position_or_gradient<CACHED>(s, G, j, at), s.acc[j]}; },
                     [&](uint32_t e, const GPosVec<R>& d, R* t) {
-        const V3<R> g = c.kern.template grad<KAHAN>(xk - xyz<R>(d.x));
+        const V3<R> g = gradient_of<CACHED, KAHAN>(c, xk, d.x);
         t[0] = d.x.w * ((e & kBoundaryBit) ? dotf<KAHAN>(ak, g) : dotf<KAHAN>(ak - xyz<R>(d.v), g));
         return 1u;
     });
@@ -425,8 +444,8 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_pressure_update
 // ---------------------------------------------------------------------------
 // IISPH 2D second loop and pressure iteration (iisph2d_l2_at, ...)
 // ---------------------------------------------------------------------------
-template <typename R, bool KAHAN>
-__global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_l2(int64_t n, State<R> s, Lists L, SolverConsts<R> c,
+template <typename R, bool KAHAN, bool CACHED>
+__global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_l2(int64_t n, State<R> s, Lists L, SolverConsts<R> c, Gradients<R> G,
                                                                     const StepScalars* FSB_R sc,
                                                                     const int* FSB_R status) {
     __shared__ GroupRows<R, 4> rows[kGroupsPerBlock];
@@ -440,9 +459,11 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_l2(int64_t n, S
     const V3<R> xk = xyz<R>(pk), vsk = xyz<R>(s.vstar[kk]);
     Acc<R, KAHAN> acc;   // sum 0, internal 1-3
     group_sum<4, 4>(L, kk, nn, rows[threadIdx.x / kGroup], acc,
-                    [&](uint32_t j) { return GPosVec<R>{s.pos[j], s.vstar[j]}; },
+                    [&](uint32_t j, int64_t at) {
+                                         return GPosVec<R>{position_or_gradient<CACHED>(s, G, j, at), s.vstar[j]};
+                                     },
                     [&](uint32_t e, const GPosVec<R>& d, R* t) {
-        const V3<R> g = c.kern.template grad<KAHAN>(xk - xyz<R>(d.x));
+        const V3<R> g = gradient_of<CACHED, KAHAN>(c, xk, d.x);
         t[0] = d.x.w * dot(vsk - xyz<R>(d.v), g);
         if (!(e & kBoundaryBit)) put3(t + 1, ((d.x.w / c.rest_density) / c.rest_density) * g);
         else put3(t + 1, (((c.two_gamma * d.x.w) / c.rest_density) / c.rest_density) * g);
@@ -451,15 +472,15 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_l2(int64_t n, S
     const R sum = group_total(acc, 0);
     const V3<R> neg_in = -group_total3(acc, 1);
     const R mi = (pk.w / c.rest_density) / c.rest_density;
-    auto pos = [&](uint32_t j) { return GPos<R>{s.pos[j]}; };
+    auto pos = [&](uint32_t j, int64_t at) { return GPos<R>{position_or_gradient<CACHED>(s, G, j, at)}; };
     GroupRows<R, 1>& row = rows1[threadIdx.x / kGroup];
     Acc<R, KAHAN> d;   // over every neighbor, then over the fluid ones
     group_sum<1, 1>(L, kk, nn, row, d, pos, [&](uint32_t, const GPos<R>& q, R* t) {
-        t[0] = q.x.w * dot(neg_in, c.kern.template grad<KAHAN>(xk - xyz<R>(q.x)));
+        t[0] = q.x.w * dot(neg_in, gradient_of<CACHED, KAHAN>(c, xk, q.x));
         return 1u;
     });
     group_sum<1, 1>(L, kk, nn, row, d, pos, [&](uint32_t e, const GPos<R>& q, R* t) {
-        const V3<R> g = c.kern.template grad<KAHAN>(xk - xyz<R>(q.x));
+        const V3<R> g = gradient_of<CACHED, KAHAN>(c, xk, q.x);
         t[0] = q.x.w * dot(mi * (-g), g);
         return (e & kBoundaryBit) ? 0u : 1u;
     });
@@ -472,9 +493,9 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_l2(int64_t n, S
     s.p[k] = R(0);
 }
 
-template <typename R, bool KAHAN>
+template <typename R, bool KAHAN, bool CACHED>
 __global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_pressure_acc(int64_t n, State<R> s, Lists L,
-                                                                              SolverConsts<R> c,
+                                                                              SolverConsts<R> c, Gradients<R> G,
                                                                               const StepScalars* FSB_R sc,
                                                                               const int* FSB_R status) {
     __shared__ GroupRows<R, 3> rows[kGroupsPerBlock];
@@ -486,9 +507,9 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_pressure_acc(in
     const R pr = (s.p[kk] / c.rest_density) / c.rest_density;
     Acc<R, KAHAN> acc;
     group_sum<3, 3>(L, kk, fluid ? L.size(kk) : 0u, rows[threadIdx.x / kGroup], acc,
-                    [&](uint32_t j) { return GPosScalar<R>{s.pos[j], s.p[j]}; },
+                    [&](uint32_t j, int64_t at) { return GPosScalar<R>{position_or_gradient<CACHED>(s, G, j, at), s.p[j]}; },
                     [&](uint32_t e, const GPosScalar<R>& d, R* t) {
-        const V3<R> g = c.kern.template grad<KAHAN>(xk - xyz<R>(d.x));
+        const V3<R> g = gradient_of<CACHED, KAHAN>(c, xk, d.x);
         if (!(e & kBoundaryBit)) put3(t, (d.x.w * (pr + (d.a / c.rest_density) / c.rest_density)) * g);
         else put3(t, (((c.gamma * d.x.w) * R(2)) * pr) * g);
         return 1u;
@@ -497,9 +518,9 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_pressure_acc(in
     if (fluid && group_lane() == 0) s.acc[k] = v4<R>(-a, R(0));
 }
 
-template <typename R, bool KAHAN>
+template <typename R, bool KAHAN, bool CACHED>
 __global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_pressure_update(int64_t n, State<R> s, Lists L,
-                                                                                 SolverConsts<R> c,
+                                                                                 SolverConsts<R> c, Gradients<R> G,
                                                                                  StepScalars* FSB_R sc,
                                                                                  const int* FSB_R status) {
     __shared__ GroupRows<R, 1> rows[kGroupsPerBlock];
@@ -510,9 +531,9 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_pressure_update
     const V3<R> xk = xyz<R>(s.pos[kk]), ak = xyz<R>(s.acc[kk]);
     Acc<R, KAHAN> acc;
     group_sum<1, 1>(L, kk, fluid ? L.size(kk) : 0u, rows[threadIdx.x / kGroup], acc,
-                    [&](uint32_t j) { return GPosVec<R>{s.pos[j], s.acc[j]}; },
+                    [&](uint32_t j, int64_t at) { return GPosVec<R>{position_or_gradient<CACHED>(s, G, j, at), s.acc[j]}; },
                     [&](uint32_t e, const GPosVec<R>& d, R* t) {
-        const V3<R> g = c.kern.template grad<KAHAN>(xk - xyz<R>(d.x));
+        const V3<R> g = gradient_of<CACHED, KAHAN>(c, xk, d.x);
         t[0] = d.x.w * ((e & kBoundaryBit) ? dot(ak, g) : dot(ak - xyz<R>(d.v), g));
         return 1u;
     });

@@ -44,7 +44,7 @@ struct Lists {
 // order) is unchanged.
 constexpr int kBatch = 4;
 template <typename R, typename F>
-__device__ __forceinline__ void for_neighbors(const Lists& L, int64_t k, const V4<R>* FSB_R pos, F&& f) {
+__device__ __forceinline__ void for_neighbors_at(const Lists& L, int64_t k, const V4<R>* FSB_R pos, F&& f) {
     const uint32_t n = L.size(k);
     uint32_t q = 0;
     for (; q + kBatch <= n; q += kBatch) {
@@ -55,12 +55,16 @@ __device__ __forceinline__ void for_neighbors(const Lists& L, int64_t k, const V
 #pragma unroll
         for (int b = 0; b < kBatch; b++) p[b] = pos[e[b] & kIndexMask];
 #pragma unroll
-        for (int b = 0; b < kBatch; b++) f(e[b], p[b]);
+        for (int b = 0; b < kBatch; b++) f(q + b, e[b], p[b]);
     }
     for (; q < n; q++) {
         const uint32_t e = FSB_LDG(&L.nbr[(int64_t)q * L.stride + k]);
-        f(e, pos[e & kIndexMask]);
+        f(q, e, pos[e & kIndexMask]);
     }
+}
+template <typename R, typename F>
+__device__ __forceinline__ void for_neighbors(const Lists& L, int64_t k, const V4<R>* FSB_R pos, F&& f) {
+    for_neighbors_at<R>(L, k, pos, [&](uint32_t, uint32_t e, const V4<R>& pj) { f(e, pj); });
 }
 
 // As for_neighbors, also handing d = x_k - x_j and gradW(d).
@@ -120,11 +124,18 @@ __device__ __forceinline__ float warp_max(float v) {
 //   return (2 nu) * tmp
 // rho_of(j, entry) supplies the neighbor density the reference reads.
 // ===========================================================================
-template <typename R, bool KAHAN, typename RhoOf>
+struct NoSink {
+    template <typename A, typename B> __device__ __forceinline__ void operator()(uint32_t, const A&, const B&) const {}
+};
+// sink(q, gradW, pj): called for every entry q of the list
+template <typename R, bool KAHAN, typename RhoOf, typename Sink = NoSink>
 __device__ __forceinline__ V3<R> viscosity(int64_t k, const State<R>& s, const Lists& L, const SolverConsts<R>& c,
-                                           V3<R> xi, V3<R> vi, RhoOf&& rho_of) {
+                                           V3<R> xi, V3<R> vi, RhoOf&& rho_of, Sink&& sink = Sink()) {
     Acc3<R, KAHAN> tmp;
-    for_neighbors_grad<R, KAHAN>(L, k, s.pos, xi, c.kern, [&](uint32_t e, const V4<R>& pj, V3<R> xij, V3<R> g) {
+    for_neighbors_at<R>(L, k, s.pos, [&](uint32_t q, uint32_t e, const V4<R>& pj) {
+        const V3<R> xij = xi - xyz<R>(pj);
+        const V3<R> g = c.kern.template grad<KAHAN>(xij);
+        sink(q, g, pj);
         const uint32_t j = e & kIndexMask;
         const R rj = rho_of(j, e);
         if (rj == R(0)) return;
@@ -147,9 +158,9 @@ __device__ __forceinline__ V3<R> viscosity(int64_t k, const State<R>& s, const L
 //                the previous one otherwise -- the order the reference's serial
 //                loop produces (it overwrites densities while reading them).
 // ===========================================================================
-template <typename R, bool KAHAN, bool SPLIT>
+template <typename R, bool KAHAN, bool SPLIT, typename Sink = NoSink>
 __device__ __forceinline__ void iisph3d_l1_one(int64_t k, const State<R>& s, const Lists& L, const SolverConsts<R>& c,
-                                               R dt) {
+                                               R dt, Sink&& sink = Sink()) {
     const uint8_t t = s.type[k];
     if (t == FS_TYPE_INACTIVE) {
         if (!SPLIT) s.rho[k] = s.rho_prev[k];  // carry the density through the double buffer
@@ -167,10 +178,10 @@ __device__ __forceinline__ void iisph3d_l1_one(int64_t k, const State<R>& s, con
             visc = viscosity<R, KAHAN>(k, s, L, c, xyz<R>(pk), xyz<R>(vk), [&](uint32_t j, uint32_t e) -> R {
                 if (!(e & kBoundaryBit) && s.hidx[j] < hk) return s.rho[j];
                 return s.rho_prev[j];
-            });
+            }, sink);
         } else {
             visc = viscosity<R, KAHAN>(k, s, L, c, xyz<R>(pk), xyz<R>(vk),
-                                       [&](uint32_t j, uint32_t) -> R { return s.rho_prev[j]; });
+                                       [&](uint32_t j, uint32_t) -> R { return s.rho_prev[j]; }, sink);
         }
         npa = npa + visc;
     }

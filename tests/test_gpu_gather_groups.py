@@ -50,3 +50,34 @@ def test_groups_equal_single_threads(solver, search, precision, exact, spacing):
         assert ma > 64
     for f in ("position", "velocity", "acceleration", "density", "pressure"):
         assert bits_equal(getattr(a, f), getattr(b, f)), f
+
+
+@pytest.mark.parametrize("precision,exact", [("fp32", True), ("fp64", False), ("fp32", False)])
+def test_stored_gradients_keep_the_sums(precision, exact):
+    """Both forms of the pressure passes on stored gradients (eight threads per owner up to 20,480 fluid particles, one
+    beyond) and both forms of the first loop that stores them (up to 65,536, in FP64 45,056) against each other: the
+    same block of fluid alone and with as many far-away single particles as it takes to change the form."""
+    rng = np.random.default_rng(23)
+    m = 10
+    g = np.stack(np.meshgrid(*[np.arange(m)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    block = (g * 0.9 + rng.uniform(-0.03, 0.03, g.shape)).astype(np.float32)
+    typ = (g[:, 1] == 0).astype(np.uint8)
+    out = []
+    for far in (0, 21000, 66000):
+        side = int(np.ceil(far ** (1 / 3))) or 1
+        grid = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3)[:far]
+        pos = np.concatenate([block, (grid * 5.0 + 30.0).astype(np.float32)])
+        s = make_solver("iisph-3d", "hashed-3d", [0.001, 5, 5, 0.5, 0.7, 0.01, 1.0, 1.1], (0.001, 0.4, 0.25),
+                        precision=precision, reference_order=exact)
+        s.data.collection = ParticleCollection(position=pos, velocity=np.zeros_like(pos),
+                                               mass=np.ones(len(pos), np.float32),
+                                               density=np.ones(len(pos), np.float32),
+                                               type=np.concatenate([typ, np.zeros(far, np.uint8)]))
+        st = s.run(3)
+        assert st.iterations == 5
+        out.append(s.collection())
+        s.close()
+    n = len(block)
+    for other in out[1:]:
+        for f in ("position", "velocity", "acceleration", "density", "pressure"):
+            assert bits_equal(getattr(out[0], f)[:n], getattr(other, f)[:n]), f
