@@ -173,6 +173,9 @@ Lists lists_of(fs_ctx* c) {
 // instead of one of 592) 21.5 and 27.1, 512,000 110.6 and 115.5.
 int tile_cap_of(const fs_ctx* c) {
     if (c->tuning.cap > 0) return c->tuning.cap;
+    // (SESPH has no iterations to gain from it, and its pressure is the
+    // density's small excess, in which another order of the sums shows)
+    if (c->prm.solver != FS_SOLVER_IISPH_3D) return kTileCap;
     const int64_t tiles = (c->n_owners + kTileOwners - 1) / kTileOwners, sms = c->sms;
     auto rounds = [&](int64_t per_sm) { return (tiles + per_sm * sms - 1) / (per_sm * sms); };
     const bool small = tiles <= 2 * sms || (tiles > 4 * sms && rounds(3) <= rounds(4));
