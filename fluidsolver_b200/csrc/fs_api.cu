@@ -286,6 +286,8 @@ fs_status free_all(fs_ctx* c) {
     if (c->body_stream) cudaStreamDestroy(c->body_stream);
     for (auto& e : c->ev)
         if (e) cudaEventDestroy(e);
+    for (cudaEvent_t e : {c->counted, c->copied})
+        if (e) cudaEventDestroy(e);
     if (c->stream) cudaStreamDestroy(c->stream);
     return FS_OK;
 }
@@ -391,7 +393,9 @@ fs_status choose_grids(fs_ctx* c, const int* lo, const int* hi) {
     if (base > (int64_t(1) << 30)) return fail(FS_ERR_INVALID, "the scenes' cell grids exceed 2^30 cells");
     for (int a = 0; a < 3; a++) c->dims[a] = a == 0 ? c->grids_host[0].d0 : (a == 1 ? c->grids_host[0].d1 : c->grids_host[0].d2);
     c->cells = base;
-    FS_CUDA(cudaMemcpyAsync(c->grids, c->grids_host.data(), sizeof(SceneGrid) * S, cudaMemcpyHostToDevice, c->stream));
+    // (a single scene's grid goes with the packing kernel)
+    if (c->scenes > 0)
+        FS_CUDA(cudaMemcpyAsync(c->grids, c->grids_host.data(), sizeof(SceneGrid) * S, cudaMemcpyHostToDevice, c->stream));
     return FS_OK;
 }
 
@@ -435,8 +439,15 @@ __global__ void k_pack(int64_t n, int dim, const float* __restrict__ pos, const 
                        const float* __restrict__ acc, const float* __restrict__ ext, const float* __restrict__ mass,
                        const float* __restrict__ rho, const float* __restrict__ p, const uint8_t* __restrict__ type,
                        float rest_density, State<R> s, uint8_t* __restrict__ type_out, uint32_t* __restrict__ hidx_out,
-                       const int64_t* __restrict__ offsets, int scenes, uint16_t* __restrict__ scene_out) {
+                       const int64_t* __restrict__ offsets, int scenes, uint16_t* __restrict__ scene_out,
+                       SearchState* __restrict__ census, int* __restrict__ box, SceneGrid grid,
+                       SceneGrid* __restrict__ grids) {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    // the census's counts and boxes, read by now, start afresh; a single scene's grid
+    for (int64_t b = i; b < 6 * (int64_t)scenes; b += (int64_t)gridDim.x * blockDim.x)
+        box[b] = b < 3 * scenes ? 0x7f7f7f7f : (int)0x80808080;
+    if (i < 4) census->counts[i] = 0ull;
+    if (i == 0 && grids) grids[0] = grid;
     if (i >= n) return;
     auto ld = [&](const float* a) -> V3<R> {
         if (!a) return v3<R>(R(0), R(0), R(0));
@@ -453,32 +464,43 @@ __global__ void k_pack(int64_t n, int dim, const float* __restrict__ pos, const 
     if (scene_out) scene_out[i] = (uint16_t)scene_of_host(offsets, scenes, i);
 }
 
-// field f of the sorted state, scattered to host order
-template <typename R>
-__global__ void k_unpack(int64_t n, int dim, int field, State<R> s, float* __restrict__ out, uint8_t* __restrict__ out_u8,
-                         uint32_t* __restrict__ out_u32) {
-    int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// fields of the sorted state, scattered to host order (null: not wanted)
+struct UnpackTo {
+    float *position, *velocity, *acceleration, *external, *mass, *density, *pressure;
+    uint8_t* type;
+    uint32_t* tag;
+    float *predicted_velocity, *non_pressure_acceleration, *source_term, *diagonal_element;
+};
+template <typename R> __global__ void k_unpack(int64_t n, int dim, State<R> s, UnpackTo to) {
+    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n) return;
     const uint32_t h = s.hidx[k];
-    auto st = [&](V3<R> v) {
+    auto st = [&](float* out, const V4<R>& v) {
         out[(int64_t)h * dim] = (float)v.x;
         out[(int64_t)h * dim + 1] = (float)v.y;
         if (dim == 3) out[(int64_t)h * dim + 2] = (float)v.z;
     };
-    switch (field) {
-        case 0: st(xyz<R>(s.pos[k])); break;
-        case 1: st(xyz<R>(s.vel[k])); break;
-        case 2: st(xyz<R>(s.acc[k])); break;
-        case 3: st(xyz<R>(s.ext[k])); break;
-        case 4: out[h] = (float)s.pos[k].w; break;
-        case 5: out[h] = (float)s.rho[k]; break;
-        case 6: out[h] = (float)s.p[k]; break;
-        case 7: out_u8[h] = s.type[k]; break;
-        case 8: out_u32[h] = h; break;
-        case 9: st(xyz<R>(s.vstar[k])); break;
-        case 10: st(xyz<R>(s.anp[k])); break;
-        case 11: out[h] = (float)s.vstar[k].w; break;
-        case 12: out[h] = (float)s.anp[k].w; break;
+    if (to.position || to.mass) {
+        const V4<R> x = s.pos[k];
+        if (to.position) st(to.position, x);
+        if (to.mass) to.mass[h] = (float)x.w;
+    }
+    if (to.velocity) st(to.velocity, s.vel[k]);
+    if (to.acceleration) st(to.acceleration, s.acc[k]);
+    if (to.external) st(to.external, s.ext[k]);
+    if (to.density) to.density[h] = (float)s.rho[k];
+    if (to.pressure) to.pressure[h] = (float)s.p[k];
+    if (to.type) to.type[h] = s.type[k];
+    if (to.tag) to.tag[h] = h;
+    if (to.predicted_velocity || to.source_term) {
+        const V4<R> v = s.vstar[k];
+        if (to.predicted_velocity) st(to.predicted_velocity, v);
+        if (to.source_term) to.source_term[h] = (float)v.w;
+    }
+    if (to.non_pressure_acceleration || to.diagonal_element) {
+        const V4<R> v = s.anp[k];
+        if (to.non_pressure_acceleration) st(to.non_pressure_acceleration, v);
+        if (to.diagonal_element) to.diagonal_element[h] = (float)v.w;
     }
 }
 
@@ -486,15 +508,11 @@ __global__ void k_unpack(int64_t n, int dim, int field, State<R> s, float* __res
 // invalid types) and, per axis, the min/max of floor(x / r) over the finite
 // coordinates (|x| < 1e30, clamped to +-1e9) of the particles that take part
 // in the cell structure.
-struct UploadCensus {
-    unsigned long long counts[4];
-};
-
 // one particle per thread; per-scene boxes in bbox (mins [3 scenes], maxs
 // [3 scenes]), reduced per block when the block lies in one scene
 __global__ void k_census(int64_t n, int dim, const float* __restrict__ pos, const uint8_t* __restrict__ type, float r,
                          bool include_inactive, const int64_t* __restrict__ offsets, int scenes,
-                         UploadCensus* __restrict__ out, int* __restrict__ bbox) {
+                         SearchState* __restrict__ out, int* __restrict__ bbox) {
     __shared__ unsigned int s_cnt[4];
     __shared__ int s_first;
     __shared__ int s_b[6][32];
@@ -561,7 +579,6 @@ struct StagedUpload {
     const float *pos = nullptr, *vel = nullptr, *acc = nullptr, *ext = nullptr;
     const float *mass = nullptr, *rho = nullptr, *p = nullptr;
     const uint8_t* type = nullptr;
-    UploadCensus* census = nullptr;
 };
 
 // resets the per-scene box table (mins high, maxs low)
@@ -572,88 +589,144 @@ fs_status reset_bbox(fs_ctx* c) {
     return FS_OK;
 }
 
-// boxes: per-scene census box (mins [3 scenes], maxs [3 scenes])
-fs_status stage_upload(fs_ctx* c, const fs_particles* in, StagedUpload& d, UploadCensus& h, std::vector<int>& boxes) {
+// Enqueues the copies of the host arrays and the census of positions and
+// types, and waits for the census: counts (per type, index 3: invalid) and
+// per-scene boxes (mins [3 scenes], maxs [3 scenes]) in c->upload_host. The
+// positions and types go first, so that the census and its readback run
+// while the other arrays are copied; c->copied marks the last copy's end.
+fs_status stage_upload(fs_ctx* c, const fs_particles* in, StagedUpload& d) {
     const int64_t n = in->n;
+    const int S = c->nsc();
     const size_t vec = (size_t)n * c->dim * sizeof(float), sc = (size_t)n * sizeof(float);
-    FS_TRY(ensure_staging(c, 4 * vec + 3 * sc + (size_t)n + 16 * 9 + sizeof(UploadCensus)));
+    FS_TRY(ensure_staging(c, 4 * vec + 3 * sc + (size_t)n + 16 * 9));
+    UploadHost& h = *c->upload_host;
+    h = UploadHost{};
+    int* boxes = c->upload_boxes();
+    for (int i = 0; i < 6 * S; i++) boxes[i] = i < 3 * S ? 0x7f7f7f7f : (int)0x80808080;
     char* st = (char*)c->staging;
     size_t off = 0;
     cudaError_t e = cudaSuccess;
     auto put = [&](const void* src, size_t bytes) -> const void* {
-        if (!src) return nullptr;
+        if (!src || bytes == 0) return nullptr;
         char* dst = st + off;
         off += (bytes + 15) & ~size_t(15);
         if (e == cudaSuccess) e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream);
         return dst;
     };
     d.pos = (const float*)put(in->position, vec);
+    d.type = (const uint8_t*)put(in->type, (size_t)n);
+    if (n > 0 && e == cudaSuccess) {
+        c->launches++;
+        k_census<<<grid_for(n, 256), 256, 0, c->stream>>>(n, c->dim, d.pos, d.type, c->search_radius,
+                                                           c->include_inactive, c->d_scene_offsets, S, c->search_state,
+                                                           c->search_box);
+        e = cudaGetLastError();
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(h.counts, c->search_state->counts, sizeof(h.counts), cudaMemcpyDeviceToHost, c->stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(boxes, c->search_box, sizeof(int) * 6 * S, cudaMemcpyDeviceToHost, c->stream);
+    }
+    if (e == cudaSuccess) e = cudaEventRecord(c->counted, c->stream);
     d.vel = (const float*)put(in->velocity, vec);
     d.acc = (const float*)put(in->acceleration, vec);
     d.ext = (const float*)put(in->external, vec);
     d.mass = (const float*)put(in->mass, sc);
     d.rho = (const float*)put(in->density, sc);
     d.p = (const float*)put(in->pressure, sc);
-    d.type = (const uint8_t*)put(in->type, (size_t)n);
-    d.census = (UploadCensus*)(st + off);
-    h = UploadCensus{{0, 0, 0, 0}};
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d.census, &h, sizeof(h), cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess) e = cudaEventRecord(c->copied, c->stream);
+    if (e == cudaSuccess) e = cudaEventSynchronize(c->counted);
     if (e != cudaSuccess) return fail(FS_ERR_CUDA, cudaGetErrorString(e));
-    FS_TRY(reset_bbox(c));
-    const int S = c->nsc();
-    if (n > 0) {
-        c->launches++;
-        k_census<<<grid_for(n, 256), 256, 0, c->stream>>>(n, c->dim, d.pos, d.type, c->search_radius,
-                                                           c->include_inactive, c->d_scene_offsets, S, d.census,
-                                                           c->bbox);
-        FS_CUDA(cudaGetLastError());
-    }
-    boxes.assign(6 * (size_t)S, 0);
-    FS_CUDA(cudaMemcpyAsync(&h, d.census, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-    FS_CUDA(cudaMemcpyAsync(boxes.data(), c->bbox, sizeof(int) * 6 * S, cudaMemcpyDeviceToHost, c->stream));
-    FS_CUDA(cudaStreamSynchronize(c->stream));
     return FS_OK;
 }
 
+// packs the staged arrays into the state; also clears the census and, for a
+// single scene, stores its grid
 template <typename R> fs_status pack_upload(fs_ctx* c, const StagedUpload& d, int64_t n) {
     c->cur = 0;
-    if (n == 0) return FS_OK;
     State<R> s = state_of<R>(c);
     c->launches++;
     k_pack<R><<<grid_for(n), kBlock, 0, c->stream>>>(n, c->dim, d.pos, d.vel, d.acc, d.ext, d.mass, d.rho, d.p, d.type,
                                                      c->prm.rest_density, s, c->type[0], c->hidx[0],
-                                                     c->d_scene_offsets, c->nsc(), c->scene_of[0]);
+                                                     c->d_scene_offsets, c->nsc(), c->scene_of[0], c->search_state,
+                                                     c->search_box, c->grids_host[0],
+                                                     c->scenes > 0 ? nullptr : c->grids);
     FS_CUDA(cudaGetLastError());
-    FS_CUDA(cudaStreamSynchronize(c->stream));
     return FS_OK;
 }
 
+// The wanted fields to host order in the staging buffer and from there to the
+// caller. From kOverlapBytes on, the first field's copy runs on a second stream
+// while the others are still scattered.
 template <typename R> fs_status download_impl(fs_ctx* c, fs_particles* out) {
     const int64_t n = c->n;
     const int dim = c->dim;
-    const size_t vec = (size_t)n * dim * sizeof(float);
-    FS_TRY(ensure_staging(c, std::max<size_t>(vec, (size_t)n * 4) + 64));
+    const size_t vec = (size_t)n * dim * sizeof(float), sc = (size_t)n * 4;
+    constexpr size_t kOverlapBytes = size_t(4) << 20;
     State<R> s = state_of<R>(c);
+    UnpackTo to{};
     struct F {
-        int field;
         void* dst;
         size_t bytes;
+        void** staged;
     } fields[] = {
-        {0, out->position, vec}, {1, out->velocity, vec}, {2, out->acceleration, vec}, {3, out->external, vec},
-        {4, out->mass, (size_t)n * 4}, {5, out->density, (size_t)n * 4}, {6, out->pressure, (size_t)n * 4},
-        {7, out->type, (size_t)n}, {8, out->tag, (size_t)n * 4}, {9, out->predicted_velocity, vec},
-        {10, out->non_pressure_acceleration, vec}, {11, out->source_term, (size_t)n * 4},
-        {12, out->diagonal_element, (size_t)n * 4},
+        {out->position, vec, (void**)&to.position}, {out->velocity, vec, (void**)&to.velocity},
+        {out->acceleration, vec, (void**)&to.acceleration}, {out->external, vec, (void**)&to.external},
+        {out->mass, sc, (void**)&to.mass}, {out->density, sc, (void**)&to.density},
+        {out->pressure, sc, (void**)&to.pressure}, {out->type, (size_t)n, (void**)&to.type},
+        {out->tag, sc, (void**)&to.tag}, {out->predicted_velocity, vec, (void**)&to.predicted_velocity},
+        {out->non_pressure_acceleration, vec, (void**)&to.non_pressure_acceleration},
+        {out->source_term, sc, (void**)&to.source_term}, {out->diagonal_element, sc, (void**)&to.diagonal_element},
     };
-    for (auto& f : fields) {
-        if (!f.dst) continue;
-    c->launches++;
-        k_unpack<R><<<grid_for(n), kBlock, 0, c->stream>>>(n, dim, f.field, s, (float*)c->staging,
-                                                           (uint8_t*)c->staging, (uint32_t*)c->staging);
-        FS_CUDA(cudaGetLastError());
-        FS_CUDA(cudaMemcpyAsync(f.dst, c->staging, f.bytes, cudaMemcpyDeviceToHost, c->stream));
+    size_t total = 0;
+    for (const F& f : fields)
+        if (f.dst) total += (f.bytes + 15) & ~size_t(15);
+    if (total == 0) {
+        FS_CUDA(cudaStreamSynchronize(c->stream));
+        return FS_OK;
     }
-    FS_CUDA(cudaStreamSynchronize(c->stream));
+    FS_TRY(ensure_staging(c, total));
+    const bool overlap = total >= kOverlapBytes;
+    cudaStream_t cs = overlap ? c->body_stream : c->stream;
+    size_t off = 0;
+    UnpackTo rest{};
+    int wanted = 0, launched = 0;
+    auto unpack = [&](const UnpackTo& u) {
+        c->launches++;
+        k_unpack<R><<<grid_for(n), kBlock, 0, c->stream>>>(n, dim, s, u);
+        return cudaGetLastError();
+    };
+    cudaError_t e = cudaSuccess;
+    for (F& f : fields) {
+        if (!f.dst) continue;
+        *f.staged = (char*)c->staging + off;
+        off += (f.bytes + 15) & ~size_t(15);
+        if (overlap && wanted == 0) {   // the first field on its own
+            e = unpack(to);
+            if (e == cudaSuccess) e = cudaEventRecord(c->counted, c->stream);
+            launched = 1;
+        }
+        wanted++;
+    }
+    rest = to;
+    if (overlap)
+        for (F& f : fields)
+            if (f.dst) {
+                *(void**)((char*)&rest + ((char*)f.staged - (char*)&to)) = nullptr;   // done above
+                break;
+            }
+    if (e == cudaSuccess && wanted > launched) e = unpack(rest);
+    if (overlap && e == cudaSuccess) e = cudaEventRecord(c->copied, c->stream);
+    if (overlap && e == cudaSuccess) e = cudaStreamWaitEvent(cs, c->counted, 0);
+    int copied = 0;
+    for (const F& f : fields) {
+        if (!f.dst) continue;
+        if (overlap && copied == 1 && e == cudaSuccess) e = cudaStreamWaitEvent(cs, c->copied, 0);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(f.dst, *f.staged, f.bytes, cudaMemcpyDeviceToHost, cs);
+        copied++;
+    }
+    const cudaError_t e1 = cudaStreamSynchronize(cs), e2 = cudaStreamSynchronize(c->stream);
+    for (cudaError_t q : {e, e1, e2})
+        if (q != cudaSuccess) return fail(FS_ERR_CUDA, cudaGetErrorString(q));
     return FS_OK;
 }
 
@@ -882,16 +955,15 @@ void set_layout(fs_ctx* c, int64_t n, int64_t nf, int64_t nb, int64_t ni) {
     c->n_owners = c->reference_order ? c->n_struct : nf;
 }
 
-fs_status read_scalars(fs_ctx* c) {
-    FS_CUDA(cudaMemcpyAsync(c->scalars_host, c->scalars, sizeof(StepScalars) * c->nsc(), cudaMemcpyDeviceToHost,
-                            c->stream));
+// the status word, and with scalars the step scalars too, in one wait
+fs_status read_back(fs_ctx* c, bool scalars, int* st = nullptr) {
+    if (scalars)
+        FS_CUDA(cudaMemcpyAsync(c->scalars_host, c->scalars, sizeof(StepScalars) * c->nsc(), cudaMemcpyDeviceToHost,
+                                c->stream));
+    if (st)
+        FS_CUDA(cudaMemcpyAsync(&c->upload_host->status, c->status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     FS_CUDA(cudaStreamSynchronize(c->stream));
-    return FS_OK;
-}
-
-fs_status read_status(fs_ctx* c, int* st) {
-    FS_CUDA(cudaMemcpyAsync(st, c->status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    FS_CUDA(cudaStreamSynchronize(c->stream));
+    if (st) *st = c->upload_host->status;
     return FS_OK;
 }
 
@@ -1002,7 +1074,7 @@ fs_status enqueue_pressure_loop(fs_ctx* c, bool capture, bool two_d, bool fp64_t
     if (!capture) {
         auto all_done = [&]() -> fs_status {
             FS_CUDA(cudaGetLastError());
-            FS_TRY(read_scalars(c));
+            FS_TRY(read_back(c, true));
             bool d = true;
             for (int i = 0; i < c->nsc(); i++) d = d && c->scalars_host[i].done;
             return d ? FS_ERR_STATE : FS_OK;   // FS_ERR_STATE here only means "stop"
@@ -1453,18 +1525,20 @@ fs_status fill_stats(fs_ctx* c, fs_step_stats* stats, int st, int entries = 1) {
 // neighborhood search of a step (with solver lists). A list overflow stops
 // every later kernel (they check the status word); with an automatic
 // capacity the lists are grown and the search is repeated once.
-fs_status search_for_step(fs_ctx* c, float dt) {
+// mark_end: also records the search's end (phase timestamp 1).
+fs_status search_for_step(fs_ctx* c, float dt, bool mark_end = false) {
     for (int attempt = 0; attempt < 3; attempt++) {
         c->launches++;
         k_step_begin<<<grid_for(c->nsc(), 128), 128, 0, c->stream>>>(c->scalars, c->nsc(), dt, false);
         FS_CUDA(cudaMemsetAsync(c->status, 0, sizeof(int), c->stream));
         cudaEventRecord(c->ev[0], c->stream);
         FS_TRY(search_dispatch(c, c->prm.solver != FS_SOLVER_NONE));
+        if (mark_end) cudaEventRecord(c->ev[1], c->stream);
         int st = 0;
-        FS_TRY(read_status(c, &st));
+        FS_TRY(read_back(c, false, &st));
         if (st == FS_ERR_CAPACITY && attempt < 2 && c->prm.neighbor_capacity == 0 &&
             c->prm.solver != FS_SOLVER_NONE) {
-            FS_TRY(read_scalars(c));
+            FS_TRY(read_back(c, true));
             int K = 32;
             while (K < c->scalars_host->max_neighbors) K *= 2;
             FS_TRY(ensure_lists(c, K));
@@ -1562,9 +1636,8 @@ fs_status solve_after_search(fs_ctx* c, float dt, fs_step_stats* stats) {
     }
     c->have_lists = false;  // positions moved: the lists belong to the old positions
     c->small_last = false;
-    FS_TRY(read_scalars(c));
     int st = 0;
-    FS_TRY(read_status(c, &st));
+    FS_TRY(read_back(c, true, &st));
     for (int i = 0; i < 5; i++) cudaEventElapsedTime(&c->phase_ms[i], c->ev[i], c->ev[i + 1]);
     fill_stats(c, stats, st);
     if (st != FS_OK) return fail((fs_status)st, "device reported an error during the step");
@@ -1693,8 +1766,7 @@ fs_status read_phase_times(fs_ctx* c) {
 }
 
 fs_status finish_steps(fs_ctx* c, fs_step_stats* stats, int* st) {
-    FS_TRY(read_scalars(c));
-    FS_TRY(read_status(c, st));
+    FS_TRY(read_back(c, true, st));
     FS_TRY(read_phase_times(c));
     fill_stats(c, stats, *st);
     return FS_OK;
@@ -1846,8 +1918,13 @@ static fs_status create_ctx(const fs_params* p, int32_t scenes, const int64_t* o
             return bail(fail(FS_ERR_CUDA, "copy of the scene offsets failed"));
     }
     FS_ALLOC(c->nbr_count, (cap + kTileOwners - 1) / kTileOwners * kTileOwners);   // whole tiles
-    if (cudaMallocHost((void**)&c->scalars_host, sizeof(StepScalars) * S) != cudaSuccess)
+    if (cudaMallocHost((void**)&c->scalars_host,
+                       sizeof(StepScalars) * S + sizeof(UploadHost) + sizeof(int) * 6 * S) != cudaSuccess)
         return bail(fail(FS_ERR_CUDA, "cudaMallocHost failed"));
+    c->upload_host = reinterpret_cast<UploadHost*>(c->scalars_host + S);
+    for (cudaEvent_t* e : {&c->counted, &c->copied})
+        if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess)
+            return bail(fail(FS_ERR_CUDA, "cudaEventCreate failed"));
     // the radix sort's per-tile digit counts for the largest sort
     FS_ALLOC(c->sort_hist, (size_t)sort_hist_entries((int64_t)cap));
     if (prepare_small_sort() != cudaSuccess) return bail(fail(FS_ERR_CUDA, "small-sort shared memory"));
@@ -1904,14 +1981,25 @@ fs_status fs_upload(fs_ctx* c, const fs_particles* in) {
         return fail(FS_ERR_INVALID, "a batched upload holds exactly the particles of every scene");
     FS_CUDA(cudaSetDevice(c->device));
     StagedUpload d;
-    UploadCensus h;
-    std::vector<int> boxes;
-    FS_TRY(stage_upload(c, in, d, h, boxes));
-    if (h.counts[3]) return fail(FS_ERR_INVALID, "particle type must be 0, 1 or 2");
+    // whatever ends the call, the copies from the caller's arrays are over by then
+    struct CopiesDone {
+        fs_ctx* c;
+        bool all = true;
+        ~CopiesDone() { all ? cudaStreamSynchronize(c->stream) : cudaEventSynchronize(c->copied); }
+    } done{c};
+    FS_TRY(stage_upload(c, in, d));
+    const unsigned long long* counts = c->upload_host->counts;
+    const bool invalid = counts[3] != 0;
     const int64_t n_before = c->n, owners_before = c->n_owners;
-    set_layout(c, in->n, (int64_t)h.counts[0], (int64_t)h.counts[1], (int64_t)h.counts[2]);
+    if (invalid) {   // the census starts afresh; the state stays as it was
+        FS_CUDA(cudaMemsetAsync(c->search_state->counts, 0, sizeof(c->search_state->counts), c->stream));
+        FS_CUDA(cudaMemsetAsync(c->search_box, 0x7f, 3 * c->nsc() * sizeof(int), c->stream));
+        FS_CUDA(cudaMemsetAsync(c->search_box + 3 * c->nsc(), 0x80, 3 * c->nsc() * sizeof(int), c->stream));
+        return fail(FS_ERR_INVALID, "particle type must be 0, 1 or 2");
+    }
+    set_layout(c, in->n, (int64_t)counts[0], (int64_t)counts[1], (int64_t)counts[2]);
     if (c->n != n_before || c->n_owners != owners_before) clear_graphs(c);
-    FS_TRY(choose_grids(c, boxes.data(), boxes.data() + 3 * c->nsc()));
+    FS_TRY(choose_grids(c, c->upload_boxes(), c->upload_boxes() + 3 * c->nsc()));
     FS_TRY(ensure_cells(c));
     fs_status r = c->precision == FS_PRECISION_FP64 ? pack_upload<double>(c, d, in->n) : pack_upload<float>(c, d, in->n);
     if (r != FS_OK) return r;
@@ -1925,6 +2013,7 @@ fs_status fs_upload(fs_ctx* c, const fs_particles* in) {
     c->have_state = true;
     c->have_lists = false;
     c->have_cells = false;
+    done.all = c->scenes > 0;   // (the packing may still run; a batch's grids are copied behind it)
     return FS_OK;
 }
 
@@ -1940,9 +2029,7 @@ fs_status fs_find_neighbors(fs_ctx* c) {
     if (!c) return fail(FS_ERR_INVALID, "ctx is null");
     if (!c->have_state) return fail(FS_ERR_STATE, "no particles uploaded");
     FS_CUDA(cudaSetDevice(c->device));
-    FS_TRY(search_for_step(c, c->prm.timestep));
-    cudaEventRecord(c->ev[1], c->stream);
-    FS_CUDA(cudaStreamSynchronize(c->stream));
+    FS_TRY(search_for_step(c, c->prm.timestep, true));
     cudaEventElapsedTime(&c->phase_ms[0], c->ev[0], c->ev[1]);
     return FS_OK;
 }
@@ -2415,6 +2502,7 @@ fs_status fs_run(fs_ctx* c, int32_t steps, float desired_dt, fs_step_stats* stat
     }
     // one step first: it settles the list capacity (and captures the graph)
     FS_TRY(one_step(c, desired_dt, stats));
+    if (steps == 1) return FS_OK;
     const float dt = desired_of(c, desired_dt);
     FS_TRY(enqueue_steps(c, steps - 1, dt));
     int st = 0;

@@ -27,6 +27,13 @@
 #include "fs_sort.cuh"
 #include "fs_tiles.cuh"
 
+// pinned mirror of what an upload or a step reads back (the per-scene boxes follow it)
+struct UploadHost {
+    unsigned long long counts[4] = {0, 0, 0, 0};   // particles per type; index 3: invalid types
+    int status = 0;
+    int pad = 0;
+};
+
 struct fs_ctx {
     fs_params prm{};
     int dim = 3;
@@ -136,7 +143,10 @@ struct fs_ctx {
     fsb::StatsPart* stats_parts = nullptr;  // global statistics: per-block partials and the result
     fsb::StatsOut* stats_out = nullptr;
     fsb::StepScalars* scalars = nullptr;    // device
-    fsb::StepScalars* scalars_host = nullptr;  // pinned mirror
+    fsb::StepScalars* scalars_host = nullptr;  // pinned mirror, followed by upload_host and its boxes
+    UploadHost* upload_host = nullptr;
+    int* upload_boxes() const { return reinterpret_cast<int*>(upload_host + 1); }
+    cudaEvent_t counted = nullptr, copied = nullptr;   // of an upload: census read back, last copy done
 
     // CUDA graphs of the solver phases (the IISPH loop is a conditional WHILE
     // node inside), one per buffer assignment they were captured with

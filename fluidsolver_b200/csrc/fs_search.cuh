@@ -329,6 +329,7 @@ __global__ void k_reorder(int64_t n, const uint32_t* FSB_R perm, const V4<R>* FS
 struct SearchState {
     uint32_t box_ticket;     // blocks of k_search_box that are done (its last block clears it)
     uint32_t scan_ticket;    // tiles of the scan handed out (cleared by k_search_box)
+    unsigned long long counts[4];   // an upload's particles per type (index 3: invalid types; cleared when it is packed)
 };
 
 template <typename R>
