@@ -911,10 +911,11 @@ template <typename R> fs_status search_impl(fs_ctx* c, bool solver_lists) {
         if constexpr (std::is_same<R, float>::value) {
             if (tiled_mode(c) && c->n_owners > 0) {
                 const int64_t tiles = (c->n_owners + kTileOwners - 1) / kTileOwners;
+                const bool spread = c->prm.solver == FS_SOLVER_IISPH_3D && lists_can_spread(c->nbr_capacity, tile_cap_of(c));
                 c->launches++;
                 k_build_tiles<<<(unsigned)tiles, kTileOwners, tile_build_smem(c->nbr_capacity, tile_cap_of(c)), st>>>(
                     c->n_owners, s.pos, s.type, c->cell_start, w, c->tile_desc, c->tile_ent, c->tile_stride, c->nbr,
-                    c->nbr_stride, c->nbr_capacity, tile_cap_of(c), c->nbr_count, c->status, c->scalars);
+                    c->nbr_stride, c->nbr_capacity, tile_cap_of(c), spread, c->nbr_count, c->status, c->scalars);
                 built = true;
             }
         }
