@@ -182,6 +182,16 @@ int tile_cap_of(const fs_ctx* c) {
     return small ? kTileCapSmall : kTileCap;
 }
 
+// Whether the tile lists are spread over the shared-memory banks (k_build_tiles):
+// IISPH scenes whose pressure passes take more than one round of resident
+// blocks. Below, a pass is a chain of latencies: an iteration took 12.8 us at
+// 8,000 particles and 21.9 at 60,800 with and without it (13.3 and 13.0 at
+// 29,791); 28.9 and 26.6 at 100,000.
+bool spread_lists(const fs_ctx* c) {
+    return c->prm.solver == FS_SOLVER_IISPH_3D && c->n_owners > (int64_t)kTileOwners * 4 * c->sms &&
+           lists_can_spread(c->nbr_capacity, tile_cap_of(c));
+}
+
 TileLists tile_lists_of(fs_ctx* c) {
     TileLists T;
     T.desc = c->tile_desc;
@@ -911,11 +921,10 @@ template <typename R> fs_status search_impl(fs_ctx* c, bool solver_lists) {
         if constexpr (std::is_same<R, float>::value) {
             if (tiled_mode(c) && c->n_owners > 0) {
                 const int64_t tiles = (c->n_owners + kTileOwners - 1) / kTileOwners;
-                const bool spread = c->prm.solver == FS_SOLVER_IISPH_3D && lists_can_spread(c->nbr_capacity, tile_cap_of(c));
                 c->launches++;
                 k_build_tiles<<<(unsigned)tiles, kTileOwners, tile_build_smem(c->nbr_capacity, tile_cap_of(c)), st>>>(
                     c->n_owners, s.pos, s.type, c->cell_start, w, c->tile_desc, c->tile_ent, c->tile_stride, c->nbr,
-                    c->nbr_stride, c->nbr_capacity, tile_cap_of(c), spread, c->nbr_count, c->status, c->scalars);
+                    c->nbr_stride, c->nbr_capacity, tile_cap_of(c), spread_lists(c), c->nbr_count, c->status, c->scalars);
                 built = true;
             }
         }

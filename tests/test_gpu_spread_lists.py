@@ -1,6 +1,7 @@
 """The order of the tile lists' entries: spread over the shared-memory banks, or,
 when the lists are too long for the memory that the sorting needs (a capacity
-of 256 here), as the rows of cells give them. The lists hold the same entries,
+of 256 here) or on a 148-SM device up to 75,776 owners, as the rows of cells
+give them. The lists hold the same entries,
 so the results differ by the rounding of the sums alone: a density is a
 compensated sum of partial sums of 8 terms (8 roundings of 2^-24 on either
 side, 1e-6); a velocity hangs on the density's difference from the rest
@@ -16,8 +17,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,spacing,capacity", [
-    (7, 1.0, 0), (128, 1.0, 0), (129, 1.0, 0), (5000, 1.0, 0), (5000, 1.0, 104), (5000, 0.8, 0), (5000, 0.8, 120),
-    (40000, 0.9, 88)])
+    (75776, 1.0, 0), (75777, 1.0, 0), (80001, 1.0, 104), (80001, 0.85, 88), (80001, 0.8, 120)])
 def test_spread_lists_hold_the_same_entries(n, spacing, capacity):
     col = dam(n, n % 89)
     col.position = np.ascontiguousarray(col.position * np.float32(spacing))
