@@ -104,6 +104,7 @@ template <typename R> State<R> state_of(fs_ctx* c) {
     s.type = c->type[c->cur];
     s.hidx = c->hidx[c->cur];
     s.scene = c->scene_of[c->cur];
+    s.phase_at = c->scalars->phase_at;
     return s;
 }
 
@@ -977,14 +978,12 @@ fs_status read_back(fs_ctx* c, bool scalars, int* st = nullptr) {
     return FS_OK;
 }
 
-// Phase timestamp i on stream st. While the stream is being captured the
-// event becomes an event-record node of the graph (recorded when the graph
-// runs), so the phase times stay measurable in graph mode.
+// Phase timestamp i of the host-driven path. In a captured step the kernels
+// write their own (StepScalars::phase_at).
 fs_status mark(fs_ctx* c, int i, cudaStream_t st) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     FS_CUDA(cudaStreamIsCapturing(st, &cs));
-    if (cs == cudaStreamCaptureStatusActive) FS_CUDA(cudaEventRecordWithFlags(c->ev[i], st, cudaEventRecordExternal));
-    else FS_CUDA(cudaEventRecord(c->ev[i], st));
+    if (cs == cudaStreamCaptureStatusNone) FS_CUDA(cudaEventRecord(c->ev[i], st));
     return FS_OK;
 }
 
@@ -997,6 +996,7 @@ __global__ void k_step_begin(StepScalars* sc, int scenes, float desired_dt, bool
     z.desired_dt = desired_dt;
     z.dt = desired_dt;
     if (keep_search) z.max_neighbors = sc[i].max_neighbors;
+    z.phase_at[0] = global_ns();
     sc[i] = z;
 }
 
@@ -1017,10 +1017,13 @@ float cfl_default(const fs_ctx* c) { return dynamic_timestep(c) ? c->prm.max_tim
 // Resets the step scalars before the solver phases; with the dynamic
 // generator also chooses the desired time step from the state on the device
 // (Simulator.cpp:18-25 runs the generator before the step).
-fs_status begin_solver_phases(fs_ctx* c, float dt, cudaStream_t st) {
-    c->launches++;
-    k_step_begin<<<grid_for(c->nsc(), 128), 128, 0, st>>>(c->scalars, c->nsc(), dt, true);
-    FS_CUDA(cudaGetLastError());
+// reset false: the search of the same graph follows such a reset.
+fs_status begin_solver_phases(fs_ctx* c, float dt, cudaStream_t st, bool reset = true) {
+    if (reset) {
+        c->launches++;
+        k_step_begin<<<grid_for(c->nsc(), 128), 128, 0, st>>>(c->scalars, c->nsc(), dt, true);
+        FS_CUDA(cudaGetLastError());
+    }
     if (!dynamic_timestep(c)) return FS_OK;
     const fs_params& p = c->prm;
     c->launches += 2;
@@ -1535,15 +1538,15 @@ fs_status fill_stats(fs_ctx* c, fs_step_stats* stats, int st, int entries = 1) {
 // neighborhood search of a step (with solver lists). A list overflow stops
 // every later kernel (they check the status word); with an automatic
 // capacity the lists are grown and the search is repeated once.
-// mark_end: also records the search's end (phase timestamp 1).
-fs_status search_for_step(fs_ctx* c, float dt, bool mark_end = false) {
+// Phase timestamps 0 and 1 are its begin and end.
+fs_status search_for_step(fs_ctx* c, float dt) {
     for (int attempt = 0; attempt < 3; attempt++) {
         c->launches++;
         k_step_begin<<<grid_for(c->nsc(), 128), 128, 0, c->stream>>>(c->scalars, c->nsc(), dt, false);
         FS_CUDA(cudaMemsetAsync(c->status, 0, sizeof(int), c->stream));
         cudaEventRecord(c->ev[0], c->stream);
         FS_TRY(search_dispatch(c, c->prm.solver != FS_SOLVER_NONE));
-        if (mark_end) cudaEventRecord(c->ev[1], c->stream);
+        cudaEventRecord(c->ev[1], c->stream);
         int st = 0;
         FS_TRY(read_back(c, false, &st));
         if (st == FS_ERR_CAPACITY && attempt < 2 && c->prm.neighbor_capacity == 0 &&
@@ -1602,10 +1605,9 @@ fs_status solve_graph(fs_ctx* c, float dt, bool with_search = false) {
     if (with_search) {
         c->launches++;
         k_step_begin<<<grid_for(c->nsc(), 128), 128, 0, c->stream>>>(c->scalars, c->nsc(), dt, false);
-        r = mark(c, 0, c->stream);
-        if (r == FS_OK) r = search_dispatch(c, true);
+        r = search_dispatch(c, true);
     }
-    if (r == FS_OK) r = begin_solver_phases(c, dt, c->stream);
+    if (r == FS_OK) r = begin_solver_phases(c, dt, c->stream, !with_search);
     if (r == FS_OK) r = step_dispatch_any(c, true);
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
@@ -1634,6 +1636,16 @@ fs_status solve_graph(fs_ctx* c, float dt, bool with_search = false) {
     return FS_OK;
 }
 
+// the phase times [first, 5) of the last captured step (after read_back with
+// the scalars); a phase that no kernel began (0) has none
+void phase_times_of_stamps(fs_ctx* c, int first) {
+    unsigned long long at[6];
+    std::memcpy(at, c->scalars_host[0].phase_at, sizeof(at));
+    for (int i = 4; i > 0; i--)
+        if (at[i] == 0) at[i] = at[i + 1];
+    for (int i = first; i < 5; i++) c->phase_ms[i] = at[i + 1] >= at[i] ? (float)((double)(at[i + 1] - at[i]) * 1e-6) : 0.f;
+}
+
 // solver phases of a step on the lists of the last search
 fs_status solve_after_search(fs_ctx* c, float dt, fs_step_stats* stats) {
     if (!c->have_lists) return fail(FS_ERR_STATE, "execute the neighborhood search first");
@@ -1648,7 +1660,12 @@ fs_status solve_after_search(fs_ctx* c, float dt, fs_step_stats* stats) {
     c->small_last = false;
     int st = 0;
     FS_TRY(read_back(c, true, &st));
-    for (int i = 0; i < 5; i++) cudaEventElapsedTime(&c->phase_ms[i], c->ev[i], c->ev[i + 1]);
+    if (graphs) {
+        cudaEventElapsedTime(&c->phase_ms[0], c->ev[0], c->ev[1]);   // the search by itself
+        phase_times_of_stamps(c, 1);
+    } else {
+        for (int i = 0; i < 5; i++) cudaEventElapsedTime(&c->phase_ms[i], c->ev[i], c->ev[i + 1]);
+    }
     fill_stats(c, stats, st);
     if (st != FS_OK) return fail((fs_status)st, "device reported an error during the step");
     return FS_OK;
@@ -1762,11 +1779,11 @@ fs_status enqueue_steps(fs_ctx* c, int32_t steps, float dt) {
 }
 
 // the phase times of the last step (search, first loop, second loop,
-// pressure iterations, integration): from the events of the step-by-step
-// path or the small-scene kernel's timestamps
+// pressure iterations, integration): from the timestamps of its kernels or of
+// the small-scene kernel
 fs_status read_phase_times(fs_ctx* c) {
     if (!c->small_last) {
-        for (int i = 0; i < 5; i++) cudaEventElapsedTime(&c->phase_ms[i], c->ev[i], c->ev[i + 1]);
+        phase_times_of_stamps(c, 0);
         return FS_OK;
     }
     unsigned long long t[6];
@@ -2039,7 +2056,7 @@ fs_status fs_find_neighbors(fs_ctx* c) {
     if (!c) return fail(FS_ERR_INVALID, "ctx is null");
     if (!c->have_state) return fail(FS_ERR_STATE, "no particles uploaded");
     FS_CUDA(cudaSetDevice(c->device));
-    FS_TRY(search_for_step(c, c->prm.timestep, true));
+    FS_TRY(search_for_step(c, c->prm.timestep));
     cudaEventElapsedTime(&c->phase_ms[0], c->ev[0], c->ev[1]);
     return FS_OK;
 }

@@ -57,6 +57,7 @@ template <typename R, bool KAHAN, bool SPLIT>
 __global__ void __launch_bounds__(128) k_cached_iisph3d_l1(int64_t n, State<R> s, Lists L, SolverConsts<R> c,
                                                            Gradients<R> G, const StepScalars* FSB_R sc,
                                                            const int* FSB_R status) {
+    phase_begins(s.phase_at, 1);
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n || *status) return;
     iisph3d_l1_one<R, KAHAN, SPLIT>(k, s, L, c, (R)sc->dt, [&](uint32_t q, const V3<R>& g, const V4<R>& pj) {
@@ -69,6 +70,7 @@ template <typename R, bool KAHAN, bool TWO_PASS>
 __global__ void __launch_bounds__(128) k_cached_iisph3d_l2(int64_t n, State<R> s, Lists L, SolverConsts<R> c,
                                                            Gradients<R> G, const StepScalars* FSB_R sc,
                                                            const int* FSB_R status) {
+    phase_begins(s.phase_at, 2);
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n || *status || s.type[k] != FS_TYPE_NORMAL) return;
     const R dt = (R)sc->dt;
@@ -114,6 +116,7 @@ template <typename R, bool KAHAN>
 __global__ void __launch_bounds__(128) k_cached_iisph3d_pressure_acc(int64_t n, State<R> s, Lists L, SolverConsts<R> c,
                                                                      Gradients<R> G, const StepScalars* FSB_R sc,
                                                                      const int* FSB_R status) {
+    phase_begins(s.phase_at, 3);
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n || *status || sc->done || s.type[k] != FS_TYPE_NORMAL) return;
     const R pk = s.p[k], qk = pk / c.rho0_sq;

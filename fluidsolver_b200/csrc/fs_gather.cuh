@@ -180,6 +180,7 @@ __device__ __forceinline__ R group_density(int64_t k, uint32_t n, V3<R> xk, cons
 template <typename R, bool KAHAN>
 __global__ void __launch_bounds__(kGroupThreads) k_group_sesph_density(int64_t n, State<R> s, Lists L,
                                                                        SolverConsts<R> c, const int* FSB_R status) {
+    phase_begins(s.phase_at, 1);
     __shared__ GroupRows<R, 1> rows[kGroupsPerBlock];
     if (*status) return;
     const int64_t k = group_owner();
@@ -197,6 +198,7 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_sesph_density(int64_t n
 template <typename R, bool KAHAN, bool GAMMA>
 __global__ void __launch_bounds__(kGroupThreads) k_group_iisph_density(int64_t n, State<R> s, Lists L,
                                                                        SolverConsts<R> c, const int* FSB_R status) {
+    phase_begins(s.phase_at, 1);
     __shared__ GroupRows<R, 1> rows[kGroupsPerBlock];
     if (*status) return;
     const int64_t k = group_owner();
@@ -213,6 +215,7 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph_density(int64_t n
 template <typename R, bool KAHAN>
 __global__ void __launch_bounds__(kGroupThreads) k_group_sesph_accel(int64_t n, State<R> s, Lists L, SolverConsts<R> c,
                                                                      const int* FSB_R status) {
+    phase_begins(s.phase_at, 2);
     __shared__ GroupRows<R, 6> rows[kGroupsPerBlock];
     if (*status) return;
     const int64_t k = group_owner();
@@ -258,6 +261,7 @@ template <typename R, bool KAHAN, bool SPLIT, bool TWO_D>
 __global__ void __launch_bounds__(kGroupThreads) k_group_iisph_l1(int64_t n, State<R> s, Lists L, SolverConsts<R> c,
                                                                   Gradients<R> G, const StepScalars* FSB_R sc,
                                                                   const int* FSB_R status) {
+    phase_begins(s.phase_at, 1);
     __shared__ GroupRows<R, 3> rows3[kGroupsPerBlock];
     __shared__ GroupRows<R, 1> rows1[SPLIT ? 1 : kGroupsPerBlock];
     if (*status) return;
@@ -317,6 +321,7 @@ template <typename R, bool KAHAN, bool TWO_PASS, bool CACHED>
 __global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_l2(int64_t n, State<R> s, Lists L, SolverConsts<R> c, Gradients<R> G,
                                                                     const StepScalars* FSB_R sc,
                                                                     const int* FSB_R status) {
+    phase_begins(s.phase_at, 2);
     constexpr int NC = TWO_PASS ? 4 : 8;
     __shared__ GroupRows<R, NC> rows[kGroupsPerBlock];
     if (*status) return;
@@ -383,6 +388,7 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_pressure_acc(in
                                                                               SolverConsts<R> c, Gradients<R> G,
                                                                               const StepScalars* FSB_R sc,
                                                                               const int* FSB_R status) {
+    phase_begins(s.phase_at, 3);
     __shared__ GroupRows<R, 3> rows[kGroupsPerBlock];
     if (*status || sc->done) return;
     const int64_t k = group_owner();
@@ -448,6 +454,7 @@ template <typename R, bool KAHAN, bool CACHED>
 __global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_l2(int64_t n, State<R> s, Lists L, SolverConsts<R> c, Gradients<R> G,
                                                                     const StepScalars* FSB_R sc,
                                                                     const int* FSB_R status) {
+    phase_begins(s.phase_at, 2);
     __shared__ GroupRows<R, 4> rows[kGroupsPerBlock];
     __shared__ GroupRows<R, 1> rows1[kGroupsPerBlock];
     if (*status) return;
@@ -498,6 +505,7 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_pressure_acc(in
                                                                               SolverConsts<R> c, Gradients<R> G,
                                                                               const StepScalars* FSB_R sc,
                                                                               const int* FSB_R status) {
+    phase_begins(s.phase_at, 3);
     __shared__ GroupRows<R, 3> rows[kGroupsPerBlock];
     if (*status || sc->done) return;
     const int64_t k = group_owner();

@@ -14,12 +14,6 @@
 namespace fsb {
 namespace {
 
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
 __device__ __forceinline__ int status_now(const int* status) { return *(const volatile int*)status; }
 
 // The launch is one cluster of CTAs (1 to kSmallMaxCtas, one per SM). The

@@ -92,6 +92,7 @@ template <typename R> struct State {
     const uint8_t* FSB_R type;
     const uint32_t* FSB_R hidx;
     const uint16_t* FSB_R scene;  // per-particle scene (batched contexts), else null
+    unsigned long long* phase_at; // StepScalars::phase_at of scene 0
     __device__ __forceinline__ int scene_of(int64_t k) const { return scene ? scene[k] : 0; }
 };
 
@@ -207,6 +208,7 @@ __device__ __forceinline__ void iisph3d_l1_one(int64_t k, const State<R>& s, con
 template <typename R, bool KAHAN, bool SPLIT>
 __global__ void k_iisph3d_l1(int64_t n, State<R> s, Lists L, SolverConsts<R> c, const StepScalars* FSB_R sc,
                              const int* FSB_R status) {
+    phase_begins(s.phase_at, 1);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n || *status) return;
     iisph3d_l1_one<R, KAHAN, SPLIT>(k, s, L, c, (R)sc->dt);
@@ -235,6 +237,7 @@ __device__ __forceinline__ void iisph3d_density_at(int64_t k, const State<R>& s,
 }
 template <typename R, bool KAHAN>
 __global__ void k_iisph3d_density(int64_t n, State<R> s, Lists L, SolverConsts<R> c, const int* FSB_R status) {
+    phase_begins(s.phase_at, 1);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n || *status) return;
     iisph3d_density_at<R, KAHAN>(k, s, L, c);
@@ -299,6 +302,7 @@ __device__ __forceinline__ void iisph3d_l2_one(int64_t k, const State<R>& s, con
 template <typename R, bool KAHAN, bool TWO_PASS>
 __global__ void k_iisph3d_l2(int64_t n, State<R> s, Lists L, SolverConsts<R> c, const StepScalars* FSB_R sc,
                              const int* FSB_R status) {
+    phase_begins(s.phase_at, 2);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n || *status) return;
     if (s.type[k] != FS_TYPE_NORMAL) return;
@@ -336,6 +340,7 @@ __device__ __forceinline__ void iisph3d_pressure_acc_one(int64_t k, const State<
 template <typename R, bool KAHAN>
 __global__ void k_iisph3d_pressure_acc(int64_t n, State<R> s, Lists L, SolverConsts<R> c,
                                        const StepScalars* FSB_R sc, const int* FSB_R status) {
+    phase_begins(s.phase_at, 3);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n || *status || sc->done) return;
     if (s.type[k] != FS_TYPE_NORMAL) return;
@@ -723,9 +728,10 @@ __device__ __forceinline__ void iisph3d_integrate_at(int64_t k, const State<R>& 
 template <typename R>
 __global__ void k_iisph3d_integrate(int64_t n, State<R> s, const StepScalars* FSB_R sc,
                                     const int* FSB_R status) {
+    phase_begins(s.phase_at, 4);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k >= n || *status) return;
-    iisph3d_integrate_at<R>(k, s, sc);
+    if (k < n && !*status) iisph3d_integrate_at<R>(k, s, sc);
+    step_ends(s.phase_at);
 }
 
 // ===========================================================================
@@ -755,6 +761,7 @@ __device__ __forceinline__ void sesph_density_one(int64_t k, const State<R>& s, 
 
 template <typename R, bool KAHAN>
 __global__ void k_sesph_density(int64_t n, State<R> s, Lists L, SolverConsts<R> c, const int* FSB_R status) {
+    phase_begins(s.phase_at, 1);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n || *status) return;
     if (s.type[k] != FS_TYPE_NORMAL) return;
@@ -793,6 +800,7 @@ __device__ __forceinline__ void sesph_accel_one(int64_t k, const State<R>& s, co
 
 template <typename R, bool KAHAN>
 __global__ void k_sesph_accel(int64_t n, State<R> s, Lists L, SolverConsts<R> c, const int* FSB_R status) {
+    phase_begins(s.phase_at, 2);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n || *status) return;
     if (s.type[k] != FS_TYPE_NORMAL) return;
@@ -813,6 +821,7 @@ __device__ __forceinline__ void sesph_maxima_at(int64_t k, const State<R>& s, co
 }
 template <typename R>
 __global__ void k_sesph_maxima(int64_t n, State<R> s, StepScalars* FSB_R sc, const int* FSB_R status) {
+    phase_begins(s.phase_at, 3);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (*status) return;
     float a2 = 0.f, v2 = 0.f;
@@ -848,9 +857,10 @@ __device__ __forceinline__ void sesph_integrate_at(int64_t k, const State<R>& s,
 template <typename R>
 __global__ void k_sesph_integrate(int64_t n, State<R> s, const StepScalars* FSB_R sc,
                                   const int* FSB_R status) {
+    phase_begins(s.phase_at, 4);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k >= n || *status) return;
-    sesph_integrate_at<R>(k, s, sc);
+    if (k < n && !*status) sesph_integrate_at<R>(k, s, sc);
+    step_ends(s.phase_at);
 }
 
 // ===========================================================================
@@ -905,6 +915,7 @@ __device__ __forceinline__ void iisph2d_l1_at(int64_t k, const State<R>& s, cons
 template <typename R, bool KAHAN, bool SPLIT>
 __global__ void k_iisph2d_l1(int64_t n, State<R> s, Lists L, SolverConsts<R> c, const StepScalars* FSB_R sc,
                              const int* FSB_R status) {
+    phase_begins(s.phase_at, 1);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n || *status) return;
     iisph2d_l1_at<R, KAHAN, SPLIT>(k, s, L, c, (R)sc->dt);
@@ -929,6 +940,7 @@ __device__ __forceinline__ void iisph2d_density_at(int64_t k, const State<R>& s,
 }
 template <typename R, bool KAHAN>
 __global__ void k_iisph2d_density(int64_t n, State<R> s, Lists L, SolverConsts<R> c, const int* FSB_R status) {
+    phase_begins(s.phase_at, 1);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n || *status) return;
     iisph2d_density_at<R, KAHAN>(k, s, L, c);
@@ -978,6 +990,7 @@ __device__ __forceinline__ void iisph2d_l2_at(int64_t k, const State<R>& s, cons
 template <typename R, bool KAHAN>
 __global__ void k_iisph2d_l2(int64_t n, State<R> s, Lists L, SolverConsts<R> c, const StepScalars* FSB_R sc,
                              const int* FSB_R status) {
+    phase_begins(s.phase_at, 2);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n || *status) return;
     iisph2d_l2_at<R, KAHAN>(k, s, L, c, (R)sc->dt);
@@ -1006,6 +1019,7 @@ __device__ __forceinline__ void iisph2d_pressure_acc_at(int64_t k, const State<R
 template <typename R, bool KAHAN>
 __global__ void k_iisph2d_pressure_acc(int64_t n, State<R> s, Lists L, SolverConsts<R> c,
                                        const StepScalars* FSB_R sc, const int* FSB_R status) {
+    phase_begins(s.phase_at, 3);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n || *status || sc->done) return;
     iisph2d_pressure_acc_at<R, KAHAN>(k, s, L, c);
@@ -1082,9 +1096,10 @@ __device__ __forceinline__ void iisph2d_integrate_at(int64_t k, const State<R>& 
 template <typename R>
 __global__ void k_iisph2d_integrate(int64_t n, State<R> s, const StepScalars* FSB_R sc,
                                     const int* FSB_R status) {
+    phase_begins(s.phase_at, 4);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k >= n || *status) return;
-    iisph2d_integrate_at<R>(k, s, sc);
+    if (k < n && !*status) iisph2d_integrate_at<R>(k, s, sc);
+    step_ends(s.phase_at);
 }
 
 }  // namespace fsb

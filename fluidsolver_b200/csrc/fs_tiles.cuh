@@ -884,6 +884,7 @@ __global__ void __launch_bounds__(kPassThreads, kL1GlobalEntries ? 4 : 3) k_tile
                                                                   SolverConsts<float> c,
                                                                   const StepScalars* __restrict__ sc,
                                                                   int* __restrict__ status) {
+    phase_begins(s.phase_at, 1);
     extern __shared__ float4 tile_smem[];
     if (blockIdx.x >= n_tiles) {
         if (*status) return;
@@ -970,6 +971,7 @@ __global__ void __launch_bounds__(kPassThreads, kL2GlobalEntries ? 4 : 3) k_tile
                                                                   Lists L, SolverConsts<float> c,
                                                                   StepScalars* __restrict__ sc,
                                                                   int* __restrict__ status) {
+    phase_begins(s.phase_at, 2);
     extern __shared__ float4 tile_smem[];
     const int half = threadIdx.x & 1;
     const int64_t k = blockIdx.x * (int64_t)kTileOwners + (threadIdx.x >> 1);
@@ -1153,6 +1155,7 @@ template <int AHEAD, int TPO>
 __global__ void __launch_bounds__(pressure_threads<TPO>(), acc_blocks_per_sm<TPO>()) k_tile_iisph3d_pressure_acc(
     int64_t n_fluid, State<float> s, TileLists T, Lists L, SolverConsts<float> c, const StepScalars* __restrict__ sc,
     int* __restrict__ status) {
+    phase_begins(s.phase_at, 3);
     static_assert(kPressureGlobalEntries, "the pressure passes read their entries from the global octet planes");
     extern __shared__ float4 tile_smem[];
     launch_dependents();   // the update pass may be scheduled while this grid runs
@@ -1415,6 +1418,7 @@ __global__ void __launch_bounds__(kPassThreads, ONE ? kLoopOneBlocksPerSm : kLoo
     k_tile_iisph3d_pressure_loop(int64_t n_fluid, int64_t tiles, State<float> s, TileLists T, Lists L,
                                  SolverConsts<float> c, LoopTest lt, StepScalars* __restrict__ sc,
                                  int* __restrict__ status) {
+    phase_begins(s.phase_at, 3);
     extern __shared__ float4 tile_smem[];
     __shared__ TileStage stg;
     __shared__ int s_done;
@@ -1604,6 +1608,7 @@ template <int AHEAD>
 __global__ void __launch_bounds__(kPassThreads, 5) k_tile_sesph3d_density(int64_t n_fluid, State<float> s,
                                                                           TileLists T, Lists L, SolverConsts<float> c,
                                                                           int* __restrict__ status) {
+    phase_begins(s.phase_at, 1);
     extern __shared__ float4 tile_smem[];
     const int half = threadIdx.x & 1;
     const int64_t k = blockIdx.x * (int64_t)kTileOwners + (threadIdx.x >> 1);
@@ -1668,6 +1673,7 @@ template <int AHEAD>
 __global__ void __launch_bounds__(kPassThreads, 4) k_tile_sesph3d_accel(int64_t n_fluid, State<float> s,
                                                                         TileLists T, Lists L, SolverConsts<float> c,
                                                                         int* __restrict__ status) {
+    phase_begins(s.phase_at, 2);
     extern __shared__ float4 tile_smem[];
     const int half = threadIdx.x & 1;
     const int64_t k = blockIdx.x * (int64_t)kTileOwners + (threadIdx.x >> 1);
