@@ -865,8 +865,37 @@ bool counting_order(const fs_ctx* c) {
     return c->n - c->n_struct <= 1024 && c->n_struct <= 128 * c->box_cells;
 }
 
+// Launches kernel<<<grid, block, smem, st>>>(args...), as a programmatic
+// dependent of the kernel before it on st when pdl is set (the kernel then
+// calls grid_dependency_wait before it reads that kernel's results).
+template <typename... KArgs, typename... Args>
+void launch_pdl(bool pdl, void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+                Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// Whether the kernels of the search and of the SESPH steps are launched as
+// programmatic dependents of one another: in small scenes, where the gaps
+// between kernels show (20 2D SESPH steps of 2,500 particles 793 -> 757 us, 10 of
+// 40,000 785 -> 743, 10 2D IISPH steps 966 -> 949). In larger ones they don't
+// (8,000 particles and more in 3D: the same). The IISPH phases stay apart:
+// blocks that came early landed unevenly on the SMs, and an iteration of
+// the bit-exact passes over 100,000 particles took 14 % longer.
+bool chained(const fs_ctx* c) { return c->n <= 65536; }
+
 // The same order and table as order_by_radix_sort, by counting.
 template <typename R> fs_status order_by_counting(fs_ctx* c, State<R> s) {
+    const bool pdl = chained(c);
     const int64_t n = c->n;
     cudaStream_t st = c->stream;
     const bool single = c->reference_order;
@@ -881,17 +910,20 @@ template <typename R> fs_status order_by_counting(fs_ctx* c, State<R> s) {
     uint32_t* order = single ? c->perm[1] : nullptr;
     const int nx = c->cur ^ 1;
     c->launches += 5;
-    k_search_box<R><<<gb, 256, 0, st>>>(n, s.pos, s.type, s.scene, c->nsc(), c->include_inactive, c->search_radius,
+    launch_pdl(pdl, k_search_box<R>, gb, 256, 0, st, n, s.pos, s.type, s.scene, c->nsc(), c->include_inactive,
+               c->search_radius,
                                         c->truncate_cells, c->search_box, c->grids, c->search_state,
                                         (uint4*)c->cell_start, (entries + 3) / 4, c->look_tiles, tiles);
-    k_search_keys<R><<<grid_for(n, pb), pb, 0, st>>>(n, s.pos, s.type, s.hidx, c->include_inactive, single,
+    launch_pdl(pdl, k_search_keys<R>, grid_for(n, pb), pb, 0, st, n, s.pos, s.type, s.hidx, c->include_inactive,
+               single,
                                                      c->search_radius, c->truncate_cells, c->grids, s.scene, c->cells,
                                                      excluded, entry, slot, order, c->h2d_cell, c->h2d_rank,
                                                      c->cell_start, c->status);
-    k_search_scan<<<(unsigned)tiles, kLookThreads, 0, st>>>(c->cell_start, entries, c->look_tiles, c->search_state,
+    launch_pdl(pdl, k_search_scan, (unsigned)tiles, kLookThreads, 0, st, c->cell_start, entries, c->look_tiles,
+               c->search_state,
                                                             c->status);
-    k_search_scatter<<<grid_for(n, pb), pb, 0, st>>>(n, entry, slot, c->cell_start, list, c->status);
-    k_search_reorder<R><<<grid_for(n, pb), pb, 0, st>>>(
+    launch_pdl(pdl, k_search_scatter, grid_for(n, pb), pb, 0, st, n, entry, slot, c->cell_start, list, c->status);
+    launch_pdl(pdl, k_search_reorder<R>, grid_for(n, pb), pb, 0, st,
         n, c->n_struct, excluded, list, entry, order, c->cell_start, (const V4<R>*)c->pos[c->cur], (V4<R>*)c->pos[nx],
         (const V4<R>*)c->vel[c->cur], (V4<R>*)c->vel[nx], (const V4<R>*)c->acc[c->cur], (V4<R>*)c->acc[nx],
         (const V4<R>*)c->ext[c->cur], (V4<R>*)c->ext[nx], (const R*)c->rho[c->cur], (R*)c->rho[nx],
@@ -912,12 +944,14 @@ template <typename R> fs_status search_impl(fs_ctx* c, bool solver_lists) {
     }
     State<R> s = state_of<R>(c);
     if (c->hash_table) return compact_search_impl<R>(c, s, solver_lists);
-    FS_TRY(counting_order(c) ? order_by_counting<R>(c, s) : order_by_radix_sort<R>(c, s));
+    const bool counted = counting_order(c);
+    FS_TRY(counted ? order_by_counting<R>(c, s) : order_by_radix_sort<R>(c, s));
     s = state_of<R>(c);
     if (solver_lists) {
         WalkParams w = walk_of(c, true);
         const uint32_t owners = 1u << FS_TYPE_NORMAL;
         const bool rows = !c->reference_order && c->dim == 3;
+        const bool pdl = counted && chained(c);
         bool built = false;
         if constexpr (std::is_same<R, float>::value) {
             if (tiled_mode(c) && c->n_owners > 0) {
@@ -934,12 +968,12 @@ template <typename R> fs_status search_impl(fs_ctx* c, bool solver_lists) {
             c->launches++;
             auto* kernel = c->dim == 2 ? (c->sort_lists_by_host ? k_group_lists<R, 3, true> : k_group_lists<R, 3, false>)
                                        : (c->sort_lists_by_host ? k_group_lists<R, 7, true> : k_group_lists<R, 7, false>);
-            kernel<<<group_grid(c->n_owners), kGroupThreads, 0, st>>>(
+            launch_pdl(pdl, kernel, group_grid(c->n_owners), kGroupThreads, 0, st,
                 c->n_owners, s.pos, s.type, s.hidx, c->cell_start, w, owners, rows, c->nbr, c->nbr_stride,
                 c->nbr_capacity, c->nbr_count, c->status, c->scalars);
         } else if (!built) {
             c->launches++;
-            k_build_lists<R><<<grid_for(c->n_owners), kBlock, 0, st>>>(
+            launch_pdl(pdl, k_build_lists<R>, grid_for(c->n_owners), kBlock, 0, st,
                 c->n_owners, s.pos, s.type, c->cell_start, w, owners, rows, c->nbr, c->nbr_stride,
                 c->nbr_capacity, c->nbr_count, c->status, c->scalars);
         }
@@ -990,6 +1024,7 @@ fs_status mark(fs_ctx* c, int i, cudaStream_t st) {
 // resets the per-step scalars; keep_search keeps the statistics of the
 // search that precedes the solver phases
 __global__ void k_step_begin(StepScalars* sc, int scenes, float desired_dt, bool keep_search) {
+    chain_entry();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= scenes) return;
     StepScalars z{};
@@ -1040,25 +1075,6 @@ fs_status begin_solver_phases(fs_ctx* c, float dt, cudaStream_t st, bool reset =
 // ---------------------------------------------------------------------------
 // solver steps
 // ---------------------------------------------------------------------------
-// Launches kernel<<<grid, block, smem, st>>>(args...), as a programmatic
-// dependent of the kernel before it on st when pdl is set (the kernel then
-// calls grid_dependency_wait before it reads that kernel's results).
-template <typename... KArgs, typename... Args>
-void launch_pdl(bool pdl, void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
-                Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
 // The IISPH pressure iterations. Eagerly, the host reads the exit flag after
 // every iteration. While the stream is being captured, the loop becomes a
 // conditional WHILE node: its body is the iteration followed by the
@@ -1213,9 +1229,11 @@ fs_status step_iisph3d_tiled(fs_ctx* c, bool capture) {
     State<float> s = state_of<float>(c);
     FS_TRY(mark(c, 1, st));
     c->launches++;
-    FSB_AHEAD_SWITCH(c->tuning.l1_ahead, k_tile_iisph3d_l1,
-                     <<<tiles + rest, kPassThreads, tile_pass_smem(36, T.K, !kL1GlobalEntries, T.cap), st>>>(
-                         nf, n, tiles, s, T, L, k, c->scalars, c->status))
+    const size_t l1_smem = tile_pass_smem(36, T.K, !kL1GlobalEntries, T.cap);
+#define FSB_L1_LAUNCH(...) \
+    __VA_ARGS__<<<tiles + rest, kPassThreads, l1_smem, st>>>(nf, n, tiles, s, T, L, k, c->scalars, c->status)
+    FSB_AHEAD_SWITCH(c->tuning.l1_ahead, k_tile_iisph3d_l1, FSB_L1_LAUNCH)
+#undef FSB_L1_LAUNCH
     FS_CUDA(cudaGetLastError());
     FS_TRY(mark(c, 2, st));
     c->launches++;
@@ -1360,47 +1378,53 @@ template <typename R, bool KAHAN> fs_status step_iisph3d(fs_ctx* c, bool capture
     return FS_OK;
 }
 
+#define FSB_DENSITY_LAUNCH(...) \
+    launch_pdl(pdl, __VA_ARGS__, tiles, kPassThreads, density_smem, st, nf, s, T, L, k, c->status)
+#define FSB_ACCEL_LAUNCH(...) \
+    launch_pdl(pdl, __VA_ARGS__, tiles, kPassThreads, accel_smem, st, nf, s, T, L, k, c->status)
 // 3D SESPH in the fast mode on tile lists (fs_tiles.cuh): the density and
 // acceleration passes; maxima, CFL clamp and integration as in step_sesph
 fs_status step_sesph3d_tiled(fs_ctx* c) {
+    const bool pdl = chained(c);
     cudaStream_t st = c->stream;
     const int64_t n = c->n, nf = c->n_owners;
     const unsigned tiles = (unsigned)((nf + kTileOwners - 1) / kTileOwners);
     const SolverConsts<float> k = consts_of<float>(c);
     const Lists L = lists_of(c);
     const TileLists T = tile_lists_of(c);
+    const size_t density_smem = tile_pass_smem(16, T.K, false, T.cap), accel_smem = tile_pass_smem(36, T.K, false, T.cap);
     State<float> s = state_of<float>(c);
     FS_TRY(mark(c, 1, st));
     c->launches++;
-    FSB_AHEAD_SWITCH(c->tuning.l1_ahead, k_tile_sesph3d_density,
-                     <<<tiles, kPassThreads, tile_pass_smem(16, T.K, false, T.cap), st>>>(nf, s, T, L, k, c->status))
+    FSB_AHEAD_SWITCH(c->tuning.l1_ahead, k_tile_sesph3d_density, FSB_DENSITY_LAUNCH)
     FS_CUDA(cudaGetLastError());
     FS_TRY(mark(c, 2, st));
     c->launches++;
-    FSB_AHEAD_SWITCH(c->tuning.l1_ahead, k_tile_sesph3d_accel,
-                     <<<tiles, kPassThreads, tile_pass_smem(36, T.K, false, T.cap), st>>>(nf, s, T, L, k, c->status))
+    FSB_AHEAD_SWITCH(c->tuning.l1_ahead, k_tile_sesph3d_accel, FSB_ACCEL_LAUNCH)
     FS_CUDA(cudaGetLastError());
     FS_TRY(mark(c, 3, st));
     c->launches++;
-    k_sesph_maxima<float><<<grid_for(n), kBlock, 0, st>>>(n, s, c->scalars, c->status);
+    launch_pdl(pdl, k_sesph_maxima<float>, grid_for(n), kBlock, 0, st, n, s, c->scalars, c->status);
     c->launches++;
-    k_sesph_maxima_final<<<1, 1, 0, st>>>(c->scalars);
-    c->launches++;
-    k_cfl<<<1, 128, 0, st>>>(c->scalars, c->nsc(), c->prm.particle_size, cfl_default(c), c->prm.lambda_v,
-                             c->prm.lambda_a, c->status);
+    launch_pdl(pdl, k_sesph_maxima_cfl, 1, 1, 0, st, c->scalars, c->prm.particle_size, cfl_default(c), c->prm.lambda_v,
+               c->prm.lambda_a, c->status);
     FS_TRY(mark(c, 4, st));
     c->launches++;
-    k_sesph_integrate<float><<<grid_for(n), kBlock, 0, st>>>(n, s, c->scalars, c->status);
+    launch_pdl(pdl, k_sesph_integrate<float>, grid_for(n), kBlock, 0, st, n, s, c->scalars, c->status);
     FS_CUDA(cudaGetLastError());
     FS_TRY(mark(c, 5, st));
     return FS_OK;
 }
+
+#undef FSB_DENSITY_LAUNCH
+#undef FSB_ACCEL_LAUNCH
 
 template <typename R, bool KAHAN> fs_status step_sesph(fs_ctx* c) {
     if constexpr (std::is_same<R, float>::value && KAHAN) {
         if (tiled_mode(c) && c->n_owners > 0) return step_sesph3d_tiled(c);
     }
     cudaStream_t st = c->stream;
+    const bool pdl = chained(c);
     const int64_t n = c->n, no = c->n_owners;
     const SolverConsts<R> k = consts_of<R>(c);
     const Lists L = lists_of(c);
@@ -1409,25 +1433,23 @@ template <typename R, bool KAHAN> fs_status step_sesph(fs_ctx* c) {
     c->launches++;
     const bool group = grouped(c);
     const unsigned go = group_grid(no);
-    if (group) k_group_sesph_density<R, KAHAN><<<go, kGroupThreads, 0, st>>>(no, s, L, k, c->status);
-    else k_sesph_density<R, KAHAN><<<grid_for(no), kBlock, 0, st>>>(no, s, L, k, c->status);
+    if (group) launch_pdl(pdl, k_group_sesph_density<R, KAHAN>, go, kGroupThreads, 0, st, no, s, L, k, c->status);
+    else launch_pdl(pdl, k_sesph_density<R, KAHAN>, grid_for(no), kBlock, 0, st, no, s, L, k, c->status);
     FS_TRY(mark(c, 2, st));
     c->launches++;
-    if (group) k_group_sesph_accel<R, KAHAN><<<go, kGroupThreads, 0, st>>>(no, s, L, k, c->status);
-    else k_sesph_accel<R, KAHAN><<<grid_for(no), kBlock, 0, st>>>(no, s, L, k, c->status);
+    if (group) launch_pdl(pdl, k_group_sesph_accel<R, KAHAN>, go, kGroupThreads, 0, st, no, s, L, k, c->status);
+    else launch_pdl(pdl, k_sesph_accel<R, KAHAN>, grid_for(no), kBlock, 0, st, no, s, L, k, c->status);
     FS_TRY(mark(c, 3, st));
     if (c->dim == 3) {
     c->launches++;
-        k_sesph_maxima<R><<<grid_for(n), kBlock, 0, st>>>(n, s, c->scalars, c->status);
+        launch_pdl(pdl, k_sesph_maxima<R>, grid_for(n), kBlock, 0, st, n, s, c->scalars, c->status);
     c->launches++;
-        k_sesph_maxima_final<<<1, 1, 0, st>>>(c->scalars);
-    c->launches++;
-        k_cfl<<<1, 128, 0, st>>>(c->scalars, c->nsc(), c->prm.particle_size, cfl_default(c), c->prm.lambda_v,
-                                 c->prm.lambda_a, c->status);
+        launch_pdl(pdl, k_sesph_maxima_cfl, 1, 1, 0, st, c->scalars, c->prm.particle_size, cfl_default(c),
+                   c->prm.lambda_v, c->prm.lambda_a, c->status);
     }
     FS_TRY(mark(c, 4, st));
     c->launches++;
-    k_sesph_integrate<R><<<grid_for(n), kBlock, 0, st>>>(n, s, c->scalars, c->status);
+    launch_pdl(pdl, k_sesph_integrate<R>, grid_for(n), kBlock, 0, st, n, s, c->scalars, c->status);
     FS_CUDA(cudaGetLastError());
     FS_TRY(mark(c, 5, st));
     return FS_OK;

@@ -200,6 +200,14 @@ __device__ __forceinline__ void raise_status(int* status, int code) { atomicCAS(
 // launch_dependents lets the next such kernel start early.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// The first statement of the kernels that launch_pdl chains: the next kernel's
+// blocks may take their places, and this one's work waits for the kernel before
+// it. All kernels of the chain wait, so that a kernel's end implies the end of
+// all before it.
+__device__ __forceinline__ void chain_entry() {
+    launch_dependents();
+    grid_dependency_wait();
+}
 
 // One scene's cell grid: dims, this step's origin (cell coordinates) and the
 // offset of its cells in the concatenated cell tables.

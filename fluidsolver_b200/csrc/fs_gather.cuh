@@ -180,6 +180,7 @@ __device__ __forceinline__ R group_density(int64_t k, uint32_t n, V3<R> xk, cons
 template <typename R, bool KAHAN>
 __global__ void __launch_bounds__(kGroupThreads) k_group_sesph_density(int64_t n, State<R> s, Lists L,
                                                                        SolverConsts<R> c, const int* FSB_R status) {
+    chain_entry();
     phase_begins(s.phase_at, 1);
     __shared__ GroupRows<R, 1> rows[kGroupsPerBlock];
     if (*status) return;
@@ -215,6 +216,7 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph_density(int64_t n
 template <typename R, bool KAHAN>
 __global__ void __launch_bounds__(kGroupThreads) k_group_sesph_accel(int64_t n, State<R> s, Lists L, SolverConsts<R> c,
                                                                      const int* FSB_R status) {
+    chain_entry();
     phase_begins(s.phase_at, 2);
     __shared__ GroupRows<R, 6> rows[kGroupsPerBlock];
     if (*status) return;
@@ -587,6 +589,7 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_lists(int64_t n_owners,
                                                                uint32_t owner_mask, bool rows, uint32_t* FSB_R nbr,
                                                                int64_t stride, int K, uint32_t* FSB_R count,
                                                                int* FSB_R status, StepScalars* FSB_R sc) {
+    chain_entry();
     __shared__ ListGroup lists[kGroupsPerBlock];
     __shared__ ListSort sorts[SORT ? kGroupsPerBlock : 1];
     {   // an overflow elsewhere does not stop the counting: the largest list decides how far the lists grow

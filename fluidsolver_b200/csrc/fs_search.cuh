@@ -337,6 +337,7 @@ __global__ void k_search_box(int64_t n, const V4<R>* FSB_R pos, const uint8_t* F
                              int scenes, bool include_inactive, float r, bool trunc, int* FSB_R box,
                              SceneGrid* FSB_R grids, SearchState* FSB_R st, uint4* FSB_R table, int64_t table16,
                              unsigned long long* FSB_R tiles, int64_t ntiles) {
+    chain_entry();
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, total = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = t; i < table16; i += total) table[i] = make_uint4(0u, 0u, 0u, 0u);
     for (int64_t i = t; i < ntiles; i += total) tiles[i] = 0ull;
@@ -372,6 +373,7 @@ __global__ void k_search_keys(int64_t n, const V4<R>* FSB_R pos, const uint8_t* 
                               uint32_t excluded, uint32_t* FSB_R entry, uint32_t* FSB_R slot, uint32_t* FSB_R order,
                               int2* FSB_R h2d_cell, const uint32_t* FSB_R h2d_rank, uint32_t* FSB_R counts,
                               int* FSB_R status) {
+    chain_entry();
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     uint32_t e = 0xffffffffu;   // no particle
     if (k < n) {
@@ -404,6 +406,7 @@ inline int64_t look_tiles(int64_t m) { return (m + kLookTile - 1) / kLookTile; }
 static __global__ void __launch_bounds__(kLookThreads) k_search_scan(uint32_t* FSB_R a, int64_t m,
                                                                      unsigned long long* FSB_R tiles,
                                                                      SearchState* FSB_R st, int* FSB_R status) {
+    chain_entry();
     __shared__ uint32_t s_warp[kLookThreads / 32], s_tile, s_before;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     const unsigned all = 0xffffffffu;
@@ -479,6 +482,7 @@ static __global__ void __launch_bounds__(kLookThreads) k_search_scan(uint32_t* F
 static __global__ void k_search_scatter(int64_t n, const uint32_t* FSB_R entry, const uint32_t* FSB_R slot,
                                         const uint32_t* FSB_R cell_start, uint32_t* FSB_R list,
                                         const int* FSB_R status) {
+    chain_entry();
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n || *status == FS_ERR_TIMEOUT) return;
     list[cell_start[entry[k]] + slot[k]] = (uint32_t)k;
@@ -496,6 +500,7 @@ __global__ void k_search_reorder(int64_t n, int64_t n_struct, uint32_t excluded,
                                  uint8_t* FSB_R t1, const uint32_t* FSB_R h0, uint32_t* FSB_R h1,
                                  const uint16_t* FSB_R sc0, uint16_t* FSB_R sc1, uint32_t* FSB_R h2d_rank,
                                  const int* FSB_R status) {
+    chain_entry();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n || *status == FS_ERR_TIMEOUT) return;
     const uint32_t k = list[i], e = entry[k];
@@ -810,6 +815,7 @@ __global__ void __launch_bounds__(128) k_build_lists(int64_t n_owners, const V4<
                                                      bool rows, uint32_t* FSB_R nbr, int64_t stride, int K,
                                                      uint32_t* FSB_R count, int* FSB_R status,
                                                      StepScalars* FSB_R sc) {
+    chain_entry();
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n_owners) return;
     // an overflow elsewhere does not stop the counting: the largest list decides how far the lists grow

@@ -761,6 +761,7 @@ __device__ __forceinline__ void sesph_density_one(int64_t k, const State<R>& s, 
 
 template <typename R, bool KAHAN>
 __global__ void k_sesph_density(int64_t n, State<R> s, Lists L, SolverConsts<R> c, const int* FSB_R status) {
+    chain_entry();
     phase_begins(s.phase_at, 1);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n || *status) return;
@@ -800,6 +801,7 @@ __device__ __forceinline__ void sesph_accel_one(int64_t k, const State<R>& s, co
 
 template <typename R, bool KAHAN>
 __global__ void k_sesph_accel(int64_t n, State<R> s, Lists L, SolverConsts<R> c, const int* FSB_R status) {
+    chain_entry();
     phase_begins(s.phase_at, 2);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n || *status) return;
@@ -821,6 +823,7 @@ __device__ __forceinline__ void sesph_maxima_at(int64_t k, const State<R>& s, co
 }
 template <typename R>
 __global__ void k_sesph_maxima(int64_t n, State<R> s, StepScalars* FSB_R sc, const int* FSB_R status) {
+    chain_entry();
     phase_begins(s.phase_at, 3);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (*status) return;
@@ -841,7 +844,13 @@ __device__ __forceinline__ void sesph_maxima_final_one(StepScalars* FSB_R sc) {
     sc->max_a2_bits = 0u;
     sc->max_v2_bits = 0u;
 }
-static __global__ void k_sesph_maxima_final(StepScalars* FSB_R sc) { sesph_maxima_final_one(sc); }
+// the maxima's end and the clamp (k_cfl)
+static __global__ void k_sesph_maxima_cfl(StepScalars* FSB_R sc, float particle_size, float timestep, float lambda_v,
+                                          float lambda_a, const int* FSB_R status) {
+    chain_entry();
+    sesph_maxima_final_one(sc);
+    if (!*status) cfl_one(sc, particle_size, timestep, lambda_v, lambda_a);
+}
 
 // Euler-Cromer for every active particle: v += dt a; x += dt v
 template <typename R>
@@ -857,6 +866,7 @@ __device__ __forceinline__ void sesph_integrate_at(int64_t k, const State<R>& s,
 template <typename R>
 __global__ void k_sesph_integrate(int64_t n, State<R> s, const StepScalars* FSB_R sc,
                                   const int* FSB_R status) {
+    chain_entry();
     phase_begins(s.phase_at, 4);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k < n && !*status) sesph_integrate_at<R>(k, s, sc);

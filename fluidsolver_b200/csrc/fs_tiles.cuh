@@ -1608,6 +1608,7 @@ template <int AHEAD>
 __global__ void __launch_bounds__(kPassThreads, 5) k_tile_sesph3d_density(int64_t n_fluid, State<float> s,
                                                                           TileLists T, Lists L, SolverConsts<float> c,
                                                                           int* __restrict__ status) {
+    chain_entry();
     phase_begins(s.phase_at, 1);
     extern __shared__ float4 tile_smem[];
     const int half = threadIdx.x & 1;
@@ -1673,6 +1674,7 @@ template <int AHEAD>
 __global__ void __launch_bounds__(kPassThreads, 4) k_tile_sesph3d_accel(int64_t n_fluid, State<float> s,
                                                                         TileLists T, Lists L, SolverConsts<float> c,
                                                                         int* __restrict__ status) {
+    chain_entry();
     phase_begins(s.phase_at, 2);
     extern __shared__ float4 tile_smem[];
     const int half = threadIdx.x & 1;
@@ -1777,12 +1779,12 @@ __global__ void k_export_solver_lists(int64_t n_owners, bool tiled, TileLists T,
 }
 
 // the instantiation of a tuned kernel for a prefetch depth in 1..kMaxAhead
-#define FSB_AHEAD_SWITCH(ahead, KERNEL, ...)       \
-    switch (ahead) {                                  \
-        case 1: KERNEL<1> __VA_ARGS__; break;         \
-        case 2: KERNEL<2> __VA_ARGS__; break;         \
-        case 3: KERNEL<3> __VA_ARGS__; break;         \
-        default: KERNEL<kMaxAhead> __VA_ARGS__; break; \
+#define FSB_AHEAD_SWITCH(ahead, KERNEL, CALL) \
+    switch (ahead) {                          \
+        case 1: CALL(KERNEL<1>); break;       \
+        case 2: CALL(KERNEL<2>); break;       \
+        case 3: CALL(KERNEL<3>); break;       \
+        default: CALL(KERNEL<kMaxAhead>); break; \
     }
 
 // the pressure passes' instantiation for a prefetch depth and a number of
