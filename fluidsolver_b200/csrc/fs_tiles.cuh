@@ -1272,7 +1272,8 @@ __global__ void __launch_bounds__(pressure_threads<TPO>(), update_blocks_per_sm<
 //
 // Measured on a B200, one iteration of a dam's loop, the WHILE node against this:
 // 512 fluid particles 17.0 -> 12.6 us, 8,000 16.4 -> 11.9, 29,791 18.8 -> 13.9,
-// 100,000 34.6 -> 28.9, 250,047 65.5 -> 60.9, 512,000 115 -> 110. A pass of a
+// 100,000 34.6 -> 28.9, 250,047 65.5 -> 60.9, 512,000 115 -> 110 (26.6, 57.6 and
+// 106 since the entries are spread over the banks, k_build_tiles). A pass of a
 // small scene is a chain of latencies (copying the field 0.7 us, the walk 1.4,
 // the barrier 1.7), and the fallback tiles' are the longest.
 //
