@@ -376,12 +376,19 @@ void choose_dims(int dim, int64_t max_cells, const int* lo_in, const int* hi_in,
     for (int a = 0; a < 3; a++) dims[a] = (int)ext[a];
 }
 
+// the grids of an upload's scenes, before the context takes them over
+struct GridPlan {
+    std::vector<SceneGrid> grids;
+    int64_t cells = 0;       // of all scenes
+    int64_t box_cells = 0;   // of the particles' boxes
+};
+
 // every scene's grid from its box (lo[3 s + a], hi[3 s + a]); scene s may
 // hold up to max(4M, 8 * its particles) cells, and all scenes 2^30
-fs_status choose_grids(fs_ctx* c, const int* lo, const int* hi) {
+fs_status choose_grids(const fs_ctx* c, const int* lo, const int* hi, GridPlan& plan) {
     const int S = c->nsc();
-    c->grids_host.assign(S, SceneGrid{});
-    c->box_cells = 0;
+    plan.grids.assign(S, SceneGrid{});
+    plan.box_cells = 0;
     int64_t base = 0;
     for (int sidx = 0; sidx < S; sidx++) {
         const int64_t np = c->scenes > 0 ? c->scene_offsets[sidx + 1] - c->scene_offsets[sidx] : c->cap;
@@ -393,8 +400,8 @@ fs_status choose_grids(fs_ctx* c, const int* lo, const int* hi) {
             const int64_t e = (int64_t)hi[3 * sidx + a] - lo[3 * sidx + a] + 1;
             in_box *= std::max<int64_t>(1, std::min<int64_t>(e, d[a]));
         }
-        c->box_cells += in_box;
-        SceneGrid& g = c->grids_host[sidx];
+        plan.box_cells += in_box;
+        SceneGrid& g = plan.grids[sidx];
         g.d0 = d[0];
         g.d1 = d[1];
         g.d2 = d[2];
@@ -402,27 +409,40 @@ fs_status choose_grids(fs_ctx* c, const int* lo, const int* hi) {
         base += (int64_t)d[0] * d[1] * d[2];
     }
     if (base > (int64_t(1) << 30)) return fail(FS_ERR_INVALID, "the scenes' cell grids exceed 2^30 cells");
-    for (int a = 0; a < 3; a++) c->dims[a] = a == 0 ? c->grids_host[0].d0 : (a == 1 ? c->grids_host[0].d1 : c->grids_host[0].d2);
-    c->cells = base;
-    // (a single scene's grid goes with the packing kernel)
-    if (c->scenes > 0)
-        FS_CUDA(cudaMemcpyAsync(c->grids, c->grids_host.data(), sizeof(SceneGrid) * S, cudaMemcpyHostToDevice, c->stream));
+    plan.cells = base;
     return FS_OK;
 }
-
-// cell tables for the current dims
-fs_status ensure_cells(fs_ctx* c) {
+fs_status take_grids(fs_ctx* c, GridPlan& plan) {
+    c->grids_host.swap(plan.grids);
+    c->cells = plan.cells;
+    c->box_cells = plan.box_cells;
+    const SceneGrid& g = c->grids_host[0];
+    c->dims[0] = g.d0;
+    c->dims[1] = g.d1;
+    c->dims[2] = g.d2;
     c->key_bits = 1;
     while ((int64_t(1) << c->key_bits) < c->cells) c->key_bits++;
     c->regions = c->reference_order ? 1 : (c->include_inactive ? 3 : 2);
-    const int64_t need = c->cells + 1;
-    if (!c->cell_start || c->cell_alloc < need) {
+    // (a single scene's grid goes with the packing kernel)
+    if (c->scenes > 0)
+        FS_CUDA(cudaMemcpyAsync(c->grids, c->grids_host.data(), sizeof(SceneGrid) * c->nsc(), cudaMemcpyHostToDevice,
+                                c->stream));
+    return FS_OK;
+}
+
+// cell tables for grids of that many cells. Where their allocation fails, the
+// next search tries it again.
+fs_status ensure_cells(fs_ctx* c, int64_t cells) {
+    const int64_t need = cells + 1;
+    if (c->cell_alloc < need) {
         clear_graphs(c);
         if (c->cell_start) cudaFree(c->cell_start);
         if (c->cell_partials) cudaFree(c->cell_partials);
         if (c->look_tiles) cudaFree(c->look_tiles);
         c->cell_start = c->cell_partials = nullptr;
         c->look_tiles = nullptr;
+        c->cell_alloc = 0;
+        c->have_cells = false;
         FS_TRY(dalloc(&c->cell_start, (size_t)3 * need + 4));   // the counting path's extra entry, whole uint4
         FS_TRY(dalloc(&c->cell_partials, (size_t)scan_tiles(3 * need)));
         FS_TRY(dalloc(&c->look_tiles, (size_t)look_tiles(3 * need + 1)));
@@ -1562,6 +1582,7 @@ fs_status fill_stats(fs_ctx* c, fs_step_stats* stats, int st, int entries = 1) {
 // capacity the lists are grown and the search is repeated once.
 // Phase timestamps 0 and 1 are its begin and end.
 fs_status search_for_step(fs_ctx* c, float dt) {
+    FS_TRY(ensure_cells(c, c->cells));
     for (int attempt = 0; attempt < 3; attempt++) {
         c->launches++;
         k_step_begin<<<grid_for(c->nsc(), 128), 128, 0, c->stream>>>(c->scalars, c->nsc(), dt, false);
@@ -1789,6 +1810,7 @@ fs_status enqueue_small_steps(fs_ctx* c, int32_t steps, float dt) {
 }
 
 fs_status enqueue_steps(fs_ctx* c, int32_t steps, float dt) {
+    FS_TRY(ensure_cells(c, c->cells));
     FS_CUDA(cudaMemsetAsync(c->status, 0, sizeof(int), c->stream));
     c->small_last = small_eligible(c);
     if (c->small_last) {
@@ -2030,28 +2052,39 @@ fs_status fs_upload(fs_ctx* c, const fs_particles* in) {
         return fail(FS_ERR_INVALID, "a batched upload holds exactly the particles of every scene");
     FS_CUDA(cudaSetDevice(c->device));
     StagedUpload d;
-    // whatever ends the call, the copies from the caller's arrays are over by then
-    struct CopiesDone {
+    // However the call ends, the copies from the caller's arrays are over by
+    // then; and if it ends before the packing, which clears the census, that
+    // starts afresh.
+    struct Ending {
         fs_ctx* c;
-        bool all = true;
-        ~CopiesDone() { all ? cudaStreamSynchronize(c->stream) : cudaEventSynchronize(c->copied); }
-    } done{c};
+        bool packed = false, all = true;
+        ~Ending() {
+            if (!packed) {
+                const size_t half = 3 * (size_t)c->nsc() * sizeof(int);
+                (void)cudaMemsetAsync(c->search_state->counts, 0, sizeof(c->search_state->counts), c->stream);
+                (void)cudaMemsetAsync(c->search_box, 0x7f, half, c->stream);
+                (void)cudaMemsetAsync(c->search_box + 3 * c->nsc(), 0x80, half, c->stream);
+            }
+            all ? cudaStreamSynchronize(c->stream) : cudaEventSynchronize(c->copied);
+        }
+    } ending{c};
     FS_TRY(stage_upload(c, in, d));
     const unsigned long long* counts = c->upload_host->counts;
-    const bool invalid = counts[3] != 0;
+    if (counts[3] != 0) return fail(FS_ERR_INVALID, "particle type must be 0, 1 or 2");
+    if (counts[0] + counts[1] + counts[2] != (unsigned long long)in->n)
+        return fail(FS_ERR_CUDA, "the upload's particle counts do not add up");
+    // whatever can fail comes before the context takes the new layout: until
+    // then the state stays as it was
+    GridPlan plan;
+    FS_TRY(choose_grids(c, c->upload_boxes(), c->upload_boxes() + 3 * c->nsc(), plan));
+    FS_TRY(ensure_cells(c, plan.cells));
     const int64_t n_before = c->n, owners_before = c->n_owners;
-    if (invalid) {   // the census starts afresh; the state stays as it was
-        FS_CUDA(cudaMemsetAsync(c->search_state->counts, 0, sizeof(c->search_state->counts), c->stream));
-        FS_CUDA(cudaMemsetAsync(c->search_box, 0x7f, 3 * c->nsc() * sizeof(int), c->stream));
-        FS_CUDA(cudaMemsetAsync(c->search_box + 3 * c->nsc(), 0x80, 3 * c->nsc() * sizeof(int), c->stream));
-        return fail(FS_ERR_INVALID, "particle type must be 0, 1 or 2");
-    }
     set_layout(c, in->n, (int64_t)counts[0], (int64_t)counts[1], (int64_t)counts[2]);
     if (c->n != n_before || c->n_owners != owners_before) clear_graphs(c);
-    FS_TRY(choose_grids(c, c->upload_boxes(), c->upload_boxes() + 3 * c->nsc()));
-    FS_TRY(ensure_cells(c));
+    FS_TRY(take_grids(c, plan));
     fs_status r = c->precision == FS_PRECISION_FP64 ? pack_upload<double>(c, d, in->n) : pack_upload<float>(c, d, in->n);
     if (r != FS_OK) return r;
+    ending.packed = true;
     // The 2D hashed grid's history lives as long as the context, like the
     // reference's search object, whose grid survives changes of the
     // collection's contents; a different particle count starts it afresh.
@@ -2062,7 +2095,7 @@ fs_status fs_upload(fs_ctx* c, const fs_particles* in) {
     c->have_state = true;
     c->have_lists = false;
     c->have_cells = false;
-    done.all = c->scenes > 0;   // (the packing may still run; a batch's grids are copied behind it)
+    ending.all = c->scenes > 0;   // (the packing may still run; a batch's grids are copied behind it)
     return FS_OK;
 }
 
