@@ -651,7 +651,9 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_steps(SmallStepArgs<
                 for (int64_t k = T.first(no); k < T.end(no); k += kSmallThreads) f(k);
                 for (int64_t k = no + T.first(n - no); k < no + T.end(n - no); k += kSmallThreads) f(k);
             };
-            if (ok1 && a.split) {
+            if (!ok1) {
+                all_particles([&](int64_t k) { carry_density(k, n, s); });
+            } else if (a.split) {
                 all_particles([&](int64_t k) {
                     if (two_d) iisph2d_density_at<R, KAHAN>(k, v, Lv, a.c);
                     else iisph3d_density_at<R, KAHAN>(k, v, Lv, a.c);

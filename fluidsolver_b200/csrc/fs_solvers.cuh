@@ -118,6 +118,13 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
+// The first loop reads the previous densities and writes the new ones to
+// another buffer. A step that an error has ended computes none: it carries the
+// densities over, so that the state stays whole.
+template <typename R> __device__ __forceinline__ void carry_density(int64_t k, int64_t n, const State<R>& s) {
+    if (k < n) s.rho[k] = s.rho_prev[k];
+}
+
 // ===========================================================================
 // viscosity term (IISPHFluidSolver3D.hpp:43-76, SESPHFluidSolver3D.hpp:293-324,
 // IISPHFluidSolver.hpp:240-277, SESPHFluidSolver.hpp:254-285):
@@ -210,7 +217,11 @@ __global__ void k_iisph3d_l1(int64_t n, State<R> s, Lists L, SolverConsts<R> c, 
                              const int* FSB_R status) {
     phase_begins(s.phase_at, 1);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k >= n || *status) return;
+    if (*status) {
+        if (!SPLIT) carry_density(k, n, s);   // (SPLIT: the density pass has)
+        return;
+    }
+    if (k >= n) return;
     iisph3d_l1_one<R, KAHAN, SPLIT>(k, s, L, c, (R)sc->dt);
 }
 
@@ -239,7 +250,8 @@ template <typename R, bool KAHAN>
 __global__ void k_iisph3d_density(int64_t n, State<R> s, Lists L, SolverConsts<R> c, const int* FSB_R status) {
     phase_begins(s.phase_at, 1);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k >= n || *status) return;
+    if (*status) return carry_density(k, n, s);
+    if (k >= n) return;
     iisph3d_density_at<R, KAHAN>(k, s, L, c);
 }
 
@@ -927,7 +939,11 @@ __global__ void k_iisph2d_l1(int64_t n, State<R> s, Lists L, SolverConsts<R> c, 
                              const int* FSB_R status) {
     phase_begins(s.phase_at, 1);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k >= n || *status) return;
+    if (*status) {
+        if (!SPLIT) carry_density(k, n, s);   // (SPLIT: the density pass has)
+        return;
+    }
+    if (k >= n) return;
     iisph2d_l1_at<R, KAHAN, SPLIT>(k, s, L, c, (R)sc->dt);
 }
 
@@ -952,7 +968,8 @@ template <typename R, bool KAHAN>
 __global__ void k_iisph2d_density(int64_t n, State<R> s, Lists L, SolverConsts<R> c, const int* FSB_R status) {
     phase_begins(s.phase_at, 1);
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k >= n || *status) return;
+    if (*status) return carry_density(k, n, s);
+    if (k >= n) return;
     iisph2d_density_at<R, KAHAN>(k, s, L, c);
 }
 
