@@ -956,9 +956,11 @@ __global__ void __launch_bounds__(128) k_csr_fill(int64_t n, const V4<R>* FSB_R 
 
 // Sorts the lists of host indices [h0, h1) into out (from out[0], 64-bit). A
 // warp per list of at most kCsrWarpMax members: each member's place is the
-// number of smaller members (they are distinct), counted over the list's copy
-// in shared memory, four at a time by broadcast reads. Quadratic, but about
-// 300 warp instructions at 34 members, and no exchange network's barriers.
+// number of smaller members and of equal ones before it (beyond 2^30 cells,
+// where compact hashing's coordinates end, a list holds a member several
+// times), counted over the list's copy in shared memory, four at a time by
+// broadcast reads. Quadratic, but about 400 warp instructions at 34 members,
+// and no exchange network's barriers.
 constexpr int kCsrWarpMax = 512;
 constexpr int kCsrSortWarps = 4;
 static __global__ void __launch_bounds__(32 * kCsrSortWarps) k_csr_sort(int64_t h0, int64_t h1,
@@ -981,7 +983,8 @@ static __global__ void __launch_bounds__(32 * kCsrSortWarps) k_csr_sort(int64_t 
         int r = 0;
         for (int q = 0; q < L4; q += 4) {
             const uint4 x = *reinterpret_cast<const uint4*>(s + q);
-            r += (x.x < v) + (x.y < v) + (x.z < v) + (x.w < v);
+            // (indices are below 2^31: x < v + 1 is x <= v)
+            r += (x.x < v + (q < e)) + (x.y < v + (q + 1 < e)) + (x.z < v + (q + 2 < e)) + (x.w < v + (q + 3 < e));
         }
         o[r] = (int64_t)v;
     }
