@@ -336,9 +336,7 @@ fs_status ensure_lists(fs_ctx* c, int K) {
         c->tile_stride = tiles * kTileOwners;
         FS_TRY(dalloc(&c->tile_desc, (size_t)tiles));
         FS_TRY(dalloc(&c->tile_ent, (size_t)(K / 8) * c->tile_stride));
-        FS_CUDA(cudaFuncSetAttribute(k_build_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)tile_build_smem(K, kTileCapMax)));
-        FS_CUDA(set_tile_pass_smem(K));
+        FS_CUDA(set_tile_smem(K));
     }
     // stored gradients of the IISPH gather phases (fs_cached.cuh): up to
     // kGradientBytes, and as a convenience only (without them the phases

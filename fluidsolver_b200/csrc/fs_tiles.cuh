@@ -26,6 +26,8 @@
 // reference, which the compensated sums absorb.
 #pragma once
 
+#include <mutex>
+
 #include "fs_common.cuh"
 #include "fs_search.cuh"
 #include "fs_solvers.cuh"
@@ -1807,40 +1809,44 @@ __global__ void k_export_solver_lists(int64_t n_owners, bool tiled, TileLists T,
     }
 static_assert(kMaxAhead == 4, "FSB_PRESSURE_SWITCH lists depths 1..4");
 
+// Lets a kernel ask for `needs` bytes of dynamic shared memory (more than a
+// block may have: cudaErrorInvalidValue). The limit belongs to the process and
+// is only ever raised: lowered to what one context's capacity needs, it would
+// refuse the launches of a context with longer lists.
+template <typename Kernel> inline cudaError_t allow_smem(Kernel* kernel, size_t needs) {
+    static std::mutex one_at_a_time;
+    const std::lock_guard<std::mutex> lock(one_at_a_time);
+    cudaFuncAttributes f{};
+    const cudaError_t e = cudaFuncGetAttributes(&f, kernel);
+    if (e != cudaSuccess || (size_t)f.maxDynamicSharedSizeBytes >= needs) return e;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)needs);
+}
+
 template <int AHEAD, int TPO> inline cudaError_t set_pressure_smem(int K) {
-    cudaError_t e = cudaFuncSetAttribute(k_tile_iisph3d_pressure_acc<AHEAD, TPO>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)tile_pass_smem(20, K, false, kTileCapMax));
+    cudaError_t e = allow_smem(k_tile_iisph3d_pressure_acc<AHEAD, TPO>, tile_pass_smem(20, K, false, kTileCapMax));
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_tile_iisph3d_pressure_update<AHEAD, TPO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)tile_pass_smem(32, K, false, kTileCapMax));
+        e = allow_smem(k_tile_iisph3d_pressure_update<AHEAD, TPO>, tile_pass_smem(32, K, false, kTileCapMax));
     return e;
 }
 
 template <int AHEAD> inline cudaError_t set_tuned_pass_smem(int K) {
-    cudaError_t e = cudaFuncSetAttribute(k_tile_iisph3d_l1<AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)tile_pass_smem(36, K, !kL1GlobalEntries, kTileCapMax));
+    cudaError_t e = allow_smem(k_tile_iisph3d_l1<AHEAD>, tile_pass_smem(36, K, !kL1GlobalEntries, kTileCapMax));
     if (e == cudaSuccess) e = set_pressure_smem<AHEAD, 1>(K);
     if (e == cudaSuccess) e = set_pressure_smem<AHEAD, 2>(K);
     if (e == cudaSuccess) e = set_pressure_smem<AHEAD, 4>(K);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_tile_sesph3d_density<AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)tile_pass_smem(16, K, false, kTileCapMax));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_tile_sesph3d_accel<AHEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)tile_pass_smem(36, K, false, kTileCapMax));
+    if (e == cudaSuccess) e = allow_smem(k_tile_sesph3d_density<AHEAD>, tile_pass_smem(16, K, false, kTileCapMax));
+    if (e == cudaSuccess) e = allow_smem(k_tile_sesph3d_accel<AHEAD>, tile_pass_smem(36, K, false, kTileCapMax));
     return e;
 }
 
-inline cudaError_t set_tile_pass_smem(int K) {
-    cudaError_t e = cudaFuncSetAttribute(k_tile_iisph3d_l2, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)tile_pass_smem(32, K, !kL2GlobalEntries, kTileCapMax));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_tile_iisph3d_pressure_loop<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)tile_loop_smem(false, K, kTileCapMax));
+// the tile kernels of a context with lists of K entries
+inline cudaError_t set_tile_smem(int K) {
+    cudaError_t e = allow_smem(k_build_tiles, tile_build_smem(K, kTileCapMax));
+    if (e == cudaSuccess) e = allow_smem(k_tile_iisph3d_l2, tile_pass_smem(32, K, !kL2GlobalEntries, kTileCapMax));
+    if (e == cudaSuccess) e = allow_smem(k_tile_iisph3d_pressure_loop<false>, tile_loop_smem(false, K, kTileCapMax));
     if (e == cudaSuccess)   // (the launch asks for no more than a block may have, pressure_loop_form)
-        e = cudaFuncSetAttribute(k_tile_iisph3d_pressure_loop<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)std::min<size_t>(tile_loop_smem(true, K, kTileCapMax), kLoopSmemMax));
+        e = allow_smem(k_tile_iisph3d_pressure_loop<true>,
+                       std::min<size_t>(tile_loop_smem(true, K, kTileCapMax), kLoopSmemMax));
     if (e == cudaSuccess) e = set_tuned_pass_smem<1>(K);
     if (e == cudaSuccess) e = set_tuned_pass_smem<2>(K);
     if (e == cudaSuccess) e = set_tuned_pass_smem<3>(K);
