@@ -1861,6 +1861,21 @@ fs_status one_step(fs_ctx* c, float desired_dt, fs_step_stats* stats) {
     return solve_after_search(c, dt, stats);
 }
 
+// What a captured step holds of an upload's layout beside its grid (which the
+// graphs' keys name): the counts that its kernels are given, and which
+// of them the sizes chose.
+struct CapturedLayout {
+    int64_t n, n_struct, n_owners;
+    bool counting, lists, first, pressure;
+    bool operator!=(const CapturedLayout& o) const {
+        return n != o.n || n_struct != o.n_struct || n_owners != o.n_owners || counting != o.counting ||
+               lists != o.lists || first != o.first || pressure != o.pressure;
+    }
+};
+CapturedLayout captured_layout(const fs_ctx* c) {
+    return {c->n, c->n_struct, c->n_owners, counting_order(c), grouped_lists(c), grouped(c), grouped_pressure(c)};
+}
+
 }  // namespace
 
 // ===========================================================================
@@ -2076,10 +2091,10 @@ fs_status fs_upload(fs_ctx* c, const fs_particles* in) {
     GridPlan plan;
     FS_TRY(choose_grids(c, c->upload_boxes(), c->upload_boxes() + 3 * c->nsc(), plan));
     FS_TRY(ensure_cells(c, plan.cells));
-    const int64_t n_before = c->n, owners_before = c->n_owners;
+    const CapturedLayout before = captured_layout(c);
     set_layout(c, in->n, (int64_t)counts[0], (int64_t)counts[1], (int64_t)counts[2]);
-    if (c->n != n_before || c->n_owners != owners_before) clear_graphs(c);
     FS_TRY(take_grids(c, plan));
+    if (captured_layout(c) != before) clear_graphs(c);
     fs_status r = c->precision == FS_PRECISION_FP64 ? pack_upload<double>(c, d, in->n) : pack_upload<float>(c, d, in->n);
     if (r != FS_OK) return r;
     ending.packed = true;
