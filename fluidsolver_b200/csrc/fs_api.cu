@@ -929,24 +929,20 @@ template <typename R> fs_status order_by_counting(fs_ctx* c, State<R> s) {
     const int nx = c->cur ^ 1;
     c->launches += 5;
     launch_pdl(pdl, k_search_box<R>, gb, 256, 0, st, n, s.pos, s.type, s.scene, c->nsc(), c->include_inactive,
-               c->search_radius,
-                                        c->truncate_cells, c->search_box, c->grids, c->search_state,
-                                        (uint4*)c->cell_start, (entries + 3) / 4, c->look_tiles, tiles);
-    launch_pdl(pdl, k_search_keys<R>, grid_for(n, pb), pb, 0, st, n, s.pos, s.type, s.hidx, c->include_inactive,
-               single,
-                                                     c->search_radius, c->truncate_cells, c->grids, s.scene, c->cells,
-                                                     excluded, entry, slot, order, c->h2d_cell, c->h2d_rank,
-                                                     c->cell_start, c->status);
+               c->search_radius, c->truncate_cells, c->search_box, c->grids, c->search_state, (uint4*)c->cell_start,
+               (entries + 3) / 4, c->look_tiles, tiles);
+    launch_pdl(pdl, k_search_keys<R>, grid_for(n, pb), pb, 0, st, n, s.pos, s.type, s.hidx, c->include_inactive, single,
+               c->search_radius, c->truncate_cells, c->grids, s.scene, c->cells, excluded, entry, slot, order,
+               c->h2d_cell, c->h2d_rank, c->cell_start, c->status);
     launch_pdl(pdl, k_search_scan, (unsigned)tiles, kLookThreads, 0, st, c->cell_start, entries, c->look_tiles,
-               c->search_state,
-                                                            c->status);
-    launch_pdl(pdl, k_search_scatter, grid_for(n, pb), pb, 0, st, n, entry, slot, c->cell_start, list, c->status);
-    launch_pdl(pdl, k_search_reorder<R>, grid_for(n, pb), pb, 0, st,
-        n, c->n_struct, excluded, list, entry, order, c->cell_start, (const V4<R>*)c->pos[c->cur], (V4<R>*)c->pos[nx],
-        (const V4<R>*)c->vel[c->cur], (V4<R>*)c->vel[nx], (const V4<R>*)c->acc[c->cur], (V4<R>*)c->acc[nx],
-        (const V4<R>*)c->ext[c->cur], (V4<R>*)c->ext[nx], (const R*)c->rho[c->cur], (R*)c->rho[nx],
-        (const R*)c->p[c->cur], (R*)c->p[nx], c->type[c->cur], c->type[nx], c->hidx[c->cur], c->hidx[nx],
-        c->scene_of[c->cur], c->scene_of[nx], c->h2d_rank, c->status);
+               c->search_state, c->scan_tries, c->status);
+    launch_pdl(pdl, k_search_scatter, grid_for(n, pb), pb, 0, st, n, entry, slot, c->cell_start, list, c->search_state);
+    launch_pdl(pdl, k_search_reorder<R>, grid_for(n, pb), pb, 0, st, n, c->n_struct, excluded, list, entry, order,
+               c->cell_start, (const V4<R>*)c->pos[c->cur], (V4<R>*)c->pos[nx], (const V4<R>*)c->vel[c->cur],
+               (V4<R>*)c->vel[nx], (const V4<R>*)c->acc[c->cur], (V4<R>*)c->acc[nx], (const V4<R>*)c->ext[c->cur],
+               (V4<R>*)c->ext[nx], (const R*)c->rho[c->cur], (R*)c->rho[nx], (const R*)c->p[c->cur], (R*)c->p[nx],
+               c->type[c->cur], c->type[nx], c->hidx[c->cur], c->hidx[nx], c->scene_of[c->cur], c->scene_of[nx],
+               c->h2d_rank, c->search_state);
     FS_CUDA(cudaGetLastError());
     c->cur = nx;
     return FS_OK;
@@ -1028,6 +1024,13 @@ fs_status read_back(fs_ctx* c, bool scalars, int* st = nullptr) {
     FS_CUDA(cudaStreamSynchronize(c->stream));
     if (st) *st = c->upload_host->status;
     return FS_OK;
+}
+
+// After FS_ERR_TIMEOUT: a scan that gave up (in the last search) has left no cell table.
+void note_timeout(fs_ctx* c, int st) {
+    SearchState h{};
+    if (st != FS_ERR_TIMEOUT || cudaMemcpy(&h, c->search_state, sizeof(h), cudaMemcpyDeviceToHost) != cudaSuccess) return;
+    if (h.scan_failed) c->have_cells = c->have_lists = false;
 }
 
 // Phase timestamp i of the host-driven path. In a captured step the kernels
@@ -1217,7 +1220,7 @@ fs_status enqueue_pressure_loop_launch(fs_ctx* c, int form, unsigned blocks, siz
                                        const SolverConsts<float>& k) {
     const fs_params& p = c->prm;
     const LoopTest lt{p.min_iterations, p.max_iterations, p.max_density_error, p.particle_size, cfl_default(c),
-                      p.lambda_v, p.lambda_a};
+                      p.lambda_v, p.lambda_a, c->barrier_tries};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(kPassThreads);
@@ -1598,6 +1601,7 @@ fs_status search_for_step(fs_ctx* c, float dt) {
             FS_TRY(ensure_lists(c, K));
             continue;
         }
+        note_timeout(c, st);
         if (st != FS_OK)
             return fail((fs_status)st, st == FS_ERR_CAPACITY ? "neighbor list capacity exceeded"
                                                              : "device reported an error during the search");
@@ -1836,6 +1840,7 @@ fs_status read_phase_times(fs_ctx* c) {
 
 fs_status finish_steps(fs_ctx* c, fs_step_stats* stats, int* st) {
     FS_TRY(read_back(c, true, st));
+    note_timeout(c, *st);
     FS_TRY(read_phase_times(c));
     fill_stats(c, stats, *st);
     return FS_OK;
@@ -2776,6 +2781,16 @@ fs_status fs_set_tile_wait_limit(fs_ctx* c, int32_t tries) {
     const int v = tries < 0 ? kTileWaitTries : tries;
     FS_CUDA(cudaStreamSynchronize(c->stream));
     FS_CUDA(cudaMemcpyToSymbol(g_tile_wait_tries, &v, sizeof(int)));
+    return FS_OK;
+}
+
+fs_status fs_set_grid_wait_limits(fs_ctx* c, int32_t scan_tries, int32_t barrier_tries) {
+    if (!c) return fail(FS_ERR_INVALID, "ctx is null");
+    FS_CUDA(cudaSetDevice(c->device));
+    FS_CUDA(cudaStreamSynchronize(c->stream));
+    clear_graphs(c);   // the captured steps hold the limits
+    c->scan_tries = scan_tries < 0 ? kLookTries : scan_tries;
+    c->barrier_tries = barrier_tries < 0 ? kLoopBarrierTries : barrier_tries;
     return FS_OK;
 }
 

@@ -54,6 +54,8 @@ struct fs_ctx {
     bool sort_lists_by_host = false;  // quadratic list order (reference-order mode)
     int ns_owner_mode = 0;          // 0 all in structure, 1 fluid only, 2 active only
     int precision = FS_PRECISION_FP32_KAHAN;
+    int scan_tries = fsb::kLookTries;            // bounds of the waits between a grid's blocks
+    int barrier_tries = fsb::kLoopBarrierTries;  // (fs_set_grid_wait_limits)
     fsb::TileTuning tuning;         // prefetch depths of the tile passes (fs_autotune)
     size_t real_size = 4;
 

@@ -329,6 +329,7 @@ __global__ void k_reorder(int64_t n, const uint32_t* FSB_R perm, const V4<R>* FS
 struct SearchState {
     uint32_t box_ticket;     // blocks of k_search_box that are done (its last block clears it)
     uint32_t scan_ticket;    // tiles of the scan handed out (cleared by k_search_box)
+    uint32_t scan_failed;    // the scan gave up: the table is incomplete (cleared by k_search_box)
     unsigned long long counts[4];   // an upload's particles per type (index 3: invalid types; cleared when it is packed)
 };
 
@@ -341,7 +342,7 @@ __global__ void k_search_box(int64_t n, const V4<R>* FSB_R pos, const uint8_t* F
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, total = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = t; i < table16; i += total) table[i] = make_uint4(0u, 0u, 0u, 0u);
     for (int64_t i = t; i < ntiles; i += total) tiles[i] = 0ull;
-    if (t == 0) st->scan_ticket = 0u;
+    if (t == 0) st->scan_ticket = st->scan_failed = 0u;
     bbox_block<R>(n, pos, type, scene, scenes, include_inactive, r, trunc, box);
     __threadfence();
     __syncthreads();
@@ -401,11 +402,12 @@ __global__ void k_search_keys(int64_t n, const V4<R>* FSB_R pos, const uint8_t* 
 // total, 2: the total up to its end) << 32 | value.
 constexpr int kLookThreads = 256;
 constexpr int kLookTile = kLookThreads * 16;
-constexpr int kLookTries = 1 << 22;   // polls of a predecessor before the scan gives up (FS_ERR_TIMEOUT)
+constexpr int kLookTries = 1 << 22;   // polls of a predecessor before the scan gives up
 inline int64_t look_tiles(int64_t m) { return (m + kLookTile - 1) / kLookTile; }
 static __global__ void __launch_bounds__(kLookThreads) k_search_scan(uint32_t* FSB_R a, int64_t m,
                                                                      unsigned long long* FSB_R tiles,
-                                                                     SearchState* FSB_R st, int* FSB_R status) {
+                                                                     SearchState* FSB_R st, int max_tries,
+                                                                     int* FSB_R status) {
     chain_entry();
     __shared__ uint32_t s_warp[kLookThreads / 32], s_tile, s_before;
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
@@ -449,10 +451,12 @@ static __global__ void __launch_bounds__(kLookThreads) k_search_scan(uint32_t* F
                 const int64_t i = last - lane;
                 unsigned long long x = 2ull << 32;   // before the first tile: a total of 0
                 if (i >= 0) {
-                    int tries = 0;
-                    while (((x = look[i]) >> 32) == 0ull && ++tries < kLookTries) {}
+                    x = 0ull;
+                    for (int tries = 0; tries < max_tries && (x >> 32) == 0ull; tries++) x = look[i];
                     if ((x >> 32) == 0ull) {
-                        raise_status(status, FS_ERR_TIMEOUT);
+                        // (whatever an earlier kernel has raised: nothing may be built on this table)
+                        atomicExch(status, FS_ERR_TIMEOUT);
+                        st->scan_failed = 1u;
                         x = 2ull << 32;
                     }
                 }
@@ -478,18 +482,20 @@ static __global__ void __launch_bounds__(kLookThreads) k_search_scan(uint32_t* F
     }
 }
 
-// (after a scan that gave up nothing may be placed: the table is incomplete)
+// (after a scan that gave up nothing may be placed)
 static __global__ void k_search_scatter(int64_t n, const uint32_t* FSB_R entry, const uint32_t* FSB_R slot,
                                         const uint32_t* FSB_R cell_start, uint32_t* FSB_R list,
-                                        const int* FSB_R status) {
+                                        const SearchState* FSB_R st) {
     chain_entry();
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k >= n || *status == FS_ERR_TIMEOUT) return;
+    if (k >= n || st->scan_failed) return;
     list[cell_start[entry[k]] + slot[k]] = (uint32_t)k;
 }
 
 // Particle list[i]'s place, and its fields moved there (k_reorder's); with the
-// 2D hashed grid's history also its rank in the cell (k_h2d_rank's)
+// 2D hashed grid's history also its rank in the cell (k_h2d_rank's). After a
+// scan that gave up the particles stay where they are, in the other buffer, and
+// the history starts afresh.
 template <typename R>
 __global__ void k_search_reorder(int64_t n, int64_t n_struct, uint32_t excluded, const uint32_t* FSB_R list,
                                  const uint32_t* FSB_R entry, const uint32_t* FSB_R order,
@@ -499,28 +505,32 @@ __global__ void k_search_reorder(int64_t n, int64_t n_struct, uint32_t excluded,
                                  R* FSB_R rho1, const R* FSB_R p0, R* FSB_R p1, const uint8_t* FSB_R t0,
                                  uint8_t* FSB_R t1, const uint32_t* FSB_R h0, uint32_t* FSB_R h1,
                                  const uint16_t* FSB_R sc0, uint16_t* FSB_R sc1, uint32_t* FSB_R h2d_rank,
-                                 const int* FSB_R status) {
+                                 const SearchState* FSB_R st) {
     chain_entry();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n || *status == FS_ERR_TIMEOUT) return;
-    const uint32_t k = list[i], e = entry[k];
-    const uint32_t b = cell_start[e], end = e == excluded ? (uint32_t)n : cell_start[e + 1];
+    if (i >= n) return;
+    const bool failed = st->scan_failed != 0u;
+    const uint32_t k = failed ? (uint32_t)i : list[i];
     // the particle's fields, on their way while its place is counted
     const V4<R> x = pos0[k], v = vel0[k], a = acc0[k], f = ext0[k];
     const R rho = rho0[k], p = p0[k];
     const uint8_t ty = t0[k];
     const uint32_t h = h0[k];
-    uint32_t rank = 0;
-    if (order) {
-        const uint32_t mine = order[k];
-        for (uint32_t j = b; j < end; j++) {
-            const uint32_t q = list[j], o = order[q];
-            rank += (o < mine || (o == mine && q < k)) ? 1u : 0u;
+    uint32_t d = k, rank = 0xffffffffu;
+    if (!failed) {
+        const uint32_t e = entry[k], b = cell_start[e], end = e == excluded ? (uint32_t)n : cell_start[e + 1];
+        rank = 0;
+        if (order) {
+            const uint32_t mine = order[k];
+            for (uint32_t j = b; j < end; j++) {
+                const uint32_t q = list[j], o = order[q];
+                rank += (o < mine || (o == mine && q < k)) ? 1u : 0u;
+            }
+        } else {
+            for (uint32_t j = b; j < end; j++) rank += list[j] < k ? 1u : 0u;
         }
-    } else {
-        for (uint32_t j = b; j < end; j++) rank += list[j] < k ? 1u : 0u;
+        d = b + rank;
     }
-    const uint32_t d = b + rank;
     pos1[d] = x;
     vel1[d] = v;
     acc1[d] = a;

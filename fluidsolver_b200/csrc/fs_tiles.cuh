@@ -1291,12 +1291,13 @@ struct LoopTest {
     int min_it, max_it;
     float max_err;
     float particle_size, cfl_timestep, lambda_v, lambda_a;
+    int barrier_tries;   // kLoopBarrierTries (fs_set_grid_wait_limits may lower it)
 };
 
 // Waits until `target` blocks have arrived at the launch's barriers in all
 // (every block adds 1 per barrier). False, in every thread, when the wait ran
 // out (FS_ERR_TIMEOUT raised) or another block failed.
-__device__ __forceinline__ bool loop_barrier(unsigned int* arrived, unsigned int target, int* status) {
+__device__ __forceinline__ bool loop_barrier(unsigned int* arrived, unsigned int target, int max_tries, int* status) {
     // this thread's stores, before other blocks' bulk copies (the release and
     // the block barrier before it order them for the other blocks' loads)
     asm volatile("fence.proxy.async.global;" ::: "memory");
@@ -1306,20 +1307,18 @@ __device__ __forceinline__ bool loop_barrier(unsigned int* arrived, unsigned int
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
         int tries = 0;
         while (true) {
+            if (tries >= max_tries) {
+                raise_status(status, FS_ERR_TIMEOUT);
+                failed = 1;
+                break;
+            }
             // (polled relaxed: an acquire per poll would empty L1 each time)
             unsigned int v;
             asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
             if ((int)(v - target) >= 0) break;
-            if ((++tries & 63) == 0) {
-                if (*(volatile int*)status) {
-                    failed = 1;
-                    break;
-                }
-                if (tries > kLoopBarrierTries) {
-                    raise_status(status, FS_ERR_TIMEOUT);
-                    failed = 1;
-                    break;
-                }
+            if ((++tries & 63) == 0 && *(volatile int*)status) {
+                failed = 1;
+                break;
             }
         }
         asm volatile("fence.acq_rel.gpu;" ::: "memory");
@@ -1492,7 +1491,7 @@ __global__ void __launch_bounds__(kPassThreads, ONE ? kLoopOneBlocksPerSm : kLoo
             }
             const float4 ak = pressure_acc_of(c, a, prk, gbk);
             if (!half && valid) s.acc[k] = ak;
-            if (!loop_barrier(&sc->loop_arrived, ++barriers * gridDim.x, status)) return;
+            if (!loop_barrier(&sc->loop_arrived, ++barriers * gridDim.x, lt.barrier_tries, status)) return;
             // update
             float sum;
             if (tiled) {
@@ -1516,7 +1515,7 @@ __global__ void __launch_bounds__(kPassThreads, ONE ? kLoopOneBlocksPerSm : kLoo
             if (!half && valid)
                 o = iisph3d_pressure_update_tail<float>(k, s, c, dt, v3<float>(ak.x, ak.y, ak.z), sum, vsk, gbk.w, prk);
             reduce_err_parts_to(o, loop_err_set(it, sc));
-            if (!loop_barrier(&sc->loop_arrived, ++barriers * gridDim.x, status)) return;
+            if (!loop_barrier(&sc->loop_arrived, ++barriers * gridDim.x, lt.barrier_tries, status)) return;
         }
     } else {
         for (;; it++) {
@@ -1551,7 +1550,7 @@ __global__ void __launch_bounds__(kPassThreads, ONE ? kLoopOneBlocksPerSm : kLoo
                 }
                 if (!half && valid) s.acc[k] = pressure_acc_of(c, a, prk, gbk);
             }
-            if (!loop_barrier(&sc->loop_arrived, ++barriers * gridDim.x, status)) return;
+            if (!loop_barrier(&sc->loop_arrived, ++barriers * gridDim.x, lt.barrier_tries, status)) return;
             // update
             ErrPart o;
             for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -1591,7 +1590,7 @@ __global__ void __launch_bounds__(kPassThreads, ONE ? kLoopOneBlocksPerSm : kLoo
                 }
             }
             reduce_err_parts_to(o, loop_err_set(it, sc));
-            if (!loop_barrier(&sc->loop_arrived, ++barriers * gridDim.x, status)) return;
+            if (!loop_barrier(&sc->loop_arrived, ++barriers * gridDim.x, lt.barrier_tries, status)) return;
         }
     }
 }

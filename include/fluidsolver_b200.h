@@ -329,6 +329,13 @@ fs_status fs_set_tuning(fs_ctx* ctx, const fs_tuning* in);
  * limit is one per device, shared by every context on the context's device. */
 fs_status fs_set_tile_wait_limit(fs_ctx* ctx, int32_t tries);
 
+/* The same for the waits between the blocks of a launch, for this context:
+ * how many times the search's scan polls the tiles before one (the search
+ * then returns FS_ERR_TIMEOUT and leaves the state as it was), and how many
+ * times a block of the pressure loop polls a grid barrier. tries < 0 restores
+ * the default (4,194,304); 0 gives up without a poll. */
+fs_status fs_set_grid_wait_limits(fs_ctx* ctx, int32_t scan_tries, int32_t barrier_tries);
+
 /* The searches' own sort on caller keys, for tests of the sort alone: the
  * stable least-significant-digit radix sort that orders the particles by
  * (region, cell) key every search (and, in the reference-order mode, by the
