@@ -942,7 +942,7 @@ template <typename R> fs_status order_by_counting(fs_ctx* c, State<R> s) {
                (V4<R>*)c->vel[nx], (const V4<R>*)c->acc[c->cur], (V4<R>*)c->acc[nx], (const V4<R>*)c->ext[c->cur],
                (V4<R>*)c->ext[nx], (const R*)c->rho[c->cur], (R*)c->rho[nx], (const R*)c->p[c->cur], (R*)c->p[nx],
                c->type[c->cur], c->type[nx], c->hidx[c->cur], c->hidx[nx], c->scene_of[c->cur], c->scene_of[nx],
-               c->h2d_rank, c->search_state);
+               c->h2d_rank, c->search_state, c->status);
     FS_CUDA(cudaGetLastError());
     c->cur = nx;
     return FS_OK;
