@@ -1367,6 +1367,12 @@ __device__ __forceinline__ void stage_loop_field(TileStage& stg, const TileDesc*
     }
 }
 
+// A packed tile's float field came by plain stores: this thread's, before the
+// bulk copies that fill the same memory after the next block barrier.
+__device__ __forceinline__ void packed_field_fence(const TileHead& h) {
+    if (!h.slots) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
 // The test of iteration `it` from its accumulators (check_scene's, with the
 // FP64 average); thread 0 of every block calls it. When the loop ends, block 0
 // stores the results and clamps the time step; else it clears the set of
@@ -1486,6 +1492,7 @@ __global__ void __launch_bounds__(kPassThreads, ONE ? kLoopOneBlocksPerSm : kLoo
                         q.pair(at_offset(sp, off), at_offset(s1, off >> 2));
                     }, [&] { q.flush(); });
                 a = pair_total<2>(q.pa);
+                packed_field_fence(h);
             } else {
                 a = acc_sum_fallback<2, true>(L, k, half, valid, s, pk, prk, S);
             }
@@ -1546,6 +1553,7 @@ __global__ void __launch_bounds__(kPassThreads, ONE ? kLoopOneBlocksPerSm : kLoo
                     parity ^= 1u;
                     if (!ok) return;
                     a = acc_sum_tiled<kLoopAhead, 2>(T, k, cnt, half, valid, ahead, sp, s1, pk, prk, S);
+                    packed_field_fence(h);
                     __syncthreads();   // the staged fields have been read
                 }
                 if (!half && valid) s.acc[k] = pressure_acc_of(c, a, prk, gbk);
