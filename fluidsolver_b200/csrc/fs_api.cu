@@ -994,8 +994,8 @@ template <typename R> fs_status search_impl(fs_ctx* c, bool solver_lists) {
         FS_CUDA(cudaGetLastError());
         if (c->sort_lists_by_host && !group) {
             c->launches++;
-            k_sort_lists_by_host<<<grid_for(c->n_owners), kBlock, 0, st>>>(c->n_owners, c->nbr, c->nbr_stride,
-                                                                           c->nbr_capacity, c->nbr_count, s.hidx);
+            k_sort_lists_by_host<<<grid_for(c->n_owners), kBlock, 0, st>>>(
+                c->n_owners, c->nbr, c->nbr_stride, c->nbr_capacity, c->nbr_count, s.hidx, c->status);
             FS_CUDA(cudaGetLastError());
         }
         c->have_lists = true;

@@ -859,9 +859,12 @@ __device__ __forceinline__ void sort_list_by_host_at(int64_t k, uint32_t* FSB_R 
     }
 }
 static __global__ void k_sort_lists_by_host(int64_t n_owners, uint32_t* FSB_R nbr, int64_t stride, int K,
-                                     const uint32_t* FSB_R count, const uint32_t* FSB_R hidx) {
+                                            const uint32_t* FSB_R count, const uint32_t* FSB_R hidx,
+                                            const int* FSB_R status) {
     int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= n_owners) return;
+    const int err = *status;
+    if (err && err != FS_ERR_CAPACITY) return;   // k_build_lists has left the lists as they were: never written, perhaps
     sort_list_by_host_at(k, nbr, stride, K, count, hidx);
 }
 

@@ -476,7 +476,8 @@ __device__ __forceinline__ int small_search(const SmallStepArgs<R>& a, const Tea
         uint32_t* cnt = a.stage_lists ? g.cnt - lo : a.count;
         const int64_t stride = a.stage_lists ? share : a.stride;
         const int err = status_now(a.status);
-        if (!err || err == FS_ERR_CAPACITY)
+        const bool built = !err || err == FS_ERR_CAPACITY;   // (no later kernel or phase reads lists that are not)
+        if (built)
             for (int64_t k = T.first(no); k < T.end(no); k += kSmallThreads)
                 list_owner_at<R>(k, pos, type, cs, w, a.owner_mask, a.rows, nbr, stride, a.K, cnt, a.status, a.sc);
         if (!a.stage_lists) cluster_sync();
@@ -492,8 +493,9 @@ __device__ __forceinline__ int small_search(const SmallStepArgs<R>& a, const Tea
             } else if (a.stage_lists) {
                 __syncthreads();
             }
-            for (int64_t k = T.first(no); k < T.end(no); k += kSmallThreads)
-                sort_list_by_host_at(k, nbr, stride, a.K, cnt, hidx);
+            if (built)
+                for (int64_t k = T.first(no); k < T.end(no); k += kSmallThreads)
+                    sort_list_by_host_at(k, nbr, stride, a.K, cnt, hidx);
             if (!a.stage_lists) cluster_sync();
         }
         if (a.stage_lists) {
