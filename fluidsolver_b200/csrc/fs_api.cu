@@ -1602,6 +1602,7 @@ fs_status search_for_step(fs_ctx* c, float dt) {
             continue;
         }
         note_timeout(c, st);
+        c->lists_built = st == FS_OK || st == FS_ERR_CAPACITY;
         if (st != FS_OK)
             return fail((fs_status)st, st == FS_ERR_CAPACITY ? "neighbor list capacity exceeded"
                                                              : "device reported an error during the search");
@@ -2270,7 +2271,8 @@ fs_status fs_get_neighbors_csr(fs_ctx* c, int64_t* offsets, int64_t* indices, in
 fs_status fs_get_solver_lists_csr(fs_ctx* c, int64_t* offsets, int64_t* indices, int64_t* total) {
     if (!c || !offsets) return fail(FS_ERR_INVALID, "null argument");
     if (!c->have_state) return fail(FS_ERR_STATE, "no particles uploaded");
-    if (!c->have_lists) return fail(FS_ERR_STATE, "no solver lists: execute the neighborhood search first");
+    if (!c->have_lists || !c->lists_built)
+        return fail(FS_ERR_STATE, "no solver lists: execute the neighborhood search first");
     FS_CUDA(cudaSetDevice(c->device));
     const int64_t n = c->n, no = c->n_owners;
     cudaStream_t st = c->stream;

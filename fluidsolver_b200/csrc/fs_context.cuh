@@ -46,6 +46,7 @@ struct fs_ctx {
     int64_t n_struct = 0;     // particles that take part in the cell structure
     bool have_state = false;
     bool have_lists = false;
+    bool lists_built = true;        // by the last search that the host waited for (not one that a NaN ended)
     bool have_cells = false;        // cell tables describe the current sorted order
     float searched_dt = 0.f;
     bool reference_order = false;
