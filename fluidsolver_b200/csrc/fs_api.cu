@@ -1642,6 +1642,7 @@ fs_status solve_graph(fs_ctx* c, float dt, bool with_search = false) {
             c->rho[0] = g.post_rho0;
             c->rho[1] = g.post_rho1;
             c->rho_prev = g.post_rho_prev;
+            if (with_search) c->have_cells = true;   // as the capture noted
             return FS_OK;
         }
     }
