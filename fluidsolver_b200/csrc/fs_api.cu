@@ -440,7 +440,7 @@ fs_status ensure_cells(fs_ctx* c, int64_t cells) {
         c->cell_start = c->cell_partials = nullptr;
         c->look_tiles = nullptr;
         c->cell_alloc = 0;
-        c->have_cells = false;
+        c->have_cells = c->have_table = false;
         FS_TRY(dalloc(&c->cell_start, (size_t)3 * need + 4));   // the counting path's extra entry, whole uint4
         FS_TRY(dalloc(&c->cell_partials, (size_t)scan_tiles(3 * need)));
         FS_TRY(dalloc(&c->look_tiles, (size_t)look_tiles(3 * need + 1)));
@@ -799,7 +799,7 @@ template <typename R> fs_status compact_search_impl(fs_ctx* c, State<R> s, bool 
         FS_CUDA(cudaGetLastError());
         c->have_lists = true;
     }
-    c->have_cells = true;
+    c->have_cells = c->have_table = true;
     return FS_OK;
 }
 
@@ -953,7 +953,7 @@ template <typename R> fs_status search_impl(fs_ctx* c, bool solver_lists) {
     cudaStream_t st = c->stream;
     if (n == 0) {
         c->have_lists = solver_lists;
-        c->have_cells = true;
+        c->have_cells = c->have_table = true;
         return FS_OK;
     }
     State<R> s = state_of<R>(c);
@@ -1000,7 +1000,7 @@ template <typename R> fs_status search_impl(fs_ctx* c, bool solver_lists) {
         }
         c->have_lists = true;
     }
-    c->have_cells = true;
+    c->have_cells = c->have_table = true;
     return FS_OK;
 }
 
@@ -1030,7 +1030,7 @@ fs_status read_back(fs_ctx* c, bool scalars, int* st = nullptr) {
 void note_timeout(fs_ctx* c, int st) {
     SearchState h{};
     if (st != FS_ERR_TIMEOUT || cudaMemcpy(&h, c->search_state, sizeof(h), cudaMemcpyDeviceToHost) != cudaSuccess) return;
-    if (h.scan_failed) c->have_cells = c->have_lists = false;
+    if (h.scan_failed) c->have_cells = c->have_table = c->have_lists = false;
 }
 
 // Phase timestamp i of the host-driven path. In a captured step the kernels
@@ -1642,7 +1642,7 @@ fs_status solve_graph(fs_ctx* c, float dt, bool with_search = false) {
             c->rho[0] = g.post_rho0;
             c->rho[1] = g.post_rho1;
             c->rho_prev = g.post_rho_prev;
-            if (with_search) c->have_cells = true;   // as the capture noted
+            if (with_search) c->have_cells = c->have_table = true;   // as the capture noted
             return FS_OK;
         }
     }
@@ -1818,7 +1818,10 @@ fs_status enqueue_steps(fs_ctx* c, int32_t steps, float dt) {
     FS_CUDA(cudaMemsetAsync(c->status, 0, sizeof(int), c->stream));
     c->small_last = small_eligible(c);
     if (c->small_last) {
-        if (steps > 0) FS_TRY(enqueue_small_steps(c, steps, dt));
+        if (steps > 0) {
+            FS_TRY(enqueue_small_steps(c, steps, dt));
+            c->have_table = true;
+        }
     } else {
         for (int32_t i = 0; i < steps; i++) FS_TRY(solve_graph(c, dt, true));
     }
@@ -2114,7 +2117,7 @@ fs_status fs_upload(fs_ctx* c, const fs_particles* in) {
     }
     c->have_state = true;
     c->have_lists = false;
-    c->have_cells = false;
+    c->have_cells = c->have_table = false;
     ending.all = c->scenes > 0;   // (the packing may still run; a batch's grids are copied behind it)
     return FS_OK;
 }
@@ -2157,6 +2160,8 @@ fs_status fs_get_neighbors_csr(fs_ctx* c, int64_t* offsets, int64_t* indices, in
         if (total) *total = 0;
         return FS_OK;
     }
+    // (the walk follows the cell tables, which hold another upload's particles or nothing yet)
+    if (!c->have_table) return fail(FS_ERR_STATE, "execute the neighborhood search first");
     // the counts, the longest list after them, and the 64-bit offsets with their scan's tile totals
     if (c->csr_capacity < n + 1) {
         if (c->csr_offsets) cudaFree(c->csr_offsets);

@@ -48,6 +48,7 @@ struct fs_ctx {
     bool have_lists = false;
     bool lists_built = true;        // by the last search that the host waited for (not one that a NaN ended)
     bool have_cells = false;        // cell tables describe the current sorted order
+    bool have_table = false;        // a search since the upload has filled the cell tables (the small-scene kernel's too)
     float searched_dt = 0.f;
     bool reference_order = false;
     bool include_inactive = false;  // contract lists inactive particles (2D quadratic / hashed)

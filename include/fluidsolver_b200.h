@@ -212,7 +212,8 @@ fs_status fs_download(fs_ctx* ctx, fs_particles* out);
 /* Neighborhood search on the current positions (find_neighbors). */
 fs_status fs_find_neighbors(fs_ctx* ctx);
 /* Neighbor lists of the last search in host-index space, each list ascending:
- * offsets has n+1 entries; indices may be NULL to query *total first. */
+ * offsets has n+1 entries; indices may be NULL to query *total first. Needs a
+ * search (or a step) since the last upload, FS_ERR_STATE otherwise. */
 fs_status fs_get_neighbors_csr(fs_ctx* ctx, int64_t* offsets, int64_t* indices, int64_t* total);
 /* The lists that the solver's passes walk (3D IISPH fast mode: the tile lists),
  * exported like fs_get_neighbors_csr: host-index space, each list ascending,
