@@ -34,11 +34,14 @@ fs_status fail(fs_status s, const std::string& msg) {
     return s;
 }
 
+// (a failed call's error is taken back, or the next launch's check would find it)
 #define FS_CUDA(call)                                                                              \
     do {                                                                                           \
         cudaError_t e_ = (call);                                                                   \
-        if (e_ != cudaSuccess)                                                                     \
+        if (e_ != cudaSuccess) {                                                                   \
+            (void)cudaGetLastError();                                                              \
             return fail(FS_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));          \
+        }                                                                                          \
     } while (0)
 
 #define FS_TRY(call)                       \
@@ -314,6 +317,8 @@ fs_status ensure_staging(fs_ctx* c, size_t bytes) {
 }
 
 constexpr size_t kGradientBytes = size_t(6) << 30;        // stored gradients at most
+// Lists of (at least) K entries. Where the allocation of larger ones fails, the
+// context has none, and the next search allocates those of the old capacity.
 fs_status ensure_lists(fs_ctx* c, int K) {
     const int64_t stride = ((c->cap + 31) / 32) * 32;
     const bool tiled = tiled_mode(c);
@@ -447,6 +452,12 @@ fs_status ensure_cells(fs_ctx* c, int64_t cells) {
         c->cell_alloc = need;
     }
     return FS_OK;
+}
+
+// what a search writes to, where an earlier allocation of it failed
+fs_status ensure_tables(fs_ctx* c) {
+    FS_TRY(ensure_cells(c, c->cells));
+    return ensure_lists(c, c->nbr_capacity);
 }
 
 // ---------------------------------------------------------------------------
@@ -1583,7 +1594,7 @@ fs_status fill_stats(fs_ctx* c, fs_step_stats* stats, int st, int entries = 1) {
 // capacity the lists are grown and the search is repeated once.
 // Phase timestamps 0 and 1 are its begin and end.
 fs_status search_for_step(fs_ctx* c, float dt) {
-    FS_TRY(ensure_cells(c, c->cells));
+    FS_TRY(ensure_tables(c));
     for (int attempt = 0; attempt < 3; attempt++) {
         c->launches++;
         k_step_begin<<<grid_for(c->nsc(), 128), 128, 0, c->stream>>>(c->scalars, c->nsc(), dt, false);
@@ -1814,7 +1825,7 @@ fs_status enqueue_small_steps(fs_ctx* c, int32_t steps, float dt) {
 }
 
 fs_status enqueue_steps(fs_ctx* c, int32_t steps, float dt) {
-    FS_TRY(ensure_cells(c, c->cells));
+    FS_TRY(ensure_tables(c));
     FS_CUDA(cudaMemsetAsync(c->status, 0, sizeof(int), c->stream));
     c->small_last = small_eligible(c);
     if (c->small_last) {
