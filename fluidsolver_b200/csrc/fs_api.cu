@@ -316,7 +316,29 @@ fs_status ensure_staging(fs_ctx* c, size_t bytes) {
     return FS_OK;
 }
 
-constexpr size_t kGradientBytes = size_t(6) << 30;        // stored gradients at most
+// The stored gradients of the IISPH gather phases (fs_cached.cuh), by the lists'
+// capacity: up to kGradientBytes, and as a convenience only (without them the
+// phases evaluate the kernel). In 2D only the passes with eight threads per owner
+// read them, which depends on the uploaded particles unless the context holds too
+// few for the others.
+constexpr size_t kGradientBytes = size_t(6) << 30;
+constexpr int64_t kGrouped2D = 32768;   // 2D IISPH: fluid particles up to which eight threads take an owner (grouped)
+bool grouped(const fs_ctx* c);
+bool uses_gradients(const fs_ctx* c) {
+    if (c->prm.solver == FS_SOLVER_IISPH_3D) return !tiled_mode(c);
+    return c->prm.solver == FS_SOLVER_IISPH_2D && (c->have_state || c->cap <= kGrouped2D) && grouped(c);
+}
+void ensure_gradients(fs_ctx* c) {
+    const size_t bytes = (size_t)c->nbr_capacity * c->nbr_stride * 4 * c->real_size;
+    if (c->gradients || !c->nbr || !uses_gradients(c) || bytes > kGradientBytes) return;
+    if (cudaMalloc(&c->gradients, bytes) != cudaSuccess) {
+        (void)cudaGetLastError();
+        c->gradients = nullptr;
+        return;
+    }
+    clear_graphs(c);   // captured without them
+}
+
 // Lists of (at least) K entries. Where the allocation of larger ones fails, the
 // context has none, and the next search allocates those of the old capacity.
 fs_status ensure_lists(fs_ctx* c, int K) {
@@ -343,17 +365,9 @@ fs_status ensure_lists(fs_ctx* c, int K) {
         FS_TRY(dalloc(&c->tile_ent, (size_t)(K / 8) * c->tile_stride));
         FS_CUDA(set_tile_smem(K));
     }
-    // stored gradients of the IISPH gather phases (fs_cached.cuh): up to
-    // kGradientBytes, and as a convenience only (without them the phases
-    // evaluate the kernel)
-    const size_t grad = (size_t)K * stride * 4 * c->real_size;
-    const bool iisph = c->prm.solver == FS_SOLVER_IISPH_3D || c->prm.solver == FS_SOLVER_IISPH_2D;
-    if (!tiled && iisph && grad <= kGradientBytes && cudaMalloc(&c->gradients, grad) != cudaSuccess) {
-        (void)cudaGetLastError();
-        c->gradients = nullptr;
-    }
     c->nbr_capacity = K;
     c->nbr_stride = stride;
+    ensure_gradients(c);
     return FS_OK;
 }
 
@@ -1305,7 +1319,7 @@ fs_status step_iisph3d_tiled(fs_ctx* c, bool capture) {
 // 40,000; the 3D first loop 66 -> 21 at 8,000, 76 -> 51 at 50,700 (FP64 78 -> 86).
 bool grouped(const fs_ctx* c) {
     switch (c->prm.solver) {
-        case FS_SOLVER_IISPH_2D: return c->n_fluid <= 32768;
+        case FS_SOLVER_IISPH_2D: return c->n_fluid <= kGrouped2D;
         case FS_SOLVER_IISPH_3D: return c->n_fluid <= (c->precision == FS_PRECISION_FP64 ? 45056 : 65536);
         default: return c->n_fluid <= 65536;
     }
@@ -1317,7 +1331,7 @@ bool grouped(const fs_ctx* c) {
 // 100,000. In 2D (one thread per owner evaluates) 40 -> 18 at 2,500, 42 -> 39 at
 // 25,600, 43 -> 49 at 40,000.
 bool grouped_pressure(const fs_ctx* c) {
-    return c->n_fluid <= (c->prm.solver == FS_SOLVER_IISPH_2D ? 32768 : (c->gradients ? 20480 : 45056));
+    return c->n_fluid <= (c->prm.solver == FS_SOLVER_IISPH_2D ? kGrouped2D : (c->gradients ? 20480 : 45056));
 }
 
 template <typename R, bool KAHAN> fs_status step_iisph3d(fs_ctx* c, bool capture) {
@@ -2129,6 +2143,7 @@ fs_status fs_upload(fs_ctx* c, const fs_particles* in) {
     c->have_state = true;
     c->have_lists = false;
     c->have_cells = c->have_table = false;
+    ensure_gradients(c);
     ending.all = c->scenes > 0;   // (the packing may still run; a batch's grids are copied behind it)
     return FS_OK;
 }
