@@ -64,6 +64,14 @@ template <typename T> fs_status dalloc(T** p, size_t count) {
     return FS_OK;
 }
 
+// For a context that may hold stored gradients, which it can do without: they
+// make room for an allocation that fails.
+bool drop_gradients(fs_ctx* c);
+template <typename T> fs_status dalloc(fs_ctx* c, T** p, size_t count) {
+    const fs_status s = dalloc(p, count);
+    return s != FS_OK && drop_gradients(c) ? dalloc(p, count) : s;
+}
+
 // host-side replicas of the reference's float constants
 float kernel_alpha(int dim, float h) {
     const float pi = 3.14159265358979323846f;
@@ -311,14 +319,14 @@ fs_status ensure_staging(fs_ctx* c, size_t bytes) {
     if (c->staging) cudaFree(c->staging);
     c->staging = nullptr;
     c->staging_bytes = 0;
-    FS_CUDA(cudaMalloc(&c->staging, bytes));
+    FS_TRY(dalloc(c, (char**)&c->staging, bytes));
     c->staging_bytes = bytes;
     return FS_OK;
 }
 
 // The stored gradients of the IISPH gather phases (fs_cached.cuh), by the lists'
-// capacity: up to kGradientBytes, and as a convenience only (without them the
-// phases evaluate the kernel). In 2D only the passes with eight threads per owner
+// capacity: up to kGradientBytes and a quarter of the memory that is free, and
+// as a convenience only (without them the phases evaluate the kernel). In 2D only the passes with eight threads per owner
 // read them, which depends on the uploaded particles unless the context holds too
 // few for the others.
 constexpr size_t kGradientBytes = size_t(6) << 30;
@@ -330,13 +338,26 @@ bool uses_gradients(const fs_ctx* c) {
 }
 void ensure_gradients(fs_ctx* c) {
     const size_t bytes = (size_t)c->nbr_capacity * c->nbr_stride * 4 * c->real_size;
-    if (c->gradients || !c->nbr || !uses_gradients(c) || bytes > kGradientBytes) return;
-    if (cudaMalloc(&c->gradients, bytes) != cudaSuccess) {
+    if (c->gradients || c->no_gradients || !c->nbr || !uses_gradients(c)) return;
+    size_t unused = 0, all = 0;
+    if (bytes > kGradientBytes || cudaMemGetInfo(&unused, &all) != cudaSuccess || bytes > unused / 4 ||
+        cudaMalloc(&c->gradients, bytes) != cudaSuccess) {
         (void)cudaGetLastError();
         c->gradients = nullptr;
+        c->no_gradients = true;
         return;
     }
     clear_graphs(c);   // captured without them
+}
+// (they hold nothing between two steps)
+bool drop_gradients(fs_ctx* c) {
+    if (!c->gradients) return false;
+    (void)cudaStreamSynchronize(c->stream);
+    clear_graphs(c);
+    cudaFree(c->gradients);
+    c->gradients = nullptr;
+    c->no_gradients = true;
+    return true;
 }
 
 // Lists of (at least) K entries. Where the allocation of larger ones fails, the
@@ -354,15 +375,16 @@ fs_status ensure_lists(fs_ctx* c, int K) {
     if (c->tile_desc) cudaFree(c->tile_desc);
     if (c->gradients) cudaFree(c->gradients);
     c->gradients = nullptr;
+    c->no_gradients = false;
     c->nbr = nullptr;
     c->tile_ent = nullptr;
     c->tile_desc = nullptr;
-    FS_TRY(dalloc(&c->nbr, (size_t)K * stride));
+    FS_TRY(dalloc(c, &c->nbr, (size_t)K * stride));
     if (tiled) {
         const int64_t tiles = (c->cap + kTileOwners - 1) / kTileOwners;
         c->tile_stride = tiles * kTileOwners;
-        FS_TRY(dalloc(&c->tile_desc, (size_t)tiles));
-        FS_TRY(dalloc(&c->tile_ent, (size_t)(K / 8) * c->tile_stride));
+        FS_TRY(dalloc(c, &c->tile_desc, (size_t)tiles));
+        FS_TRY(dalloc(c, &c->tile_ent, (size_t)(K / 8) * c->tile_stride));
         FS_CUDA(set_tile_smem(K));
     }
     c->nbr_capacity = K;
@@ -460,9 +482,9 @@ fs_status ensure_cells(fs_ctx* c, int64_t cells) {
         c->look_tiles = nullptr;
         c->cell_alloc = 0;
         c->have_cells = c->have_table = false;
-        FS_TRY(dalloc(&c->cell_start, (size_t)3 * need + 4));   // the counting path's extra entry, whole uint4
-        FS_TRY(dalloc(&c->cell_partials, (size_t)scan_tiles(3 * need)));
-        FS_TRY(dalloc(&c->look_tiles, (size_t)look_tiles(3 * need + 1)));
+        FS_TRY(dalloc(c, &c->cell_start, (size_t)3 * need + 4));   // the counting path's extra entry, whole uint4
+        FS_TRY(dalloc(c, &c->cell_partials, (size_t)scan_tiles(3 * need)));
+        FS_TRY(dalloc(c, &c->look_tiles, (size_t)look_tiles(3 * need + 1)));
         c->cell_alloc = need;
     }
     return FS_OK;
@@ -2195,8 +2217,8 @@ fs_status fs_get_neighbors_csr(fs_ctx* c, int64_t* offsets, int64_t* indices, in
         c->csr_offsets = nullptr;
         c->csr_counts = nullptr;
         c->csr_capacity = 0;
-        FS_TRY(dalloc(&c->csr_offsets, (size_t)(n + 1 + csr_scan_tiles(n + 1))));
-        FS_TRY(dalloc(&c->csr_counts, (size_t)n + 2));
+        FS_TRY(dalloc(c, &c->csr_offsets, (size_t)(n + 1 + csr_scan_tiles(n + 1))));
+        FS_TRY(dalloc(c, &c->csr_counts, (size_t)n + 2));
         c->csr_capacity = n + 1;
     }
     const WalkParams w = walk_of(c, false);
@@ -2246,7 +2268,7 @@ fs_status fs_get_neighbors_csr(fs_ctx* c, int64_t* offsets, int64_t* indices, in
         if (c->csr_members) cudaFree(c->csr_members);
         c->csr_members = members = nullptr;
         c->csr_members_capacity = 0;
-        FS_TRY(dalloc(&members, (size_t)tot));
+        FS_TRY(dalloc(c, &members, (size_t)tot));
         if (tot <= kCsrKeep) {
             c->csr_members = members;
             c->csr_members_capacity = tot;
@@ -2258,7 +2280,7 @@ fs_status fs_get_neighbors_csr(fs_ctx* c, int64_t* offsets, int64_t* indices, in
         if (c->csr_sorted) cudaFree(c->csr_sorted);
         c->csr_sorted = sorted = nullptr;
         c->csr_sorted_capacity = 0;
-        FS_TRY(dalloc(&sorted, (size_t)chunk));
+        FS_TRY(dalloc(c, &sorted, (size_t)chunk));
         if (chunk <= kCsrKeep) {
             c->csr_sorted = sorted;
             c->csr_sorted_capacity = chunk;
@@ -2320,7 +2342,7 @@ fs_status fs_get_solver_lists_csr(fs_ctx* c, int64_t* offsets, int64_t* indices,
         if (d_idx) cudaFree(d_idx);
     };
     if (no > 0) {
-        if (dalloc(&d_counts, (size_t)no) != FS_OK || dalloc(&d_off, (size_t)no + 1) != FS_OK) {
+        if (dalloc(c, &d_counts, (size_t)no) != FS_OK || dalloc(c, &d_off, (size_t)no + 1) != FS_OK) {
             release();
             return fail(FS_ERR_CUDA, "allocation for the list export failed");
         }
@@ -2353,7 +2375,7 @@ fs_status fs_get_solver_lists_csr(fs_ctx* c, int64_t* offsets, int64_t* indices,
         return FS_OK;
     }
     std::vector<uint32_t> idx((size_t)tot);
-    if (dalloc(&d_idx, (size_t)tot) != FS_OK ||
+    if (dalloc(c, &d_idx, (size_t)tot) != FS_OK ||
         cudaMemcpyAsync(d_off, off_sorted.data(), sizeof(int64_t) * (no + 1), cudaMemcpyHostToDevice, st) !=
             cudaSuccess) {
         release();
@@ -2431,10 +2453,8 @@ fs_status fs_global_statistics(fs_ctx* c, float zero_height, fs_global_stats* ou
     if (!c || !out) return fail(FS_ERR_INVALID, "null argument");
     if (!c->have_state) return fail(FS_ERR_STATE, "no particles uploaded");
     FS_CUDA(cudaSetDevice(c->device));
-    if (!c->stats_parts) {
-        FS_TRY(dalloc(&c->stats_parts, (size_t)kStatsBlocks));
-        FS_TRY(dalloc(&c->stats_out, (size_t)1));
-    }
+    if (!c->stats_parts) FS_TRY(dalloc(c, &c->stats_parts, (size_t)kStatsBlocks));
+    if (!c->stats_out) FS_TRY(dalloc(c, &c->stats_out, (size_t)1));
     const int blocks = (int)std::min<int64_t>(kStatsBlocks, std::max<int64_t>(1, (c->n + kStatsThreads - 1) / kStatsThreads));
     c->launches += 2;
     if (c->precision == FS_PRECISION_FP64)
@@ -2573,8 +2593,8 @@ fs_status fs_query_position(fs_ctx* c, const float* position, int64_t* out, int6
     uint32_t* d_out = nullptr;
     unsigned long long* d_cnt = nullptr;
     const int64_t room = std::max<int64_t>(cap, 0);
-    FS_TRY(dalloc(&d_out, (size_t)std::max<int64_t>(room, 1)));
-    if (dalloc(&d_cnt, 1) != FS_OK) {
+    FS_TRY(dalloc(c, &d_out, (size_t)std::max<int64_t>(room, 1)));
+    if (dalloc(c, &d_cnt, 1) != FS_OK) {
         cudaFree(d_out);
         return FS_ERR_CUDA;
     }
@@ -2989,8 +3009,8 @@ fs_status fs_trace_rays(fs_ctx* c, float surface_fraction, int64_t n, const floa
     if (n == 0) return FS_OK;
     float *d_in = nullptr, *d_out = nullptr;
     int32_t* d_hit = nullptr;
-    FS_TRY(dalloc(&d_in, (size_t)n * 6));
-    if (dalloc(&d_out, (size_t)n * 7) != FS_OK || dalloc(&d_hit, (size_t)n) != FS_OK) {
+    FS_TRY(dalloc(c, &d_in, (size_t)n * 6));
+    if (dalloc(c, &d_out, (size_t)n * 7) != FS_OK || dalloc(c, &d_hit, (size_t)n) != FS_OK) {
         cudaFree(d_in);
         cudaFree(d_out);
         return fail(FS_ERR_CUDA, "allocation for the rays failed");
@@ -3112,7 +3132,7 @@ fs_status fs_render(fs_ctx* c, const fs_camera* cam, const fs_render_settings* r
     sh.seed = r->seed;
     const int64_t np = (int64_t)cam->width * cam->height;
     float* d_rad = nullptr;
-    FS_TRY(dalloc(&d_rad, (size_t)np * 3));
+    FS_TRY(dalloc(c, &d_rad, (size_t)np * 3));
     c->launches++;
     if (c->precision == FS_PRECISION_FP64)
         k_render<double><<<grid_for(np, kRayWarps), 32 * kRayWarps, 0, c->stream>>>(state_of<double>(c), c->cell_start, rs, rc, sh, d_rad);

@@ -115,6 +115,7 @@ struct fs_ctx {
     std::vector<fsb::SceneGrid> grids_host;     // dims and bases
     uint32_t* nbr = nullptr;       // solver lists, slot-major: nbr[s * nbr_stride + k]
     void* gradients = nullptr;     // V4 [K][nbr_stride]: gradW and mass of every list entry (fs_cached.cuh), or null
+    bool no_gradients = false;     // their memory was refused, or given back for something else
     fsb::TileDesc* tile_desc = nullptr;  // tile lists (3D IISPH fast path): per tile of owners
     uint4* tile_ent = nullptr;           // [K / 8][tile_stride] octets of 16-bit entries
     int64_t tile_stride = 0;             // owners per octet plane (tiles * kTileOwners)

@@ -1,11 +1,13 @@
-"""Memory of the stored kernel gradients: 2D IISPH contexts whose passes do not
-read them (more than 32,768 fluid particles) hold none. Measured against a SESPH
-context of the same size, which has the same buffers otherwise."""
+"""Memory of the stored kernel gradients, which a context can do without. 2D
+IISPH contexts whose passes do not read them (more than 32,768 fluid particles)
+hold none, measured against a SESPH context of the same size, which has the
+same buffers otherwise. And an allocation that fails takes their place."""
 import numpy as np
 import pytest
 
 from conftest import bits_equal
 from fluidsolver_b200.solver import ParticleCollection
+from test_gpu_pressure_loop import dam
 from test_gpu_solvers import make_solver
 
 pytestmark = pytest.mark.gpu
@@ -68,3 +70,33 @@ def test_uploads_on_both_sides_of_the_line():
             assert bits_equal(getattr(x, f), getattr(y, f)), (fluid, f)
         own.close()
     kept.close()
+
+
+def test_they_make_room_for_what_a_call_cannot_do_without():
+    """With 60 MB left on the device, two million rays (112 MB) take the place of the stored gradients
+    of a bit-exact scene (130 MB); the steps go on without them, to the same state."""
+    make = lambda: make_solver("iisph-3d", "hashed-3d", [0.001, 2, 9, 0.5, 0.7, 0.01, 1.0, 1.1],  # noqa: E731
+                               (0.005, 0.4, 0.25), precision="fp32", reference_order=True)
+    s, other = make(), make()
+    s.data.collection = other.data.collection = dam(100000, 5)
+    s.run(2)
+    other.run(2)
+    rays = np.zeros((2_000_000, 3), np.float32)
+    rays[:, 1] = -1.0   # downwards from above the scene's corner, beside it
+    origins = np.full_like(rays, 1000.0)
+    torch.cuda.synchronize()
+    crowd = torch.empty(torch.cuda.mem_get_info()[0] - 60 * MB, dtype=torch.uint8, device="cuda")
+    try:
+        hits = s.trace_rays(origins, rays)
+        s.run(2)
+    finally:
+        del crowd
+        torch.cuda.empty_cache()
+    assert (hits["hit"] == -1).all()
+    other.trace_rays(origins[:1], rays[:1])   # (its search reorders too)
+    other.run(2)
+    x, y = s.collection(), other.collection()
+    for f in ("position", "velocity", "density", "pressure"):
+        assert bits_equal(getattr(x, f), getattr(y, f)), f
+    s.close()
+    other.close()
