@@ -59,11 +59,7 @@ __global__ void __launch_bounds__(128) k_cached_iisph3d_l1(int64_t n, State<R> s
                                                            const int* FSB_R status) {
     phase_begins(s.phase_at, 1);
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (*status) {
-        if (!SPLIT) carry_density(k, n, s);   // (SPLIT: the density pass has)
-        return;
-    }
-    if (k >= n) return;
+    if (k >= n || *status) return;
     iisph3d_l1_one<R, KAHAN, SPLIT>(k, s, L, c, (R)sc->dt, [&](uint32_t q, const V3<R>& g, const V4<R>& pj) {
         G.g[(int64_t)q * L.stride + k] = v4<R>(g, pj.w);
     });

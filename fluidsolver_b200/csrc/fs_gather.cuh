@@ -201,8 +201,8 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph_density(int64_t n
                                                                        SolverConsts<R> c, const int* FSB_R status) {
     phase_begins(s.phase_at, 1);
     __shared__ GroupRows<R, 1> rows[kGroupsPerBlock];
+    if (*status) return;
     const int64_t k = group_owner();
-    if (*status) return carry_density(k, n, s);   // (every lane of a group alike)
     const bool in = k < n, fluid = in && s.type[k] == FS_TYPE_NORMAL;
     const int64_t kk = in ? k : 0;
     const R r = group_density<R, KAHAN, GAMMA>(kk, fluid ? L.size(kk) : 0u, xyz<R>(s.pos[kk]), s, L, c,
@@ -266,11 +266,8 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph_l1(int64_t n, Sta
     phase_begins(s.phase_at, 1);
     __shared__ GroupRows<R, 3> rows3[kGroupsPerBlock];
     __shared__ GroupRows<R, 1> rows1[SPLIT ? 1 : kGroupsPerBlock];
+    if (*status) return;
     const int64_t k = group_owner();
-    if (*status) {
-        if (!SPLIT) carry_density(k, n, s);   // (SPLIT: the density pass has)
-        return;
-    }
     const bool in = k < n;
     const uint8_t ty = in ? s.type[k] : (uint8_t)FS_TYPE_INACTIVE;
     const bool fluid = ty == FS_TYPE_NORMAL;

@@ -653,9 +653,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_steps(SmallStepArgs<
                 for (int64_t k = T.first(no); k < T.end(no); k += kSmallThreads) f(k);
                 for (int64_t k = no + T.first(n - no); k < no + T.end(n - no); k += kSmallThreads) f(k);
             };
-            if (!ok1) {
-                all_particles([&](int64_t k) { carry_density(k, n, s); });
-            } else if (a.split) {
+            if (ok1 && a.split) {
                 all_particles([&](int64_t k) {
                     if (two_d) iisph2d_density_at<R, KAHAN>(k, v, Lv, a.c);
                     else iisph3d_density_at<R, KAHAN>(k, v, Lv, a.c);
@@ -767,11 +765,12 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_steps(SmallStepArgs<
                     cfl_one(sc, a.particle_size, a.cfl_timestep, a.lambda_v, a.lambda_a);
                 cluster_sync();
             }
-            if (!status_now(a.status))
-                for (int64_t k = T.first(n); k < T.end(n); k += kSmallThreads) {
-                    if (two_d) iisph2d_integrate_at<R>(k, s, sc);
-                    else iisph3d_integrate_at<R>(k, s, sc);
-                }
+            const bool ended = status_now(a.status);
+            for (int64_t k = T.first(n); k < T.end(n); k += kSmallThreads) {
+                if (ended) end_without_step<R>(k, s);
+                else if (two_d) iisph2d_integrate_at<R>(k, s, sc);
+                else iisph3d_integrate_at<R>(k, s, sc);
+            }
             cluster_sync();
         }
         stamp(T, a.stamps, 5);

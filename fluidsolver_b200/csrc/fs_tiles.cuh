@@ -889,8 +889,8 @@ __global__ void __launch_bounds__(kPassThreads, kL1GlobalEntries ? 4 : 3) k_tile
     phase_begins(s.phase_at, 1);
     extern __shared__ float4 tile_smem[];
     if (blockIdx.x >= n_tiles) {
+        if (*status) return;
         const int64_t k = n_fluid + (blockIdx.x - n_tiles) * (int64_t)kPassThreads + threadIdx.x;
-        if (*status) return carry_density(k, n, s);
         if (k < n) iisph3d_l1_one<float, true, false>(k, s, L, c, sc[s.scene_of(k)].dt);
         return;
     }
@@ -901,7 +901,7 @@ __global__ void __launch_bounds__(kPassThreads, kL1GlobalEntries ? 4 : 3) k_tile
     const int err = *status;
     const TileHead h = load_head(d);
     const TileRange rg = load_range(d, threadIdx.x);
-    if (__syncthreads_or(err)) return carry_density(k, n_fluid, s);   // one decision for the whole block
+    if (__syncthreads_or(err)) return;   // one decision for the whole block
     // owners past n_fluid (last tile) walk no entries but take part in the shuffles
     const bool valid = k < n_fluid;
     const int64_t kk = valid ? k : 0;
@@ -948,7 +948,7 @@ __global__ void __launch_bounds__(kPassThreads, kL1GlobalEntries ? 4 : 3) k_tile
         const uint32_t cnt = kL1GlobalEntries ? T.count[kk] : 0u;
         uint2 ahead[AHEAD];
         prefetch_tile_list<kL1GlobalEntries>(T, h, k, half, ahead);
-        if (!stage_tile_wait(stg, status)) return carry_density(k, n_fluid, s);
+        if (!stage_tile_wait(stg, status)) return;
         if (valid)
             walk_tile_list<kL1GlobalEntries, false, AHEAD>(T, slab, k, cnt, half, ahead, [&](uint32_t off, bool bnd) {
                 pair(at_offset(sp, off), at_offset(sv, off), at_offset(sr, off >> 2), bnd);

@@ -324,7 +324,7 @@ fs_status fs_set_tuning(fs_ctx* ctx, const fs_tuning* in);
 /* Test hook for the bounded waits: how many times the tile passes try the
  * wait for a tile's staged copies before they give up with FS_ERR_TIMEOUT
  * (the step then returns it and leaves the state as the last finished phase
- * left it). No reference counterpart: it exists so that the error path of a
+ * left it, the IISPH solvers' densities as they were before the step). No reference counterpart: it exists so that the error path of a
  * wait that runs out can be exercised on a GPU without faulting it. tries < 0
  * restores the default (65,536); 0 makes every wait give up at once. The
  * limit is one per device, shared by every context on the context's device. */
