@@ -3021,14 +3021,17 @@ fs_status fs_trace_rays(fs_ctx* c, float surface_fraction, int64_t n, const floa
         e = cudaMemcpyAsync(d_in + 3 * n, directions, sizeof(float) * 3 * n, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) {
         c->launches++;
+        auto trace = [&](auto* kernel, unsigned grid, unsigned block, const auto& state) {
+            kernel<<<grid, block, 0, st>>>(n, d_in, d_in + 3 * n, state, c->cell_start, rs, d_hit, d_out, d_out + 3 * n,
+                                           d_out + 6 * n);
+        };
+        const bool many = n > kManyRays;
+        const unsigned grid = many ? grid_for(n, kRayThreads) : grid_for(n, kRayWarps);
+        const unsigned block = many ? kRayThreads : 32 * kRayWarps;
         if (c->precision == FS_PRECISION_FP64)
-            k_trace_rays<double><<<grid_for(n, kRayWarps), 32 * kRayWarps, 0, st>>>(n, d_in, d_in + 3 * n, state_of<double>(c),
-                                                                 c->cell_start, rs, d_hit, d_out, d_out + 3 * n,
-                                                                 d_out + 6 * n);
+            trace(many ? k_trace_many_rays<double> : k_trace_rays<double>, grid, block, state_of<double>(c));
         else
-            k_trace_rays<float><<<grid_for(n, kRayWarps), 32 * kRayWarps, 0, st>>>(n, d_in, d_in + 3 * n, state_of<float>(c),
-                                                                c->cell_start, rs, d_hit, d_out, d_out + 3 * n,
-                                                                d_out + 6 * n);
+            trace(many ? k_trace_many_rays<float> : k_trace_rays<float>, grid, block, state_of<float>(c));
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(hit, d_hit, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, st);
