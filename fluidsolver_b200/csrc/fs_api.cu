@@ -180,9 +180,9 @@ Lists lists_of(fs_ctx* c) {
 // with a block per tile). A dam's tiles have 1,400 candidates on average, and
 // the 5-10 % of them above kTileCap, which fall back to 32-bit lists, are
 // the slowest blocks of every pass. B200, a pressure iteration with 1,536 and
-// with 2,048: 8,000 fluid particles 13.5 and 11.9 us, 100,000 34.7 and 28.9,
-// 165,000 47.1 and 40.6; but 60,800 (475 tiles, two rounds of 444 blocks
-// instead of one of 592) 21.5 and 27.1, 512,000 110.6 and 115.5.
+// with 2,048: 8,000 fluid particles 13.7 and 12.5 us, 29,791 14.8 and 13.4, 100,000
+// 32.5 and 26.9, 166,375 44.7 and 38.7; but 60,800 (475 tiles, two rounds of 444
+// blocks instead of one of 592) 20.9 and 26.3, 512,000 102.3 and 103.7.
 int tile_cap_of(const fs_ctx* c) {
     if (c->tuning.cap > 0) return c->tuning.cap;
     // (SESPH has no iterations to gain from it, and its pressure is the
@@ -196,9 +196,9 @@ int tile_cap_of(const fs_ctx* c) {
 
 // Whether the tile lists are spread over the shared-memory banks (k_build_tiles):
 // IISPH scenes whose pressure passes take more than one round of resident
-// blocks. Below, a pass is a chain of latencies: an iteration took 12.8 us at
-// 8,000 particles and 21.9 at 60,800 with and without it (13.3 and 13.0 at
-// 29,791); 28.9 and 26.6 at 100,000.
+// blocks. Below, a pass is a chain of latencies: an iteration took the same with
+// and without it at 8,000 particles and at 60,800 (13.3 and 13.0 us at 29,791);
+// 28.9 without and 26.6 with it at 100,000.
 bool spread_lists(const fs_ctx* c) {
     return c->prm.solver == FS_SOLVER_IISPH_3D && c->n_owners > (int64_t)kTileOwners * 4 * c->sms &&
            lists_can_spread(c->nbr_capacity, tile_cap_of(c));
@@ -868,7 +868,7 @@ template <typename R> fs_status order_by_radix_sort(fs_ctx* c, State<R> s) {
     // bbox of the structure's cells -> grid origin
     FS_TRY(reset_bbox(c));
     c->launches++;
-    const unsigned gb = c->scenes > 0 ? grid_for(n, 256) : std::min<unsigned>(grid_for(n, 256), 148u * 8u);
+    const unsigned gb = c->scenes > 0 ? grid_for(n, 256) : std::min(grid_for(n, 256), c->sms * 8u);
     k_bbox<R><<<gb, 256, 0, st>>>(n, s.pos, s.type, s.scene, c->nsc(), c->include_inactive,
                                                  c->search_radius, c->truncate_cells, c->bbox);
     c->launches++;
@@ -968,7 +968,7 @@ template <typename R> fs_status order_by_counting(fs_ctx* c, State<R> s) {
     const uint32_t excluded = (uint32_t)table;
     const int64_t entries = table + 1, tiles = look_tiles(entries);
     const int pb = c->tuning.block;   // the per-particle kernels' block size (fs_autotune)
-    const unsigned gb = c->scenes > 0 ? grid_for(n, 256) : std::min<unsigned>(grid_for(std::max(n, entries / 16), 256), 148u * 8u);
+    const unsigned gb = c->scenes > 0 ? grid_for(n, 256) : std::min(grid_for(std::max(n, entries / 16), 256), c->sms * 8u);
     uint32_t* entry = c->keys[0];
     uint32_t* slot = c->keys[1];
     uint32_t* list = c->perm[0];
@@ -2309,7 +2309,7 @@ fs_status fs_get_neighbors_csr(fs_ctx* c, int64_t* offsets, int64_t* indices, in
                                                                                         members, sorted);
             if (most > (uint32_t)kCsrWarpMax) {
                 c->launches++;
-                k_csr_sort_long<<<(unsigned)std::min<int64_t>(h1 - h0, 148 * 4), kCsrLongThreads, 0, st>>>(
+                k_csr_sort_long<<<(unsigned)std::min<int64_t>(h1 - h0, c->sms * 4), kCsrLongThreads, 0, st>>>(
                     h0, h1, c->csr_offsets, members, sorted);
             }
             FS_CUDA(cudaGetLastError());
@@ -2972,7 +2972,7 @@ static fs_status render_scene_of(fs_ctx* c, float surface_fraction, RenderScene&
             k_particle_box<double><<<grid_for(c->n), kBlock, 0, c->stream>>>(c->n, state_of<double>(c), d_box);
         else
             k_particle_box<float><<<grid_for(c->n), kBlock, 0, c->stream>>>(c->n, state_of<float>(c), d_box);
-        k_neighborhood_map<<<std::min<unsigned>(grid_for(c->cells, 256), 148u * 16u), 256, 0, c->stream>>>(
+        k_neighborhood_map<<<std::min(grid_for(c->cells, 256), c->sms * 16u), 256, 0, c->stream>>>(
             c->cell_start, rs.w, d_map);
         e = cudaGetLastError();
     }

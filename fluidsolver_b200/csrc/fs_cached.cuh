@@ -15,8 +15,8 @@
 // instructions; there the gradient is one rsqrt and no division.)
 //
 // Measured on a B200, a pressure iteration evaluated and from stored gradients:
-// bit-exact mode 78 -> 41 us at 100,000 fluid particles, 512 -> 307 at a million;
-// FP64 275 -> 147 at 250,047, 1,034 -> 467 at a million. The first loop's stores
+// bit-exact mode 78 -> 40 us at 100,000 fluid particles, 512 -> 307 at a million;
+// FP64 275 -> 147 at 250,047, 1,034 -> 464 at a million. The first loop's stores
 // cost it 8 % and 5 %.
 #pragma once
 

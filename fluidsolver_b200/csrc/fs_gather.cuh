@@ -44,8 +44,9 @@ __device__ __forceinline__ int64_t group_owner() {
 
 // Adds the terms of the first n entries of owner k's list to the sums: lane c
 // of the group holds sum c in acc. load(j, at): the fields of neighbor j, the
-// entry lying at `at` in the lists (-1: none, j is then 0); term(entry, fields, t): the entry's NC terms, and which of them count: bit 0
-// for t[0 .. H), bit 1 for t[H .. NC). INTERLEAVED: two terms per entry of one
+// entry lying at `at` in the lists (-1: none, j is then 0); term(entry, fields,
+// t): the entry's NC terms, and which of them count: bit 0 for t[0 .. H), bit 1
+// for t[H .. NC). INTERLEAVED: two terms per entry of one
 // sum, t[0] then t[1], held by lane 0. Every thread of the warp calls it.
 template <int NC, int H, bool INTERLEAVED = false, typename R, bool KAHAN, typename Load, typename Term>
 __device__ __forceinline__ void group_sum(const Lists& L, int64_t k, uint32_t n, GroupRows<R, NC>& rows,
@@ -320,7 +321,8 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph_l1(int64_t n, Sta
 // IISPH 3D second loop and pressure iteration (iisph3d_l2_one, ...)
 // ---------------------------------------------------------------------------
 template <typename R, bool KAHAN, bool TWO_PASS, bool CACHED>
-__global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_l2(int64_t n, State<R> s, Lists L, SolverConsts<R> c, Gradients<R> G,
+__global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_l2(int64_t n, State<R> s, Lists L, SolverConsts<R> c,
+                                                                    Gradients<R> G,
                                                                     const StepScalars* FSB_R sc,
                                                                     const int* FSB_R status) {
     phase_begins(s.phase_at, 2);
@@ -366,7 +368,10 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_l2(int64_t n, S
         __shared__ GroupRows<R, 2> rows2[kGroupsPerBlock];
         Acc<R, KAHAN> d;
         const R mi = pk.w / c.rho0_sq;
-        group_sum<2, 1, true>(L, kk, nn, rows2[threadIdx.x / kGroup], d, [&](uint32_t j, int64_t at) { return GPos<R>{position_or_gradient<CACHED>(s, G, j, at)}; },
+        group_sum<2, 1, true>(L, kk, nn, rows2[threadIdx.x / kGroup], d,
+                              [&](uint32_t j, int64_t at) {
+                                  return GPos<R>{position_or_gradient<CACHED>(s, G, j, at)};
+                              },
                               [&](uint32_t e, const GPos<R>& q, R* t) {
             const V3<R> g = gradient_of<CACHED, KAHAN>(c, xk, q.x);
             t[0] = q.x.w * dot(in, g);
@@ -401,7 +406,9 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_pressure_acc(in
     const R qk = pk / c.rho0_sq;
     Acc<R, KAHAN> acc;
     group_sum<3, 3>(L, kk, fluid ? L.size(kk) : 0u, rows[threadIdx.x / kGroup], acc,
-                    [&](uint32_t j, int64_t at) { return GPosScalar<R>{position_or_gradient<CACHED>(s, G, j, at), s.p[j]}; },
+                    [&](uint32_t j, int64_t at) {
+                        return GPosScalar<R>{position_or_gradient<CACHED>(s, G, j, at), s.p[j]};
+                    },
                     [&](uint32_t e, const GPosScalar<R>& d, R* t) {
         const V3<R> g = gradient_of<CACHED, KAHAN>(c, xk, d.x);
         const bool bnd = (e & kBoundaryBit) != 0u;
@@ -436,7 +443,9 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_pressure_update
     const V3<R> xk = xyz<R>(s.pos[kk]), ak = xyz<R>(s.acc[kk]);
     Acc<R, KAHAN> acc;
     group_sum<1, 1>(L, kk, fluid ? L.size(kk) : 0u, rows[threadIdx.x / kGroup], acc,
-                    [&](uint32_t j, int64_t at) { return GPosVec<R>{position_or_gradient<CACHED>(s, G, j, at), s.acc[j]}; },
+                    [&](uint32_t j, int64_t at) {
+                        return GPosVec<R>{position_or_gradient<CACHED>(s, G, j, at), s.acc[j]};
+                    },
                     [&](uint32_t e, const GPosVec<R>& d, R* t) {
         const V3<R> g = gradient_of<CACHED, KAHAN>(c, xk, d.x);
         t[0] = d.x.w * ((e & kBoundaryBit) ? dotf<KAHAN>(ak, g) : dotf<KAHAN>(ak - xyz<R>(d.v), g));
@@ -453,7 +462,8 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph3d_pressure_update
 // IISPH 2D second loop and pressure iteration (iisph2d_l2_at, ...)
 // ---------------------------------------------------------------------------
 template <typename R, bool KAHAN, bool CACHED>
-__global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_l2(int64_t n, State<R> s, Lists L, SolverConsts<R> c, Gradients<R> G,
+__global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_l2(int64_t n, State<R> s, Lists L, SolverConsts<R> c,
+                                                                    Gradients<R> G,
                                                                     const StepScalars* FSB_R sc,
                                                                     const int* FSB_R status) {
     phase_begins(s.phase_at, 2);
@@ -517,7 +527,9 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_pressure_acc(in
     const R pr = (s.p[kk] / c.rest_density) / c.rest_density;
     Acc<R, KAHAN> acc;
     group_sum<3, 3>(L, kk, fluid ? L.size(kk) : 0u, rows[threadIdx.x / kGroup], acc,
-                    [&](uint32_t j, int64_t at) { return GPosScalar<R>{position_or_gradient<CACHED>(s, G, j, at), s.p[j]}; },
+                    [&](uint32_t j, int64_t at) {
+                        return GPosScalar<R>{position_or_gradient<CACHED>(s, G, j, at), s.p[j]};
+                    },
                     [&](uint32_t e, const GPosScalar<R>& d, R* t) {
         const V3<R> g = gradient_of<CACHED, KAHAN>(c, xk, d.x);
         if (!(e & kBoundaryBit)) put3(t, (d.x.w * (pr + (d.a / c.rest_density) / c.rest_density)) * g);
@@ -541,7 +553,9 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_iisph2d_pressure_update
     const V3<R> xk = xyz<R>(s.pos[kk]), ak = xyz<R>(s.acc[kk]);
     Acc<R, KAHAN> acc;
     group_sum<1, 1>(L, kk, fluid ? L.size(kk) : 0u, rows[threadIdx.x / kGroup], acc,
-                    [&](uint32_t j, int64_t at) { return GPosVec<R>{position_or_gradient<CACHED>(s, G, j, at), s.acc[j]}; },
+                    [&](uint32_t j, int64_t at) {
+                        return GPosVec<R>{position_or_gradient<CACHED>(s, G, j, at), s.acc[j]};
+                    },
                     [&](uint32_t e, const GPosVec<R>& d, R* t) {
         const V3<R> g = gradient_of<CACHED, KAHAN>(c, xk, d.x);
         t[0] = d.x.w * ((e & kBoundaryBit) ? dot(ak, g) : dot(ak - xyz<R>(d.v), g));

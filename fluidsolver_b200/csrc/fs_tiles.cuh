@@ -191,7 +191,7 @@ __device__ __forceinline__ bool stage_tile_wait(TileStage& st, int* __restrict__
 // as its list has one, a candidate whose slot is p + k modulo 8, so that the
 // eight lanes read eight bank groups; entries whose class has no place left
 // take the others' free places. B200: the builder's part of the 1M dam's
-// search 300 -> 342 us, and a pressure iteration 213 -> 190, the first loop
+// search 300 -> 342 us, and a pressure iteration 213 -> 187, the first loop
 // 141 -> 135, the second 149 -> 140; 100,000 particles: an iteration 28.9 ->
 // 26.6; 64 dams in one step 14.05 -> 13.4 ms. (SESPH reads its lists twice,
 // which does not pay for the sorting.)
@@ -1273,9 +1273,9 @@ __global__ void __launch_bounds__(pressure_threads<TPO>(), update_blocks_per_sm<
 //   else  a block stages its tiles one after the other in every pass.
 //
 // Measured on a B200, one iteration of a dam's loop, the WHILE node against this:
-// 512 fluid particles 17.0 -> 12.6 us, 8,000 16.4 -> 11.9, 29,791 18.8 -> 13.9,
-// 100,000 34.6 -> 28.9, 250,047 65.5 -> 60.9, 512,000 115 -> 110 (26.6, 57.6 and
-// 106 since the entries are spread over the banks, k_build_tiles). A pass of a
+// 512 fluid particles 17.0 -> 13.1 us, 8,000 16.4 -> 12.5, 29,791 18.8 -> 13.3,
+// 100,000 34.6 -> 28.9, 250,047 65.5 -> 60.9, 512,000 115 -> 110 (26.6, 55.1 and
+// 102 since the entries are spread over the banks, k_build_tiles). A pass of a
 // small scene is a chain of latencies (copying the field 0.7 us, the walk 1.4,
 // the barrier 1.7), and the fallback tiles' are the longest.
 //

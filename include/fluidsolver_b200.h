@@ -65,7 +65,7 @@ typedef enum fs_solver_kind {
 
 /*
  * Neighbor-set contract of the reference search being replaced. One device
- * search (cell-key radix sort + cell-order reordering + cell table) serves all of
+ * search (stable ordering by cell key + cell-order reordering + cell table) serves all of
  * them; the contract fixes the predicate, which particles own a list, which
  * particles may appear in one, and the capacity limit.
  */
@@ -92,8 +92,9 @@ typedef enum fs_precision {
                                             device-side early exit inside a CUDA graph */
 #define FS_FLAG_ONE_KERNEL_STEPS 0x4u  /* fs_step / fs_run of a single scene of at most 4,096 particles (not
                                           the 3D fast mode, not compact hashing) run whole steps in one launch
-                                          of one block instead of a CUDA graph of per-phase kernels; the same
-                                          results bit for bit */
+                                          of one thread-block cluster (fs_small_blocks) instead of a CUDA graph
+                                          of per-phase kernels; the same results bit for bit, and now slower
+                                          (the 2D SESPH dam of 3,688 particles 67 against 33 us a step) */
 
 /* Particle types (Particle.hpp:7-12). */
 #define FS_TYPE_NORMAL 0
@@ -274,8 +275,7 @@ fs_status fs_last_phase_times(fs_ctx* ctx, float* ms5);
 /* The context's CUDA stream (a cudaStream_t), for callers that time or order
  * their own work against the library's. */
 void* fs_stream(fs_ctx* ctx);
-/* Number of this library's own kernel launches since the context was created
- * (library kernels such as the radix sort's are not counted). */
+/* Number of this library's own kernel launches since the context was created. */
 int64_t fs_launch_count(fs_ctx* ctx);
 /* Blocks (one thread-block cluster) of the last small-scene launch
  * (FS_FLAG_ONE_KERNEL_STEPS), 0 when the last steps took the step-by-step
@@ -337,10 +337,12 @@ fs_status fs_set_tile_wait_limit(fs_ctx* ctx, int32_t tries);
  * the default (4,194,304); 0 gives up without a poll. */
 fs_status fs_set_grid_wait_limits(fs_ctx* ctx, int32_t scan_tries, int32_t barrier_tries);
 
-/* The searches' own sort on caller keys, for tests of the sort alone: the
+/* The library's own sort on caller keys, for tests of the sort alone: the
  * stable least-significant-digit radix sort that orders the particles by
- * (region, cell) key every search (and, in the reference-order mode, by the
- * 64-bit key with the order inside a cell), run on `device` over n host keys
+ * (region, cell) key in the searches that do not order them by counting (many
+ * excluded inactive particles, or boxes with few cells for their particles;
+ * in the reference-order mode, by the 64-bit key with the order inside a
+ * cell) and in compact hashing, run on `device` over n host keys
  * of key_bytes 4 or 8 bytes. Every key must be below 2^bits (1 <= bits <=
  * 8 * key_bytes). sorted (n keys, may be null) receives the keys in
  * ascending order; order (n, may be null) the input position of each, equal
