@@ -14,7 +14,10 @@ DEFAULT = "/root/reference"
 
 
 def reference_dir() -> str:
-    return os.environ.get("FS_REFERENCE_DIR", DEFAULT)
+    """The checkout's directory. An empty directory is no checkout: the path is then one that does
+    not exist, so that whoever looks for the checkout finds it absent."""
+    d = os.environ.get("FS_REFERENCE_DIR", DEFAULT)
+    return os.path.join(d, "absent") if os.path.isdir(d) and not os.listdir(d) else d
 
 
 def present() -> bool:
